@@ -168,7 +168,7 @@ gpb_status gpb_fetch(gpb_ctx* ctx, int stage, size_t patch, void* dst, size_t ds
 gpb_status gpb_last_stats(gpb_ctx* ctx, gpb_stats* st);
 
 /* The context's autotuner: for each shape bucket of a tunable kernel (the
- * texton tile's thread count, the block step's X staging and tile queue),
+ * texton tile's thread count, the block step's tile height),
  * "key=chosen variant (median ms of each variant); ...", -1 while a bucket
  * is still being tried.  Every variant gives identical results; the first
  * launches of a bucket try them on real work.  GPB_NO_TUNE=1 in the

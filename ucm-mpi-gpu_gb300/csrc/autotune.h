@@ -1,8 +1,7 @@
 // autotune.h -- the library's online autotuner for kernel variants.
 //
 // A tunable launch has several variants that compute bit-identical results
-// (thread counts per tile, how a persistent kernel walks its tiles, how it
-// stages an operand) but run at different speeds depending on the batch's
+// (thread counts per tile, tile sizes) but run at different speeds depending on the batch's
 // shape.  For a key -- the kernel and a bucket of the launch's shape -- the
 // first launches try the variants in turn on real work, each timed with a
 // pair of CUDA events on the launching stream; once every variant has `reps`

@@ -109,7 +109,6 @@ struct Buf {
   int4* work_tex = nullptr; size_t c_wt = 0;
   int4* work_cue = nullptr; size_t c_wc = 0;
   int4* work16 = nullptr; size_t c_w16 = 0;
-  int4* work_blk = nullptr; size_t c_wb = 0;
   EigTile* tiles = nullptr; size_t c_tiles = 0;
   int* tile_begin = nullptr; size_t c_tb = 0;
   int* tile_count = nullptr; size_t c_tc = 0;
@@ -128,14 +127,13 @@ struct Buf {
   EigTile* ctiles = nullptr; size_t c_ctiles = 0;
   int* ctile_begin = nullptr; size_t c_ctb = 0;
   int* ctile_count = nullptr; size_t c_ctc = 0;
-  int4* cwork_blk = nullptr; size_t c_cwb = 0;
   int4* cwork16 = nullptr; size_t c_cw16 = 0;
   float* cwc = nullptr; size_t c_cwc = 0;
   float* cdeg = nullptr; size_t c_cdeg = 0;
   float* cdis = nullptr; size_t c_cdis = 0;
   float* cblk[4] = {nullptr, nullptr, nullptr, nullptr}; size_t c_cblk[4] = {0, 0, 0, 0};
-  float* afull = nullptr; size_t c_afull = 0;  // pixel-major fine stencil rows
-  int4* work_act = nullptr; size_t c_wact = 0;  // block-step tiles of the still active patches
+  float* afull = nullptr; size_t c_afull = 0;  // fine stencil rows in the block step's tile layout
+  int4* work_act = nullptr; size_t c_wact = 0;  // 16 x 16 tiles of the still active patches
   float* stitch = nullptr; size_t c_stitch = 0;  // BLEND accumulators [10][image]
   uint32_t* spcount = nullptr; size_t c_spcount = 0;          // superpixel histograms
   unsigned long long* spcsum = nullptr; size_t c_spcsum = 0;  // superpixel colour sums
@@ -532,10 +530,10 @@ extern "C" void gpb_destroy(gpb_ctx* ctx) {
   void* ptrs[] = {b.packed, b.grey, b.lab4, b.nbins, b.repair, b.repair_count, b.mpbo, b.go, b.mpb, b.raw,
                   b.wfull, b.counts, b.wup, b.aup, b.deg, b.dis, b.adiag, b.V[0], b.V[1], b.W[0], b.W[1], b.evec,
                   b.part, b.hbuf, b.T, b.Y, b.beta2, b.counter, b.active, b.decision, b.nkeep, b.evals,
-                  b.mm, b.spb, b.gpbo, b.nmax, b.orient, b.patches, b.work_tex, b.work_cue, b.work16, b.work_blk,
+                  b.mm, b.spb, b.gpbo, b.nmax, b.orient, b.patches, b.work_tex, b.work_cue, b.work16,
                   b.tiles, b.tile_begin, b.tile_count, ctx->d_ic, ctx->d_k32_ring, ctx->d_ring_of,
                   b.blk[0], b.blk[1], b.blk[2], b.blk[3], b.bpart, b.bgram, b.bgram2, b.bmat, b.btheta, b.bres,
-                  b.bcoef, b.bdone, b.cpatches, b.ctiles, b.ctile_begin, b.ctile_count, b.cwork_blk,
+                  b.bcoef, b.bdone, b.cpatches, b.ctiles, b.ctile_begin, b.ctile_count,
                   b.cwork16, b.cwc, b.cdeg, b.cdis, b.cblk[0], b.cblk[1], b.cblk[2], b.cblk[3], b.afull, b.berr, b.work_act, b.stitch, b.spcount, b.spcsum};
   for (void* q : ptrs)
     if (q) cudaFree(q);
@@ -608,7 +606,7 @@ namespace {
 
 struct Layout {
   std::vector<PatchDev> patches;
-  std::vector<int4> work_tex, work_cue, work16, work_blk;
+  std::vector<int4> work_tex, work_cue, work16;
   std::vector<EigTile> tiles;
   std::vector<int> tile_begin, tile_count;
   long long total_pix = 0, lvec = 0;
@@ -621,9 +619,9 @@ Layout make_layout(size_t n, const uint32_t* ws, const uint32_t* hs) {
   for (size_t i = 0; i < n; i++) wmax = std::max(wmax, (int)ws[i]);
   // the gap before and after every patch: a stencil neighbour lies at most
   // kStencilR rows + kStencilR pixels away, and a block-step tile's staged
-  // row runs kStepTileW + 2 kStencilR pixels from its left halo column
+  // row runs kStepTile + 2 kStencilR pixels from its left halo column
   const long long pad =
-      (((long long)kStencilR * wmax + kStencilR + kStepTileW + 2 * kStencilR) + 63) / 64 * 64;
+      (((long long)kStencilR * wmax + kStencilR + kStepTile + 2 * kStencilR) + 63) / 64 * 64;
   long long pix = 0, vec = pad;
   for (size_t i = 0; i < n; i++) {
     PatchDev P;
@@ -640,12 +638,10 @@ Layout make_layout(size_t n, const uint32_t* ws, const uint32_t* hs) {
     for (int y = 0; y < P.H; y += 16)
       for (int x = 0; x < P.W; x += 16) {
         L.work_tex.push_back(make_int4(pi, y, x, 0));
-        L.work16.push_back(make_int4(pi, y, x, 0));
+        L.work16.push_back(make_int4(pi, y, x, (int)L.work16.size()));
       }
     for (int y = 0; y < P.H; y += kCueTileH)
       for (int x = 0; x < P.W; x += kCueTileW) L.work_cue.push_back(make_int4(pi, y, x, 0));
-    for (int y = 0; y < P.H; y += kStepTileH)
-      for (int x = 0; x < P.W; x += kStepTileW) L.work_blk.push_back(make_int4(pi, y, x, 0));
     L.tile_begin.push_back((int)L.tiles.size());
     for (int p0 = 0; p0 < P.N; p0 += kEigTile) {
       EigTile t;
@@ -724,15 +720,14 @@ static gpb_status ensure_buffers(gpb_ctx* ctx, const Layout& L, bool layout_chan
   es.push_back(grow(b.work_tex, b.c_wt, L.work_tex.size()));
   es.push_back(grow(b.work_cue, b.c_wc, L.work_cue.size()));
   es.push_back(grow(b.work16, b.c_w16, L.work16.size()));
-  es.push_back(grow(b.work_blk, b.c_wb, L.work_blk.size()));
   es.push_back(grow(b.tiles, b.c_tiles, nt));
   es.push_back(grow(b.tile_begin, b.c_tb, np));
   es.push_back(grow(b.tile_count, b.c_tc, np));
   if (q.eig_mode != GPB_EIG_LANCZOS) {
     for (int i = 0; i < 4; i++) es.push_back(grow(b.blk[i], b.c_blk[i], (size_t)kBlk * V));
-    es.push_back(grow(b.afull, b.c_afull, (size_t)kFullNC * V));
-    es.push_back(grow(b.work_act, b.c_wact, L.work_blk.size()));
-    es.push_back(grow(b.berr, b.c_berr, 4));  // error word, spare, block-step queue [2]
+    es.push_back(grow(b.afull, b.c_afull, (size_t)kFullNC * kStepTile * kStepTile * L.work16.size()));
+    es.push_back(grow(b.work_act, b.c_wact, L.work16.size()));
+    es.push_back(grow(b.berr, b.c_berr, 1));  // the block step's error word
     es.push_back(grow(b.bpart, b.c_bpart, nt * kBlkSplit * 2 * kBlk * kBlk));  // two Gram matrices per slot
     es.push_back(grow(b.bgram, b.c_bgram, np * kBlk * kBlk));
     es.push_back(grow(b.bgram2, b.c_bgram2, np * kBlk * kBlk));
@@ -748,9 +743,8 @@ static gpb_status ensure_buffers(gpb_ctx* ctx, const Layout& L, bool layout_chan
     es.push_back(grow(b.ctiles, b.c_ctiles, ntc));
     es.push_back(grow(b.ctile_begin, b.c_ctb, np));
     es.push_back(grow(b.ctile_count, b.c_ctc, np));
-    es.push_back(grow(b.cwork_blk, b.c_cwb, C->work_blk.size()));
     es.push_back(grow(b.cwork16, b.c_cw16, C->work16.size()));
-    es.push_back(grow(b.cwc, b.c_cwc, (size_t)kCoarseNC * Vc));
+    es.push_back(grow(b.cwc, b.c_cwc, (size_t)kCoarseNC * kStepTile * kStepTile * C->work16.size()));
     es.push_back(grow(b.cdeg, b.c_cdeg, Vc));
     es.push_back(grow(b.cdis, b.c_cdis, Vc));
     for (int i = 0; i < 4; i++) es.push_back(grow(b.cblk[i], b.c_cblk[i], (size_t)kBlk * Vc));
@@ -774,10 +768,8 @@ static gpb_status ensure_buffers(gpb_ctx* ctx, const Layout& L, bool layout_chan
     cudaMemsetAsync(b.counter, 0, np * sizeof(int), s);
     if (q.eig_mode != GPB_EIG_LANCZOS) {
       for (int i = 0; i < 4; i++) cudaMemsetAsync(b.blk[i], 0, (size_t)kBlk * V * sizeof(float), s);
-      cudaMemsetAsync(b.afull, 0, (size_t)kFullNC * V * sizeof(float), s);
     }
     if (q.eig_mode == GPB_EIG_WARM && C) {
-      cudaMemsetAsync(b.cwc, 0, (size_t)kCoarseNC * C->lvec * sizeof(float), s);
       cudaMemsetAsync(b.cdis, 0, C->lvec * sizeof(float), s);
       for (int i = 0; i < 4; i++) cudaMemsetAsync(b.cblk[i], 0, (size_t)kBlk * C->lvec * sizeof(float), s);
     }
@@ -974,8 +966,8 @@ struct Level {
   const EigTile* tiles;
   const int* tile_begin;
   const int* tile_count;
-  const int4* work_blk;
-  const float* afull;  // pixel-major stencil rows of the level's operator
+  const int4* work16;
+  const float* afull;  // stencil rows of the level's operator, in the block step's tile layout
   int coarse;
   float* blk[4];
 };
@@ -990,12 +982,12 @@ static gpb_status solve_block(gpb_ctx* ctx, const Level& lv, bool have_start, do
   cudaStream_t s = ctx->st;
   const int np = (int)L.patches.size(), nt = (int)L.tiles.size(), nev = q.nvec;
   // the persistent block step walks a tile list; once patches converge it
-  // gets only the tiles of the active ones (L.work_blk is patch-major)
+  // gets only the tiles of the active ones (L.work16 is patch-major)
   std::vector<int> tb_begin(np + 1, 0);
-  for (const int4& t : L.work_blk) tb_begin[t.x + 1]++;
+  for (const int4& t : L.work16) tb_begin[t.x + 1]++;
   for (int i = 0; i < np; i++) tb_begin[i + 1] += tb_begin[i];
-  int nwb = (int)L.work_blk.size();
-  const int4* work_blk = lv.work_blk;
+  int nwb = (int)L.work16.size();
+  const int4* work_blk = lv.work16;
   std::vector<int4> act_tiles;
   std::vector<int> listed(np, 1);  // the patches the current list holds
   // a multiple of 3, so the three-buffer Chebyshev rotation ends where it
@@ -1011,7 +1003,6 @@ static gpb_status solve_block(gpb_ctx* ctx, const Level& lv, bool have_start, do
   a.a_diag = nullptr;
   a.afull = lv.afull;
   a.err = b.berr;
-  a.queue = b.berr + 2;
   a.coarse = lv.coarse;
   a.lvec = L.lvec;
   a.coef = b.bcoef;
@@ -1214,7 +1205,7 @@ static gpb_status solve_block(gpb_ctx* ctx, const Level& lv, bool have_start, do
     if (active != listed) {
       act_tiles.clear();
       for (int i = 0; i < np; i++)
-        if (active[i]) act_tiles.insert(act_tiles.end(), L.work_blk.begin() + tb_begin[i], L.work_blk.begin() + tb_begin[i + 1]);
+        if (active[i]) act_tiles.insert(act_tiles.end(), L.work16.begin() + tb_begin[i], L.work16.begin() + tb_begin[i + 1]);
       CK(cudaMemcpyAsync(b.work_act, act_tiles.data(), act_tiles.size() * sizeof(int4), cudaMemcpyHostToDevice, s));
       work_blk = b.work_act;
       nwb = (int)act_tiles.size();
@@ -1297,7 +1288,6 @@ static gpb_status solve_warm(gpb_ctx* ctx, const Layout& L, const Layout& Lc) {
   CK(cudaMemcpyAsync(b.ctiles, Lc.tiles.data(), Lc.tiles.size() * sizeof(EigTile), cudaMemcpyHostToDevice, s));
   CK(cudaMemcpyAsync(b.ctile_begin, Lc.tile_begin.data(), np * sizeof(int), cudaMemcpyHostToDevice, s));
   CK(cudaMemcpyAsync(b.ctile_count, Lc.tile_count.data(), np * sizeof(int), cudaMemcpyHostToDevice, s));
-  CK(cudaMemcpyAsync(b.cwork_blk, Lc.work_blk.data(), Lc.work_blk.size() * sizeof(int4), cudaMemcpyHostToDevice, s));
   CK(cudaMemcpyAsync(b.cwork16, Lc.work16.data(), Lc.work16.size() * sizeof(int4), cudaMemcpyHostToDevice, s));
   CoarseArgs c;
   c.fine = b.patches;
@@ -1313,7 +1303,7 @@ static gpb_status solve_warm(gpb_ctx* ctx, const Layout& L, const Layout& Lc) {
   c.disc = b.cdis;
   CK(cf_launch_coarsen(c, (int)Lc.work16.size(), s));
   ctx->launches += 2;
-  Level lc = {&Lc, b.cpatches, b.ctiles, b.ctile_begin, b.ctile_count, b.cwork_blk, b.cwc, 1,
+  Level lc = {&Lc, b.cpatches, b.ctiles, b.ctile_begin, b.ctile_count, b.cwork16, b.cwc, 1,
               {b.cblk[0], b.cblk[1], b.cblk[2], b.cblk[3]}};
   float* Xc = nullptr;
   gpb_status st = solve_block(ctx, lc, false, ctx->prm.warm_tol, false, &Xc);
@@ -1333,7 +1323,7 @@ static gpb_status solve_warm(gpb_ctx* ctx, const Layout& L, const Layout& Lc) {
     CK(cudaMemcpyAsync(b.blk[0], b.blk[1], blk_bytes, cudaMemcpyDeviceToDevice, s));
     ctx->launches += 2;
   }
-  Level lf = {&L, b.patches, b.tiles, b.tile_begin, b.tile_count, b.work_blk, b.afull, 0,
+  Level lf = {&L, b.patches, b.tiles, b.tile_begin, b.tile_count, b.work16, b.afull, 0,
               {b.blk[0], b.blk[1], b.blk[2], b.blk[3]}};
   float* Xf = nullptr;
   return solve_block(ctx, lf, true, ctx->prm.eig_tol, true, &Xf);
@@ -1360,7 +1350,7 @@ static gpb_status solve_learned(gpb_ctx* ctx, const Layout& L) {
   CK(ctx->net->forward(s));
   CK(ln_launch_start(ctx->net->patches0_dev(), b.patches, (int)L.patches.size(), maxn, ctx->net->y(), b.blk[0], s));
   ctx->launches += ctx->net->launches() - l0 + 1;
-  Level lf = {&L, b.patches, b.tiles, b.tile_begin, b.tile_count, b.work_blk, b.afull, 0,
+  Level lf = {&L, b.patches, b.tiles, b.tile_begin, b.tile_count, b.work16, b.afull, 0,
               {b.blk[0], b.blk[1], b.blk[2], b.blk[3]}};
   float* Xf = nullptr;
   return solve_block(ctx, lf, true, ctx->prm.eig_tol, true, &Xf);
@@ -1402,7 +1392,6 @@ static gpb_status run_batch(gpb_ctx* ctx, size_t n, const uint32_t* ws, const ui
   CK(cudaMemcpyAsync(b.work_tex, L.work_tex.data(), L.work_tex.size() * sizeof(int4), cudaMemcpyHostToDevice, s));
   CK(cudaMemcpyAsync(b.work_cue, L.work_cue.data(), L.work_cue.size() * sizeof(int4), cudaMemcpyHostToDevice, s));
   CK(cudaMemcpyAsync(b.work16, L.work16.data(), L.work16.size() * sizeof(int4), cudaMemcpyHostToDevice, s));
-  CK(cudaMemcpyAsync(b.work_blk, L.work_blk.data(), L.work_blk.size() * sizeof(int4), cudaMemcpyHostToDevice, s));
   CK(cudaMemcpyAsync(b.tiles, L.tiles.data(), L.tiles.size() * sizeof(EigTile), cudaMemcpyHostToDevice, s));
   CK(cudaMemcpyAsync(b.tile_begin, L.tile_begin.data(), np * sizeof(int), cudaMemcpyHostToDevice, s));
   CK(cudaMemcpyAsync(b.tile_count, L.tile_count.data(), np * sizeof(int), cudaMemcpyHostToDevice, s));
@@ -1495,7 +1484,7 @@ static gpb_status run_batch(gpb_ctx* ctx, size_t n, const uint32_t* ws, const ui
                     ctx->prm.keep_intermediates ? b.wfull : nullptr, s));
     if (blockm) {
       GK(cf_launch_full(b.patches, b.work16, (int)L.work16.size(), b.aup, b.adiag, L.lvec, b.afull, s));
-      GK(cudaMemsetAsync(b.berr, 0, 4 * sizeof(int), s));  // error word and the block step's queue
+      GK(cudaMemsetAsync(b.berr, 0, sizeof(int), s));
       ctx->launches++;
     }
     GK(stage_mark(ctx->ev[5], s));
@@ -1517,7 +1506,7 @@ static gpb_status run_batch(gpb_ctx* ctx, size_t n, const uint32_t* ws, const ui
   } else if (ctx->prm.eig_mode == GPB_EIG_LEARNED) {
     es = solve_learned(ctx, L);
   } else if (ctx->prm.eig_mode == GPB_EIG_BLOCK) {
-    Level lf = {&L, b.patches, b.tiles, b.tile_begin, b.tile_count, b.work_blk, b.afull, 0,
+    Level lf = {&L, b.patches, b.tiles, b.tile_begin, b.tile_count, b.work16, b.afull, 0,
                 {b.blk[0], b.blk[1], b.blk[2], b.blk[3]}};
     float* Xf = nullptr;
     es = solve_block(ctx, lf, false, ctx->prm.eig_tol, true, &Xf);

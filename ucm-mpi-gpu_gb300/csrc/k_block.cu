@@ -3,8 +3,9 @@
 //
 // A block of kBlk = 32 vectors is stored pixel-major ([vec][32] floats) in the
 // padded vector layout, so every stencil neighbour of a pixel is one
-// contiguous 128-byte row; the operator of the block kernels is stored
-// pixel-major too, one full stencil row per pixel (cf_full).
+// contiguous 128-byte row; the operator of the block kernels holds one full
+// stencil row per pixel, tile by tile in the order the step loads it
+// (cf_full).
 //
 //   cf_step    Y' = alpha (A Y) + beta Y + gamma X   (scaled Chebyshev
 //              recurrence, Zhou & Saad 2007; with alpha=1, beta=gamma=0 it
@@ -71,15 +72,15 @@ __device__ __forceinline__ void fma4(float4& acc, float a, const float4& x) {
 }
 
 // ------------------------------------------------------------ Chebyshev step
-// One CTA owns a kStepTileH x kStepTileW (8 x 16) pixel tile.  One thread
-// issues bulk asynchronous copies (cp.async.bulk, completion counted on an
-// mbarrier) of the tile's Y rows with an R-pixel halo -- each a contiguous
-// (16 + 2R) x 128-byte run of the pixel-major block -- and of the tile's
-// coefficient rows (pixel-major, one full stencil row per pixel).  Then lane
-// = block column: a warp computes a 4 x 4 pixel block for all 32 columns, so
-// a staged value (one conflict-free 128-byte shared row per warp) feeds up
-// to 16 pixels and one broadcast 16-byte load brings four coefficients of a
-// pixel.  About one shared-memory wavefront per output instead of 2.6.
+// The operator of a level is stored per 16 x 16 pixel tile (the tiles of the
+// 16 x 16 work list, in its order), ready for the step's loads: 4 consecutive
+// stencil coefficients of a pixel are one 16-byte slot, and a tile is [chunk
+// of 4 offsets][slot of 256].  A warp of the step owns 2 tile rows, a
+// quarter-warp 2 x 4 pixels of them, a lane 4 block columns of these 8
+// pixels.  Slot (w, k, q) = 32 w + 4 k + q holds pixel k (row k / 4, column
+// k % 4) of quarter q of warp w, so the four quarters' coefficients of a load
+// are 64 contiguous bytes, and a chunk of a tile is one contiguous copy.
+constexpr int kTilePx = kStepTile * kStepTile;
 
 // the radius-5 disk of the fine level (81 offsets in scanline order, rows
 // padded to 84 floats = 21 x 16 bytes) and the 7 x 7 square of the coarse one
@@ -107,24 +108,23 @@ static_assert(DiskStencil::index(0, 0) == kStencilN / 2 && DiskStencil::index(kS
 static_assert(SquareStencil::index(kCR, kCR) == kCN - 1, "square numbering");
 static_assert(DiskStencil::NC == kFullNC && SquareStencil::NC == kCoarseNC, "row widths");
 
-constexpr int ST_TY = kStepTileH, ST_TX = kStepTileW, ST_B = 4;  // tile and per-warp block
-static_assert((ST_TY / ST_B) * (ST_TX / ST_B) == 8, "8 warps cover the tile");
-
-template <class S>
+// Shared memory of the step for WARPS consumer warps (2 WARPS tile rows):
+// two stages of Y rows with their halo, and a ring of coefficient groups.
+template <class S, int WARPS>
 struct StepSmem {
-  static constexpr int PH = ST_TY + 2 * S::R, PW = ST_TX + 2 * S::R;
+  static constexpr int PH = 2 * WARPS + 2 * S::R, PW = kStepTile + 2 * S::R;
+  static constexpr int NCH = S::NC / 4, GC = 3, NG = (NCH + GC - 1) / GC;  // chunks, chunks per group, groups
+  static constexpr int RING = 4;
   static constexpr size_t y_bytes = (size_t)PH * PW * kBlk * sizeof(float);
-  static constexpr size_t c_bytes = (size_t)ST_TY * ST_TX * S::NC * sizeof(float);
-  static constexpr size_t stage = y_bytes + c_bytes;  // one pipeline stage
-  static constexpr size_t bytes = 2 * stage + 256;    // two stages, tile records, mbarriers
-  // the X-staging variant: one slot per consumer warp for its 4 x 4 block's X rows
-  static constexpr size_t x_slot = (size_t)ST_B * ST_B * kBlk * sizeof(float);
-  static constexpr size_t bytes_xs = bytes + 8 * x_slot;
-  static_assert(stage % 128 == 0, "stage alignment");
-  static_assert(bytes_xs <= 232448, "shared memory per CTA");
+  static constexpr size_t chunk = (size_t)WARPS * 32 * 16;
+  static constexpr size_t group = GC * chunk;
+  static constexpr size_t bars = 2 * y_bytes + RING * group;  // tile records, mbarriers
+  static constexpr size_t bytes = bars + 256;
+  static_assert(y_bytes % 128 == 0 && group % 128 == 0, "alignment");
+  static_assert(bytes <= 232448, "shared memory per CTA");
 };
 
-// what the producer warp tells the consumers about the tile in a stage
+// what the Y producer tells the consumers about the tile in a stage
 struct StepMeta {
   int end;        // 1: no more tiles for this CTA
   int W, H, y0;
@@ -160,15 +160,6 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t by
                "l"(src), "r"(bytes), "r"(smem_addr(bar))
                : "memory");
 }
-// 16-byte asynchronous global -> shared copy (L2 only); src_bytes 0 writes
-// zeros and reads nothing
-__device__ __forceinline__ void cp_async16(void* dst, const void* src, uint32_t src_bytes) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_addr(dst)), "l"(src), "r"(src_bytes)
-               : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
-
 // polls of the tile's barrier before a CTA gives up (each poll may suspend
 // the thread for a short hardware-defined time; the copies take microseconds)
 constexpr int kBarSpin = 1 << 20;
@@ -186,9 +177,55 @@ __device__ __forceinline__ float f4get(const float4& v) {
   else return v.w;
 }
 
-// one staged position (RY, DX) relative to the warp's block origin: the value
-// of this lane's column there, times the coefficient of every block pixel
-// whose stencil covers it
+// Pairs of FP32 values for the packed f32x2 instructions: each half is one
+// correctly rounded operation, so results equal the scalar ones; an
+// instruction does two, and the three-register FMA runs at 0.29 cycles per
+// value against 0.34 (measured per warp and SM).
+struct F2 {
+  uint64_t v;
+};
+__device__ __forceinline__ F2 f2(float x, float y) {
+  F2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(x), "f"(y));
+  return r;
+}
+__device__ __forceinline__ float2 f2_split(F2 a) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a.v));
+  return r;
+}
+__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
+  F2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
+__device__ __forceinline__ F2 f2_add(F2 a, F2 b) {
+  F2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F2 f2_sub(F2 a, F2 b) {
+  F2 r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+
+// The coefficient ring as a consumer warp sees it.  Group g of a tile is
+// waited for when the warp's first pixel reaches its first chunk and released
+// when the last pixel has loaded its last chunk; both places are known at
+// compile time.
+struct StepRing {
+  unsigned char* base;   // the lane's slot of pixel 0 in ring place 0
+  uint64_t *full, *empty;
+  unsigned n0;           // groups consumed before this tile
+  bool bad;              // a wait gave up: no further waits, the results are dropped
+};
+
+constexpr int SB_R = 2, SB_C = 4, SB_N = SB_R * SB_C;  // a quarter-warp's pixels
+
+// one staged position (RY, DX) relative to the quarter's block origin: the
+// value of this lane's columns there, times the coefficient of every block
+// pixel whose stencil covers it
 // C (compensated): the terms are summed by FMA in groups of four (grp) and
 // each group is folded into a float-float (acc, lo) by an exact TwoSum,
 // which removes the accumulation error of the 81-term sum -- the term that
@@ -196,310 +233,330 @@ __device__ __forceinline__ float f4get(const float4& v) {
 // sum nearly cancel -- down to the groups' own four-term rounding, at about
 // a third of the cost of a TwoSum per term; used for the Rayleigh-Ritz
 // products and residuals, not the filter
-// a half-warp's sub-block: SB_R x SB_C pixels (the two halves of a warp
-// split its 4 x 4 block by rows), two block columns per lane
-constexpr int SB_R = 2, SB_C = 4, SB_N = SB_R * SB_C;
-
-template <class S, bool C, int RY, int DX, int I>
-__device__ __forceinline__ void step_pixels(const float* __restrict__ cs, float2 v, float4 (&cw)[SB_N],
-                                            float2 (&acc)[SB_N], float2 (&lo)[SB_N], float2 (&grp)[SB_N]) {
+template <class S, int WARPS, bool C, int RY, int DX, int I>
+__device__ __forceinline__ void step_pixels(StepRing& ring, const unsigned char* (&gb)[StepSmem<S, WARPS>::NG],
+                                            const F2 (&v)[2], float4 (&cw)[SB_N], F2 (&acc)[SB_N][2],
+                                            F2 (&lo)[SB_N][2], F2 (&grp)[SB_N][2]) {
+  using SM = StepSmem<S, WARPS>;
   if constexpr (I < SB_N) {
     constexpr int bi = I / SB_C, bj = I % SB_C;
     if constexpr (S::in(RY - bi, DX - bj)) {
-      constexpr int idx = S::index(RY - bi, DX - bj);
-      // a pixel meets its offsets in scanline order, so chunk idx/4 is
-      // first needed at idx % 4 == 0
-      if constexpr (idx % 4 == 0) cw[I] = *(const float4*)(cs + (bi * ST_TX + bj) * S::NC + idx);
-      const float cf = f4get<idx % 4>(cw[I]);
-      if constexpr (C) {
-        grp[I].x = fmaf(cf, v.x, grp[I].x);
-        grp[I].y = fmaf(cf, v.y, grp[I].y);
-        // a pixel's offsets run 0 .. N-1 in order: fold after every fourth
-        if constexpr (idx % 4 == 3 || idx == S::N - 1) {
-          float t = acc[I].x + grp[I].x, z = t - acc[I].x;
-          lo[I].x += (acc[I].x - (t - z)) + (grp[I].x - z);
-          acc[I].x = t;
-          t = acc[I].y + grp[I].y;
-          z = t - acc[I].y;
-          lo[I].y += (acc[I].y - (t - z)) + (grp[I].y - z);
-          acc[I].y = t;
-          grp[I] = make_float2(0.f, 0.f);
+      constexpr int idx = S::index(RY - bi, DX - bj), ch = idx / 4, g = ch / SM::GC;
+      // a pixel meets its offsets in scanline order, so chunk idx / 4 is
+      // first needed at idx % 4 == 0; pixel 0 is the first to get there
+      // (smallest row and column), pixel SB_N - 1 the last
+      if constexpr (idx % 4 == 0) {
+        if constexpr (I == 0 && ch % SM::GC == 0) {
+          const unsigned n = ring.n0 + g;
+          if (!ring.bad) ring.bad = !mbar_wait(ring.full + n % SM::RING, (n / SM::RING) & 1);
+          gb[g] = ring.base + (n % SM::RING) * SM::group;
         }
-      } else {
-        acc[I].x = fmaf(cf, v.x, acc[I].x);
-        acc[I].y = fmaf(cf, v.y, acc[I].y);
+        cw[I] = *(const float4*)(gb[g] + (ch % SM::GC) * SM::chunk + I * 64);
+        if constexpr (I == SB_N - 1 && (ch % SM::GC == SM::GC - 1 || ch == SM::NCH - 1)) {
+          __syncwarp();
+          if ((threadIdx.x & 31) == 0) mbar_arrive(ring.empty + (ring.n0 + g) % SM::RING);
+        }
+      }
+      const float c1 = f4get<idx % 4>(cw[I]);
+      const F2 cf = f2(c1, c1);
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        if constexpr (C) {
+          grp[I][h] = f2_fma(cf, v[h], grp[I][h]);
+          // a pixel's offsets run 0 .. N-1 in order: fold after every fourth
+          if constexpr (idx % 4 == 3 || idx == S::N - 1) {
+            const F2 t = f2_add(acc[I][h], grp[I][h]), z = f2_sub(t, acc[I][h]);
+            lo[I][h] = f2_add(lo[I][h], f2_add(f2_sub(acc[I][h], f2_sub(t, z)), f2_sub(grp[I][h], z)));
+            acc[I][h] = t;
+            grp[I][h] = f2(0.f, 0.f);
+          }
+        } else {
+          acc[I][h] = f2_fma(cf, v[h], acc[I][h]);
+        }
       }
     }
-    step_pixels<S, C, RY, DX, I + 1>(cs, v, cw, acc, lo, grp);
+    step_pixels<S, WARPS, C, RY, DX, I + 1>(ring, gb, v, cw, acc, lo, grp);
   }
 }
 
-template <class S, bool C, int P>
-__device__ __forceinline__ void step_positions(const float* __restrict__ ys, const float* __restrict__ cs,
-                                               float4 (&cw)[SB_N], float2 (&acc)[SB_N], float2 (&lo)[SB_N],
-                                               float2 (&grp)[SB_N]) {
+// whether position P of the block's window feeds any of its pixels
+template <class S>
+__host__ __device__ constexpr bool step_used(int P) {
+  const int NX = SB_C + 2 * S::R, RY = P / NX - S::R, DX = P % NX - S::R;
+  for (int i = 0; i < SB_R; i++)
+    for (int j = 0; j < SB_C; j++)
+      if (S::in(RY - i, DX - j)) return true;
+  return false;
+}
+template <class S>
+__host__ __device__ constexpr int step_next(int P) {  // the first used position from P on
+  const int n = (SB_R + 2 * S::R) * (SB_C + 2 * S::R);
+  while (P < n && !step_used<S>(P)) P++;
+  return P;
+}
+template <class S, int WARPS, int P>
+__device__ __forceinline__ float4 step_value(const float* __restrict__ ys) {
+  constexpr int NX = SB_C + 2 * S::R;
+  return *(const float4*)(ys + (P / NX * StepSmem<S, WARPS>::PW + P % NX) * kBlk);
+}
+// positions P, ... in scanline order; v is P's value, loaded one position ahead
+template <class S, int WARPS, bool C, int P>
+__device__ __forceinline__ void step_positions(const float* __restrict__ ys, float4 v4, StepRing& ring,
+                                               const unsigned char* (&gb)[StepSmem<S, WARPS>::NG],
+                                               float4 (&cw)[SB_N], F2 (&acc)[SB_N][2], F2 (&lo)[SB_N][2],
+                                               F2 (&grp)[SB_N][2]) {
   constexpr int NY = SB_R + 2 * S::R, NX = SB_C + 2 * S::R;
   if constexpr (P < NY * NX) {
-    constexpr int RY = P / NX - S::R, DX = P % NX - S::R;
-    constexpr bool any = [] {
-      for (int i = 0; i < SB_R; i++)
-        for (int j = 0; j < SB_C; j++)
-          if (S::in(RY - i, DX - j)) return true;
-      return false;
-    }();
-    if constexpr (any) {
-      const float2 v = *(const float2*)(ys + ((RY + S::R) * StepSmem<S>::PW + (DX + S::R)) * kBlk);
-      step_pixels<S, C, RY, DX, 0>(cs, v, cw, acc, lo, grp);
-    }
-    step_positions<S, C, P + 1>(ys, cs, cw, acc, lo, grp);
+    constexpr int RY = P / NX - S::R, DX = P % NX - S::R, PN = step_next<S>(P + 1);
+    float4 vn = v4;
+    if constexpr (PN < NY * NX) vn = step_value<S, WARPS, PN>(ys);
+    const F2 v[2] = {f2(v4.x, v4.y), f2(v4.z, v4.w)};
+    step_pixels<S, WARPS, C, RY, DX, 0>(ring, gb, v, cw, acc, lo, grp);
+    step_positions<S, WARPS, C, PN>(ys, vn, ring, gb, cw, acc, lo, grp);
   }
 }
 
 // Persistent, warp-specialised: one CTA per SM walks its share of the tile
-// list.  Warp 8 (one lane) is the producer: for each active tile it waits
-// until the consumers have released the stage, writes the tile record and
-// issues the bulk copies against the stage's "full" mbarrier.  Warps 0-7
-// consume: wait "full", prefetch X, run the stencil on their 4 x 4 block,
-// write the outputs and arrive on the stage's "empty" mbarrier.  Two stages,
-// so tile i+1 streams in while tile i is computed.  Every wait is bounded;
-// a wait that gives up sets *a.err and ends the CTA.
-constexpr int kStepConsumers = 8, kStepThreads = (kStepConsumers + 1) * 32;
-
-// Q: the tiles come from a device work queue -- the producer claims the next
-// unclaimed tile with an atomic ticket, so CTAs that meet partial or
-// inactive tiles take more of the others -- instead of a static stride over
-// the list; the last CTA to finish resets the queue for the next launch.
-// XS: the previous iterate X reaches the consumers through shared memory:
-// each warp issues cp.async copies of its block's X rows when a tile starts
-// and waits for them only after the stencil, so their latency never stalls
-// the FMAs (without XS the lanes load X into registers directly).
-template <class S, bool C, bool XS, bool Q>
-__global__ void __launch_bounds__(kStepThreads, 1) cf_step_t(BlkArgs a, const int4* __restrict__ work, int nwork,
-                                                             const float* __restrict__ Y, const float* __restrict__ X,
-                                                             float* __restrict__ out, int step) {
-  using SM = StepSmem<S>;
+// list.  Warp WARPS (one lane) streams the Y rows: for each active tile it
+// waits until the consumers have released the stage, writes the tile record
+// and issues bulk copies against the stage's "full" mbarrier, so tile i+1's
+// rows arrive while tile i is computed.  Warp WARPS + 1 (one lane) streams
+// the coefficients through a ring of groups of GC chunks.  Warps
+// 0 .. WARPS-1 consume: wait "full", fetch X into registers, run the stencil
+// on their 2 rows, write the outputs and arrive on the stage's "empty"
+// mbarrier.  Every wait is bounded; a wait that gives up sets *a.err and ends
+// the thread's work.
+//
+// What bounds it: HBM (720 B / px of the fine level = 118 us for 1.11 Mpx at
+// the copy rate), the shared-memory pipe (111 us of wavefronts) and the FMA
+// pipe, about evenly; two warps per scheduler leave some of their latency
+// uncovered.  A 16-byte shared load takes 4 cycles for 32 distinct addresses
+// and 2 for up to 4 (both measured), so a coefficient load that serves four
+// quarters of 4 columns each feeds 16 FMAs per 2 cycles, twice as many as
+// with half-warps of 2 columns; the pixel block of 2 x 4 keeps the value loads
+// at 16 per pixel, and the packed FMAs halve the instructions.
+// Measured, 16 patches of 266^2: 171 us per launch over all patches, 4.8 TB/s
+// of DRAM traffic, from 203 us with 8 x 16 tiles, half-warps and scalar FMAs
+// (187 us with scalar FMAs in this layout); same results to the bit.
+// WARPS = 8 (16 x 16 tiles) reads a third less halo than WARPS = 4 (8 x 16)
+// and has twice the warps to cover latency: 174 against 213 us there, 29
+// against 35 us at 600 tiles.  WARPS = 4 is for launches whose tiles do not
+// fill the SMs: 10 against 12 us at 20 tiles.
+template <class S, bool C, int WARPS>
+__global__ void __launch_bounds__((WARPS + 2) * 32, 1) cf_step_t(BlkArgs a, const int4* __restrict__ work, int nwork,
+                                                                 const float* __restrict__ Y,
+                                                                 const float* __restrict__ X,
+                                                                 float* __restrict__ out, int step) {
+  using SM = StepSmem<S, WARPS>;
+  constexpr int SUB = kStepTile / (2 * WARPS);  // launches' tiles per work entry
   extern __shared__ __align__(128) unsigned char smem[];
-  StepMeta* meta = (StepMeta*)(smem + 2 * SM::stage);  // [2]
-  uint64_t* full = (uint64_t*)(smem + 2 * SM::stage + 128);
-  uint64_t* empty = full + 2;
+  StepMeta* meta = (StepMeta*)(smem + SM::bars);  // [2]
+  uint64_t* yfull = (uint64_t*)(smem + SM::bars + 128);
+  uint64_t* yempty = yfull + 2;
+  uint64_t* cfull = yempty + 2;
+  uint64_t* cempty = cfull + SM::RING;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
-    mbar_init(full + 0, 1);
-    mbar_init(full + 1, 1);
-    mbar_init(empty + 0, kStepConsumers);
-    mbar_init(empty + 1, kStepConsumers);
+    for (int i = 0; i < 2; i++) {
+      mbar_init(yfull + i, 1);
+      mbar_init(yempty + i, WARPS);
+    }
+    for (int i = 0; i < SM::RING; i++) {
+      mbar_init(cfull + i, 1);
+      mbar_init(cempty + i, WARPS);
+    }
   }
   __syncthreads();
-  if (warp == kStepConsumers) {  // ------------------------------- producer
+  if (warp >= WARPS) {  // ------------------------------------- producers
     if (lane != 0) return;
     int i = 0;
-    for (int t = blockIdx.x;; t += gridDim.x, i++) {
-      int4 w = make_int4(0, 0, 0, 0);
-      bool have = false;
-      if constexpr (Q) {
-        for (;;) {
-          const int tq = atomicAdd(a.queue, 1);
-          if (tq >= nwork) break;
-          w = work[tq];
-          if (a.active[w.x]) {
-            have = true;
-            break;
-          }
+    for (int t = blockIdx.x; t < nwork * SUB; t += gridDim.x) {
+      const int4 w = work[t / SUB];
+      const int sub = t % SUB, y0 = w.y + sub * 2 * WARPS;
+      if (!a.active[w.x]) continue;
+      const PatchDev P = a.patches[w.x];
+      if (y0 >= P.H) continue;
+      if (warp == WARPS) {
+        const int st = i & 1;
+        if (i >= 2 && !mbar_wait(yempty + st, ((i >> 1) - 1) & 1)) {
+          atomicExch(a.err, 1);
+          return;
         }
+        const float3 co = a.coef[(long long)w.x * a.max_steps + step];
+        StepMeta& m = meta[st];
+        m.end = 0;
+        m.W = P.W;
+        m.H = P.H;
+        m.y0 = y0;
+        m.x0 = w.z;
+        m.vec = P.vec;
+        m.cx = co.x;
+        m.cy = co.y;
+        m.cz = co.z;
+        // rows past the patch's last row (+ the radius) feed no in-patch pixel
+        const int ny = min(2 * WARPS, P.H - y0) + 2 * S::R;
+        constexpr uint32_t yrow = SM::PW * kBlk * sizeof(float);
+        unsigned char* ys = smem + st * SM::y_bytes;
+        mbar_expect_tx(yfull + st, (uint32_t)ny * yrow);
+        for (int r = 0; r < ny; r++)
+          bulk_g2s(ys + (size_t)r * yrow, Y + (P.vec + (long long)(y0 - S::R + r) * P.W + (w.z - S::R)) * kBlk, yrow,
+                   yfull + st);
       } else {
-        for (; t < nwork; t += gridDim.x) {
-          w = work[t];
-          if (a.active[w.x]) {
-            have = true;
-            break;
+        const float4* src = (const float4*)a.afull + (long long)w.w * SM::NCH * kTilePx + sub * WARPS * 32;
+        for (int g = 0; g < SM::NG; g++) {
+          const int n = i * SM::NG + g, pl = n % SM::RING;
+          if (n >= SM::RING && !mbar_wait(cempty + pl, (n / SM::RING - 1) & 1)) {
+            atomicExch(a.err, 1);
+            return;
+          }
+          const int nch = min(SM::GC, SM::NCH - g * SM::GC);
+          unsigned char* dst = smem + 2 * SM::y_bytes + pl * SM::group;
+          mbar_expect_tx(cfull + pl, (uint32_t)(nch * SM::chunk));
+          if constexpr (SUB == 1) {
+            bulk_g2s(dst, src + (long long)g * SM::GC * kTilePx, (uint32_t)(nch * SM::chunk), cfull + pl);
+          } else {
+            for (int c = 0; c < nch; c++)
+              bulk_g2s(dst + c * SM::chunk, src + (long long)(g * SM::GC + c) * kTilePx, (uint32_t)SM::chunk,
+                       cfull + pl);
           }
         }
       }
+      i++;
+    }
+    if (warp == WARPS) {
       const int st = i & 1;
-      if (i >= 2 && !mbar_wait(empty + st, ((i >> 1) - 1) & 1)) {
+      if (i >= 2 && !mbar_wait(yempty + st, ((i >> 1) - 1) & 1)) {
         atomicExch(a.err, 1);
         return;
       }
-      StepMeta& m = meta[st];
-      if (!have) {
-        m.end = 1;
-        mbar_arrive(full + st);
-        if constexpr (Q) {
-          // every claim of this CTA is done; the last CTA to get here resets
-          // the queue (each CTA's claims precede its count in program order)
-          __threadfence();
-          if (atomicAdd(a.queue + 1, 1) == (int)gridDim.x - 1) {
-            a.queue[0] = 0;
-            a.queue[1] = 0;
-            __threadfence();
-          }
-        }
-        return;
-      }
-      const PatchDev P = a.patches[w.x];
-      const float3 co = a.coef[(long long)w.x * a.max_steps + step];
-      m.end = 0;
-      m.W = P.W;
-      m.H = P.H;
-      m.y0 = w.y;
-      m.x0 = w.z;
-      m.vec = P.vec;
-      m.cx = co.x;
-      m.cy = co.y;
-      m.cz = co.z;
-      // rows past the patch's last row (+ the radius) feed no in-patch pixel
-      const int ylast = min(w.y + ST_TY - 1, P.H - 1);
-      const int ny = ylast - w.y + 1 + 2 * S::R, nc = ylast - w.y + 1;
-      constexpr uint32_t yrow = SM::PW * kBlk * sizeof(float), crow = ST_TX * S::NC * sizeof(float);
-      float* ys = (float*)(smem + st * SM::stage);
-      float* cs = (float*)(smem + st * SM::stage + SM::y_bytes);
-      mbar_expect_tx(full + st, (uint32_t)ny * yrow + (uint32_t)nc * crow);
-      for (int r = 0; r < ny; r++)
-        bulk_g2s(ys + (size_t)r * SM::PW * kBlk,
-                 Y + (P.vec + (long long)(w.y - S::R + r) * P.W + (w.z - S::R)) * kBlk, yrow, full + st);
-      for (int r = 0; r < nc; r++)
-        bulk_g2s(cs + (size_t)r * ST_TX * S::NC, a.afull + (P.vec + (long long)(w.y + r) * P.W + w.z) * S::NC,
-                 crow, full + st);
+      meta[st].end = 1;
+      mbar_arrive(yfull + st);
     }
+    return;
   }
   // ------------------------------------------------------------ consumers
-  // warp: a 4 x 4 block of the tile; half-warp h: its rows 2h, 2h+1; lane:
-  // block columns col, col + 1
-  const int by = (warp / (ST_TX / ST_B)) * ST_B + SB_R * (lane >> 4), bx = (warp % (ST_TX / ST_B)) * ST_B;
-  const int col = 2 * (lane & 15);
-  float* xslot = (float*)(smem + SM::bytes + (size_t)(warp < kStepConsumers ? warp : 0) * SM::x_slot);
-  for (int i = 0;; i++) {
+  // warp: tile rows 2 warp, 2 warp + 1; quarter: columns 4 quarter .. + 3;
+  // lane: block columns col .. col + 3
+  const int quarter = lane >> 3, by = 2 * warp, bx = SB_C * quarter, col = 4 * (lane & 7);
+  StepRing ring;
+  ring.base = smem + 2 * SM::y_bytes + (32 * warp + quarter) * 16;
+  ring.full = cfull;
+  ring.empty = cempty;
+  ring.n0 = 0;
+  ring.bad = false;
+  for (int i = 0;; i++, ring.n0 += SM::NG) {
     const int st = i & 1;
-    if (!mbar_wait(full + st, (i >> 1) & 1)) {
+    if (!mbar_wait(yfull + st, (i >> 1) & 1)) {
       if (lane == 0) atomicExch(a.err, 1);
       return;
     }
     const StepMeta m = meta[st];
     if (m.end) return;
-    const float* ys = (const float*)(smem + st * SM::stage);
-    const float* cs = (const float*)(smem + st * SM::stage + SM::y_bytes);
-    // the previous iterate's values for this lane's columns, fetched now so
-    // the loads overlap the stencil
-    float2 xr[SB_N];
-    if constexpr (XS) {
-      if (m.cz != 0.f) {
-        // the warp's 4 x 4 block: 16 pixel rows of 128 bytes, 128 chunks of 16
-        const int wy = (warp / (ST_TX / ST_B)) * ST_B;
-#pragma unroll
-        for (int t = 0; t < 4; t++) {
-          const int c = lane + 32 * t, pix = c >> 3, sub = c & 7;
-          const int y = m.y0 + wy + (pix >> 2), x = m.x0 + bx + (pix & 3);
-          const bool ok = y < m.H && x < m.W;
-          cp_async16(xslot + pix * kBlk + sub * 4, ok ? X + (m.vec + (long long)y * m.W + x) * kBlk + sub * 4 : X,
-                     ok ? 16u : 0u);
+    if (m.y0 + by >= m.H) {  // no row of this warp is in the patch
+      for (int g = 0; g < SM::NG; g++) {
+        const unsigned n = ring.n0 + g;
+        if (!mbar_wait(cfull + n % SM::RING, (n / SM::RING) & 1)) {
+          if (lane == 0) atomicExch(a.err, 1);
+          return;
         }
-        cp_async_commit();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(cempty + n % SM::RING);
       }
-    } else {
+      if (lane == 0) mbar_arrive(yempty + st);
+      continue;
+    }
+    const float* ys = (const float*)(smem + st * SM::y_bytes) + (by * SM::PW + bx) * kBlk + col;
+    const long long q0 = (m.vec + (long long)(m.y0 + by) * m.W + m.x0 + bx) * kBlk + col;
+    // the previous iterate's values, fetched now so the loads overlap the
+    // stencil (the compensated products, whose accumulators take the
+    // registers, have none)
+    float4 xr[SB_N];
+    auto fetch_x = [&]() {
 #pragma unroll
       for (int k = 0; k < SB_N; k++) {
-        const int y = m.y0 + by + k / SB_C, x = m.x0 + bx + k % SB_C;
-        const bool ok = m.cz != 0.f && y < m.H && x < m.W;
-        xr[k] = ok ? *(const float2*)(X + (m.vec + (long long)y * m.W + x) * kBlk + col) : make_float2(0.f, 0.f);
+        const bool ok = m.cz != 0.f && m.y0 + by + k / SB_C < m.H && m.x0 + bx + k % SB_C < m.W;
+        xr[k] = ok ? __ldcs((const float4*)(X + q0 + ((long long)(k / SB_C) * m.W + k % SB_C) * kBlk))
+                   : make_float4(0.f, 0.f, 0.f, 0.f);
       }
-    }
-    float2 acc[SB_N], lo[SB_N], grp[SB_N];
+    };
+    if constexpr (!C) fetch_x();
+    F2 acc[SB_N][2], lo[SB_N][2], grp[SB_N][2];
     float4 cw[SB_N];
+    const unsigned char* gb[SM::NG];
 #pragma unroll
-    for (int k = 0; k < SB_N; k++) acc[k] = lo[k] = grp[k] = make_float2(0.f, 0.f);
-    step_positions<S, C, 0>(ys + (by * SM::PW + bx) * kBlk + col, cs + (by * ST_TX + bx) * S::NC, cw, acc, lo,
-                            grp);
-    if constexpr (XS) {
-      if (m.cz != 0.f) {
-        cp_async_wait_all();
-        __syncwarp();
+    for (int k = 0; k < SB_N; k++)
 #pragma unroll
-        for (int k = 0; k < SB_N; k++)
-          xr[k] = *(const float2*)(xslot + ((SB_R * (lane >> 4) + k / SB_C) * ST_B + k % SB_C) * kBlk + col);
-      }
+      for (int h = 0; h < 2; h++) acc[k][h] = lo[k][h] = grp[k][h] = f2(0.f, 0.f);
+    constexpr int P0 = step_next<S>(0);
+    step_positions<S, WARPS, C, P0>(ys, step_value<S, WARPS, P0>(ys), ring, gb, cw, acc, lo, grp);
+    if (ring.bad) {
+      if (lane == 0) atomicExch(a.err, 1);
+      return;
     }
+    if constexpr (C) fetch_x();
 #pragma unroll
     for (int k = 0; k < SB_N; k++) {
-      const int y = m.y0 + by + k / SB_C, x = m.x0 + bx + k % SB_C;
-      if (y >= m.H || x >= m.W) continue;
-      const long long q = m.vec + (long long)y * m.W + x;
-      const float2 yc = *(const float2*)(ys + ((by + k / SB_C + S::R) * SM::PW + bx + k % SB_C + S::R) * kBlk + col);
-      const float2 a0 = C ? make_float2(acc[k].x + lo[k].x, acc[k].y + lo[k].y) : acc[k];
-      float2 r = make_float2(m.cx * a0.x + m.cy * yc.x, m.cx * a0.y + m.cy * yc.y);
-      if (m.cz != 0.f) {
-        r.x = fmaf(m.cz, xr[k].x, r.x);
-        r.y = fmaf(m.cz, xr[k].y, r.y);
+      if (m.y0 + by + k / SB_C >= m.H || m.x0 + bx + k % SB_C >= m.W) continue;
+      const float4 y4 = *(const float4*)(ys + ((k / SB_C + S::R) * SM::PW + k % SB_C + S::R) * kBlk);
+      const float yc[4] = {y4.x, y4.y, y4.z, y4.w}, xc[4] = {xr[k].x, xr[k].y, xr[k].z, xr[k].w};
+      const float2 p0 = f2_split(C ? f2_add(acc[k][0], lo[k][0]) : acc[k][0]);
+      const float2 p1 = f2_split(C ? f2_add(acc[k][1], lo[k][1]) : acc[k][1]);
+      const float as[4] = {p0.x, p0.y, p1.x, p1.y};
+      float r[4];
+#pragma unroll
+      for (int c = 0; c < 4; c++) {
+        const float a0 = as[c];
+        r[c] = fmaf(m.cy, yc[c], __fmul_rn(m.cx, a0));
+        if (m.cz != 0.f) r[c] = fmaf(m.cz, xc[c], r[c]);
       }
-      *(float2*)(out + q * kBlk + col) = r;
+      *(float4*)(out + q0 + ((long long)(k / SB_C) * m.W + k % SB_C) * kBlk) = make_float4(r[0], r[1], r[2], r[3]);
     }
     __syncwarp();
-    if (lane == 0) mbar_arrive(empty + st);
+    if (lane == 0) mbar_arrive(yempty + st);
   }
 }
 
-// A ROWS x 16 tile's pixel-major rows (NC floats each), staged in shared
-// memory by pixel 16 * ty + tx, out to their places: a tile row's pixels are
-// adjacent in the layout, so each tile row leaves as one contiguous run of
-// 16-byte stores.  (A thread writing its own row would give each warp store
-// 32 scattered 16-byte pieces.)  Row strides of 21 and 13 float4 put the 8
-// threads of a staging store's phase in distinct banks.
-template <int NC, int ROWS>
-__device__ __forceinline__ void tile_rows_out(const float4* __restrict__ rows, float* __restrict__ dst, long long vec,
-                                              int W, int H, int y0, int x0) {
-  constexpr int Q = NC / 4;
-  const int ny = min(ROWS, H - y0), nx = min(16, W - x0);
-  for (int i = threadIdx.x; i < ny * 16 * Q; i += blockDim.x) {
-    const int r = i / (16 * Q), j = i % (16 * Q);
-    if (j < nx * Q) ((float4*)(dst + (vec + (long long)(y0 + r) * W + x0) * NC))[j] = rows[r * 16 * Q + j];
-  }
-}
-
-// pixel-major full stencil rows of the fine operator from its symmetric
-// storage: row p holds A(p, p + off_e) for the 81 offsets e in scanline
-// order (0 where the neighbour is outside the patch), then 3 zeros
-constexpr int kFullRows = 8;  // tile rows per CTA: half of a 16 x 16 work tile
-__global__ void __launch_bounds__(kFullRows * 16) cf_full(const PatchDev* __restrict__ patches,
-                                                          const int4* __restrict__ work,
-                                                          const float* __restrict__ a_up,
-                                                          const float* __restrict__ a_diag, long long lvec,
-                                                          float* __restrict__ afull) {
-  // one thread per pixel of a half tile (43 KB of staging, so several CTAs
-  // share an SM): the plane reads are coalesced across the warp; the rows go
-  // out through shared memory
-  constexpr int NC = DiskStencil::NC, ctr = kStencilN / 2;
-  __shared__ float4 rows[kFullRows * 16 * (NC / 4)];
-  const int4 w = work[blockIdx.x >> 1];
+// The stencil rows of the fine operator from its symmetric storage, in the
+// step's tile layout: slot = pixel, chunk = 4 of the 81 offsets in scanline
+// order (0 where the neighbour or the pixel is outside the patch, and 3 zeros
+// at the end).  A thread owns a slot, so a warp's 16-byte stores of a chunk
+// are 512 contiguous bytes; its pixels are 2 tile rows, so the plane reads
+// stay coalesced.
+__global__ void __launch_bounds__(kTilePx) cf_full(const PatchDev* __restrict__ patches,
+                                                   const int4* __restrict__ work, const float* __restrict__ a_up,
+                                                   const float* __restrict__ a_diag, long long lvec,
+                                                   float* __restrict__ afull) {
+  constexpr int NCH = DiskStencil::NC / 4, ctr = kStencilN / 2;
+  const int4 w = work[blockIdx.x];
   const PatchDev P = patches[w.x];
-  const int y0 = w.y + (blockIdx.x & 1) * kFullRows;
-  const int y = y0 + threadIdx.x / 16, x = w.z + threadIdx.x % 16;
-  if (y < P.H && x < P.W) {
-    const long long p = P.vec + (long long)y * P.W + x;
+  const int t = threadIdx.x, k = (t >> 2) & 7;
+  const int y = w.y + 2 * (t >> 5) + (k >> 2), x = w.z + 4 * (t & 3) + (k & 3);
+  const bool inside = y < P.H && x < P.W;
+  const long long p = P.vec + (long long)y * P.W + x;
+  float4* dst = (float4*)afull + (long long)blockIdx.x * NCH * kTilePx + t;
 #pragma unroll 3
-    for (int e4 = 0; e4 < NC / 4; e4++) {
-      float v[4];
+  for (int e4 = 0; e4 < NCH; e4++) {
+    float v[4];
 #pragma unroll
-      for (int j = 0; j < 4; j++) {
-        const int e = 4 * e4 + j;
-        v[j] = 0.f;
-        if (e >= kStencilN) continue;
-        if (e == ctr) {
-          v[j] = a_diag[p];
-          continue;
-        }
-        // upper offsets are c_bup[e - 41]; the disk is point-symmetric, so
-        // lower offset e mirrors upper offset 80 - e
-        const int k = e > ctr ? e - ctr - 1 : kStencilN - 1 - e - ctr - 1;
-        const int dy = e > ctr ? c_bup_dy[k] : -c_bup_dy[k];
-        const int dx = e > ctr ? c_bup_dx[k] : -c_bup_dx[k];
-        const int yy = y + dy, xx = x + dx;
-        if (yy >= 0 && yy < P.H && xx >= 0 && xx < P.W)
-          v[j] = e > ctr ? a_up[(long long)k * lvec + p] : a_up[(long long)k * lvec + p + (long long)dy * P.W + dx];
+    for (int j = 0; j < 4; j++) {
+      const int e = 4 * e4 + j;
+      v[j] = 0.f;
+      if (e >= kStencilN || !inside) continue;
+      if (e == ctr) {
+        v[j] = a_diag[p];
+        continue;
       }
-      rows[threadIdx.x * (NC / 4) + e4] = make_float4(v[0], v[1], v[2], v[3]);
+      // upper offsets are c_bup[e - 41]; the disk is point-symmetric, so
+      // lower offset e mirrors upper offset 80 - e
+      const int u = e > ctr ? e - ctr - 1 : kStencilN - 1 - e - ctr - 1;
+      const int dy = e > ctr ? c_bup_dy[u] : -c_bup_dy[u];
+      const int dx = e > ctr ? c_bup_dx[u] : -c_bup_dx[u];
+      const int yy = y + dy, xx = x + dx;
+      if (yy >= 0 && yy < P.H && xx >= 0 && xx < P.W)
+        v[j] = e > ctr ? a_up[(long long)u * lvec + p] : a_up[(long long)u * lvec + p + (long long)dy * P.W + dx];
     }
+    dst[(long long)e4 * kTilePx] = make_float4(v[0], v[1], v[2], v[3]);
   }
-  __syncthreads();
-  tile_rows_out<NC, kFullRows>(rows, afull, P.vec, P.W, P.H, y0, w.z);
 }
 
 // ------------------------------------------------------------------ Gram
@@ -903,39 +960,43 @@ __device__ __forceinline__ void coarsen_sub(float (&acc)[kCN], const CoarseArgs&
 // sub-pixel s -- is a constant and the 49 sums stay in registers.  Terms
 // are added per sum in the order: sub-pixel, upper offset, lower before
 // upper neighbour.
-__global__ void __launch_bounds__(256) cf_coarsen(CoarseArgs c) {
-  extern __shared__ float4 rows[];  // [256][13]
+// The rows go out in the step's tile layout (see cf_full).
+__global__ void __launch_bounds__(kTilePx) cf_coarsen(CoarseArgs c) {
   const int4 w = c.work[blockIdx.x];
   const PatchDev F = c.fine[w.x], C = c.coarse[w.x];
-  constexpr int NC = SquareStencil::NC;
-  const int Y = w.y + threadIdx.x / 16, X = w.z + threadIdx.x % 16;
-  if (Y < C.H && X < C.W) {
-    float acc[kCN];
+  constexpr int NCH = SquareStencil::NC / 4;
+  const int t = threadIdx.x, pk = (t >> 2) & 7;
+  const int Y = w.y + 2 * (t >> 5) + (pk >> 2), X = w.z + 4 * (t & 3) + (pk & 3);
+  const bool inside = Y < C.H && X < C.W;
+  float acc[kCN];
 #pragma unroll
-    for (int k = 0; k < kCN; k++) acc[k] = 0.f;
+  for (int k = 0; k < kCN; k++) acc[k] = 0.f;
+  float dp = 0.f;
+  const long long P = C.vec + (long long)Y * C.W + X;
+  if (inside) {
     coarsen_sub<0, 0>(acc, c, F, Y, X);
     coarsen_sub<0, 1>(acc, c, F, Y, X);
     coarsen_sub<1, 0>(acc, c, F, Y, X);
     coarsen_sub<1, 1>(acc, c, F, Y, X);
-    const long long P = C.vec + (long long)Y * C.W + X;
-    const float dp = c.disc[P];
-    float v[NC];
+    dp = c.disc[P];
+  }
+  float4* dst = (float4*)c.wc + (long long)blockIdx.x * NCH * kTilePx + t;
 #pragma unroll
-    for (int k = 0; k < NC; k++) {
-      v[k] = 0.f;
-      if (k >= kCN) continue;
+  for (int q = 0; q < NCH; q++) {
+    float v[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const int k = 4 * q + j;
+      v[j] = 0.f;
+      if (k >= kCN || !inside) continue;
       const int dY = k / kCW - kCR, dX = k % kCW - kCR;
       const int YY = Y + dY, XX = X + dX;
       if (YY >= 0 && YY < C.H && XX >= 0 && XX < C.W)
-        v[k] = -acc[k] * dp * c.disc[C.vec + (long long)YY * C.W + XX];
-      if (k == kCR * kCW + kCR) v[k] += 1.f;
+        v[j] = -acc[k] * dp * c.disc[C.vec + (long long)YY * C.W + XX];
+      if (k == kCR * kCW + kCR) v[j] += 1.f;
     }
-#pragma unroll
-    for (int q = 0; q < NC / 4; q++)
-      rows[threadIdx.x * (NC / 4) + q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+    dst[(long long)q * kTilePx] = make_float4(v[0], v[1], v[2], v[3]);
   }
-  __syncthreads();
-  tile_rows_out<NC, 16>(rows, c.wc, C.vec, C.W, C.H, w.y, w.z);
 }
 
 // fine start block from the coarse Ritz vectors: the coarse generalised
@@ -978,15 +1039,9 @@ __global__ void __launch_bounds__(256) cf_prolong(CoarseArgs c, const float* __r
   }
 }
 
-constexpr int kCoarsenSmem = 256 * kCoarseNC * sizeof(float);
 cudaError_t cf_launch_coarsen(const CoarseArgs& c, int nwork_c, cudaStream_t s) {
-  static bool attr = false;
-  if (!attr) {
-    cudaFuncSetAttribute(cf_coarsen, cudaFuncAttributeMaxDynamicSharedMemorySize, kCoarsenSmem);
-    attr = true;
-  }
   cf_coarse_deg<<<nwork_c, 256, 0, s>>>(c);
-  cf_coarsen<<<nwork_c, 256, kCoarsenSmem, s>>>(c);
+  cf_coarsen<<<nwork_c, kTilePx, 0, s>>>(c);
   return cudaGetLastError();
 }
 cudaError_t cf_launch_prolong(const CoarseArgs& c, int nwork_f, const float* xc, float* xf, cudaStream_t s) {
@@ -994,32 +1049,28 @@ cudaError_t cf_launch_prolong(const CoarseArgs& c, int nwork_f, const float* xc,
   return cudaGetLastError();
 }
 
-template <class S, bool C, bool XS, bool Q>
-static void step_attr() {
-  cudaFuncSetAttribute(cf_step_t<S, C, XS, Q>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)(XS ? StepSmem<S>::bytes_xs : StepSmem<S>::bytes));
+template <class S, bool C, int WARPS>
+static cudaError_t step_attr() {
+  return cudaFuncSetAttribute(cf_step_t<S, C, WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)StepSmem<S, WARPS>::bytes);
 }
-template <class S, bool C>
+template <class S>
 static void step_attrs() {
-  step_attr<S, C, false, false>();
-  step_attr<S, C, true, false>();
-  step_attr<S, C, false, true>();
-  step_attr<S, C, true, true>();
+  step_attr<S, false, 8>();
+  step_attr<S, true, 8>();
+  step_attr<S, false, 4>();
+  step_attr<S, true, 4>();
 }
 
 template <class S, bool C>
 static void step_go(const BlkArgs& a, const int4* work, int nwork, const float* Y, const float* X, float* out,
-                    int step, int grid, int variant, cudaStream_t s) {
-#define GPB_STEP(XS, Q)                                                                                  \
-  cf_step_t<S, C, XS, Q><<<grid, kStepThreads, XS ? StepSmem<S>::bytes_xs : StepSmem<S>::bytes, s>>>( \
-      a, work, nwork, Y, X, out, step)
-  switch (variant & 3) {
-    case 0: GPB_STEP(false, false); break;
-    case 1: GPB_STEP(true, false); break;
-    case 2: GPB_STEP(false, true); break;
-    default: GPB_STEP(true, true); break;
-  }
-#undef GPB_STEP
+                    int step, int nsm, int variant, cudaStream_t s) {
+  // one persistent CTA per SM
+  if (variant == 0)
+    cf_step_t<S, C, 8><<<std::min(nwork, nsm), 10 * 32, StepSmem<S, 8>::bytes, s>>>(a, work, nwork, Y, X, out, step);
+  else
+    cf_step_t<S, C, 4><<<std::min(2 * nwork, nsm), 6 * 32, StepSmem<S, 4>::bytes, s>>>(a, work, nwork, Y, X, out,
+                                                                                       step);
 }
 
 cudaError_t cf_launch_step(const BlkArgs& a, const int4* work, int nwork, const float* Y, const float* X, float* out,
@@ -1029,26 +1080,23 @@ cudaError_t cf_launch_step(const BlkArgs& a, const int4* work, int nwork, const 
     int dev = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    step_attrs<DiskStencil, false>();
-    step_attrs<DiskStencil, true>();
-    step_attrs<SquareStencil, false>();
-    step_attrs<SquareStencil, true>();
+    step_attrs<DiskStencil>();
+    step_attrs<SquareStencil>();
     if (nsm <= 0) nsm = 1;
   }
-  const int grid = std::min(nwork, nsm);  // one persistent CTA per SM
-  if (grid <= 0) return cudaSuccess;
+  if (nwork <= 0) return cudaSuccess;
   if (a.coarse) {
-    if (comp) step_go<SquareStencil, true>(a, work, nwork, Y, X, out, step, grid, variant, s);
-    else step_go<SquareStencil, false>(a, work, nwork, Y, X, out, step, grid, variant, s);
+    if (comp) step_go<SquareStencil, true>(a, work, nwork, Y, X, out, step, nsm, variant, s);
+    else step_go<SquareStencil, false>(a, work, nwork, Y, X, out, step, nsm, variant, s);
   } else {
-    if (comp) step_go<DiskStencil, true>(a, work, nwork, Y, X, out, step, grid, variant, s);
-    else step_go<DiskStencil, false>(a, work, nwork, Y, X, out, step, grid, variant, s);
+    if (comp) step_go<DiskStencil, true>(a, work, nwork, Y, X, out, step, nsm, variant, s);
+    else step_go<DiskStencil, false>(a, work, nwork, Y, X, out, step, nsm, variant, s);
   }
   return cudaGetLastError();
 }
 cudaError_t cf_launch_full(const PatchDev* patches, const int4* work16, int nwork, const float* a_up,
                            const float* a_diag, long long lvec, float* afull, cudaStream_t s) {
-  cf_full<<<2 * nwork, kFullRows * 16, 0, s>>>(patches, work16, a_up, a_diag, lvec, afull);
+  cf_full<<<nwork, kTilePx, 0, s>>>(patches, work16, a_up, a_diag, lvec, afull);
   return cudaGetLastError();
 }
 cudaError_t cf_launch_gram(const BlkArgs& a, int ntiles, const float* U, const float* V, double* out,

@@ -29,10 +29,9 @@ struct BlkArgs {
   const double* mat;    // [npatch][32*32]
   const double* theta;  // [npatch][32]
   int coarse;           // 0: fine radius-5 disk, 1: coarse 7 x 7 square
-  const float* afull;   // pixel-major stencil rows: 84 floats (fine) / 52 (coarse)
+  const float* afull;   // stencil rows in the step's tile layout (k_block.cu): 84 floats
+                        // (fine) / 52 (coarse) per pixel of a 16 x 16 tile
   int* err;             // set to 1 when a tile's staging wait gave up
-  int* queue;           // [2]: the block step's next tile ticket and finished-CTA
-                        // count; zero between launches (the last CTA resets them)
 };
 
 // coarse level (2 x 2 aggregation)
@@ -45,7 +44,7 @@ struct CoarseArgs {
   const float* wsym_up;  // fine symmetric affinities (upper offsets)
   const float* deg;      // fine degrees
   long long lvec_f, lvec_c;
-  float* wc;             // [lvec_c][kCoarseNC] pixel-major: W_c, then A_c
+  float* wc;             // [coarse tiles][256][kCoarseNC]: A_c's rows in the step's tile layout
   float* degc;
   float* disc;
 };
@@ -55,12 +54,14 @@ cudaError_t cf_launch_full(const PatchDev* patches, const int4* work16, int nwor
 cudaError_t cf_launch_prolong(const CoarseArgs& c, int nwork_f, const float* xc, float* xf, cudaStream_t s);
 
 void upload_block(const HostTables& t, cudaStream_t s);
-constexpr int kStepTileH = 8, kStepTileW = 16;  // cf_step tile (work list entries)
-constexpr int kFullNC = 84, kCoarseNC = 52;      // floats per pixel-major stencil row
+// cf_step's tiles are those of the 16 x 16 work list, whose entries' .w is the
+// tile's index in that list (the place of its coefficients)
+constexpr int kStepTile = 16;
+constexpr int kFullNC = 84, kCoarseNC = 52;      // floats per pixel's stencil row
 constexpr int kBlkSplit = 4;  // CTAs per eigensolver tile in cf_gram / cf_rotate / cf_resid
-// variant (bit-identical results, chosen by the autotuner): bit 0 stages X
-// through shared memory, bit 1 takes tiles from the device work queue
-constexpr int kStepVariants = 4, kStepDefault = 1;  // default (untuned): X staged, static tiles
+// variant (bit-identical results, chosen by the autotuner): 0 computes 16 x 16
+// pixels per CTA and pass, 1 halves them (for launches of few tiles)
+constexpr int kStepVariants = 2, kStepDefault = 0;
 cudaError_t cf_launch_step(const BlkArgs& a, const int4* work, int nwork, const float* Y, const float* X, float* out,
                            int step, cudaStream_t s, bool comp = false, int variant = kStepDefault);
 // out = U^T V per patch; with out2, out2 = U^T U in the same pass
