@@ -25,6 +25,7 @@
 #include <algorithm>
 #include <stdlib.h>
 
+#include "f32x2.h"
 #include "gpb_internal.h"
 #include "k_block.h"
 #include "k_eig.h"
@@ -175,39 +176,6 @@ __device__ __forceinline__ float f4get(const float4& v) {
   else if constexpr (K == 1) return v.y;
   else if constexpr (K == 2) return v.z;
   else return v.w;
-}
-
-// Pairs of FP32 values for the packed f32x2 instructions: each half is one
-// correctly rounded operation, so results equal the scalar ones; an
-// instruction does two, and the three-register FMA runs at 0.29 cycles per
-// value against 0.34 (measured per warp and SM).
-struct F2 {
-  uint64_t v;
-};
-__device__ __forceinline__ F2 f2(float x, float y) {
-  F2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(x), "f"(y));
-  return r;
-}
-__device__ __forceinline__ float2 f2_split(F2 a) {
-  float2 r;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a.v));
-  return r;
-}
-__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
-  F2 r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
-  return r;
-}
-__device__ __forceinline__ F2 f2_add(F2 a, F2 b) {
-  F2 r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
-  return r;
-}
-__device__ __forceinline__ F2 f2_sub(F2 a, F2 b) {
-  F2 r;
-  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
-  return r;
 }
 
 // The coefficient ring as a consumer warp sees it.  Group g of a tile is

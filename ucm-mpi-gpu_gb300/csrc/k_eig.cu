@@ -26,6 +26,7 @@
 
 #include "gpb_internal.h"
 #include "kernels.h"
+#include "f32x2.h"
 #include "k_eig.h"
 
 namespace gpb {
@@ -54,6 +55,16 @@ __device__ __forceinline__ void ff_add_prod(float& hi, float& lo, float a, float
   const float e = (hi - (s - z)) + (p - z);
   hi = s;
   lo += e + pe;
+}
+// the same for two pixels at once
+__device__ __forceinline__ void ff_add_prod2(F2& hi, F2& lo, F2 a, F2 b) {
+  const F2 p = f2_mul(a, b);
+  const F2 pe = f2_fma(a, b, f2_neg(p));
+  const F2 s = f2_add(hi, p);
+  const F2 z = f2_sub(s, hi);
+  const F2 e = f2_add(f2_sub(hi, f2_sub(s, z)), f2_sub(p, z));
+  hi = s;
+  lo = f2_add(lo, f2_add(e, pe));
 }
 __device__ __forceinline__ void ff_add(float& hi, float& lo, float bhi, float blo) {
   const float s = hi + bhi;
@@ -100,22 +111,67 @@ __device__ __forceinline__ void cta_partials(const float2* sred, int nvals, doub
     part_row[i] = (double)hi + (double)lo;
   }
 }
-// sum of one value over the CTAs of a patch, one warp, lanes strided
-__device__ __forceinline__ double patch_sum(const double* part, int tb, int tc, int mp1, int i, int lane) {
-  double s = 0;
-  for (int b = tb + lane; b < tb + tc; b += 32) s += part[(long long)b * mp1 + i];
+// The sums of values 0 .. n-1 over the CTAs of a patch, by the patch's last
+// CTA: warp w takes the values w, w + 8, ...; each is a lane-strided FP64 sum
+// and a tree over the warp.  put(i, sum, was) on one lane per value; was =
+// before(i), loaded ahead.  This is the serial tail of every Lanczos launch
+// (one CTA works, the other SMs wait for the next launch), so all loads of a
+// warp's values are in flight together: one value at a time, each with its
+// own loads, shuffles and read-modify-write of T, took 10 of the 26 us of a
+// launch on one 321 x 481 image.
+template <class B, class F>
+__device__ __forceinline__ void patch_sums(const double* part, int tb, int tc, int mp1, int n, int warp, int lane,
+                                           B&& before, F&& put) {
+  constexpr int NI = (kMaxKrylov + 1 + kEigWarps - 1) / kEigWarps;
+  double s[NI], was[NI];
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(FULLM, s, o);
-  return s;
+  for (int u = 0; u < NI; u++) {
+    const int i = warp + u * kEigWarps;
+    s[u] = 0;
+    was[u] = i < n ? before(i) : 0.0;
+  }
+  for (int b = tb + lane; b < tb + tc; b += 32) {
+    double v[NI];
+#pragma unroll
+    for (int u = 0; u < NI; u++) {
+      const int i = warp + u * kEigWarps;
+      v[u] = i < n ? part[(long long)b * mp1 + i] : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < NI; u++)
+      if (warp + u * kEigWarps < n) s[u] += v[u];
+  }
+#pragma unroll
+  for (int u = 0; u < NI; u++) {
+    if (warp + u * kEigWarps >= n) break;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s[u] += __shfl_xor_sync(FULLM, s[u], o);
+  }
+  if (lane == 0) {
+#pragma unroll
+    for (int u = 0; u < NI; u++)
+      if (warp + u * kEigWarps < n) put(warp + u * kEigWarps, s[u], was[u]);
+  }
 }
 
 // Loads are issued in batches -- the stencil by offset for all eight pixels
 // of a thread, the basis by groups of kGrp vectors -- so each thread keeps
 // tens of independent loads in flight; every per-pixel sum still runs in the
 // same order (offsets ascending, basis vectors ascending, pixels ascending).
-// Pixels are addressed by 32-bit offsets into the vector layout, which the
-// host keeps below 2^31 entries.
+// In the passes over the basis a load's address is a CTA-uniform base (array +
+// vector + patch) plus the pixel's 32-bit byte offset in its patch (at most
+// 2^28).  The stencil keeps 64-bit sums: with four uniform bases per offset it
+// took 39 us instead of 26.
 constexpr int kGrp = 8;
+__device__ __forceinline__ float ldu(const float* base, uint32_t off) {
+  return *(const float*)((const char*)base + off);
+}
+__device__ __forceinline__ void stu(float* base, uint32_t off, float v) { *(float*)((char*)base + off) = v; }
+// the same on every lane; tells the compiler so
+__device__ __forceinline__ long long uniform(long long v) {
+  const uint32_t lo = __shfl_sync(FULLM, (uint32_t)v, 0), hi = __shfl_sync(FULLM, (uint32_t)(v >> 32), 0);
+  return (long long)(((uint64_t)hi << 32) | lo);
+}
 
 // Sums kGrp = 8 float-float values over the warp at once.  Each of the first
 // three xor rounds halves the values a lane carries (it keeps the half its
@@ -147,7 +203,7 @@ __device__ __forceinline__ float2 ff_warp_reduce8(float (&hi)[kGrp], float (&lo)
 // units of rounding times |w| (Cauchy-Schwarz over the thread partials),
 // which after the second pass leaves the basis orthogonal to ~1e-7 --
 // two orders below what the Ritz residuals need.
-__device__ __forceinline__ void basis_dots(const EigArgs& a, int j, const int (&qv)[kEigPix],
+__device__ __forceinline__ void basis_dots(const EigArgs& a, int j, long long base, const uint32_t (&qv)[kEigPix],
                                            const float (&wv)[kEigPix], const float* xj, float2* sred, int warp,
                                            int lane) {
   for (int i0 = 0; i0 <= j; i0 += kGrp) {
@@ -155,9 +211,9 @@ __device__ __forceinline__ void basis_dots(const EigArgs& a, int j, const int (&
 #pragma unroll
     for (int u = 0; u < kGrp; u++) {
       const int i = i0 + u;
-      const float* Vi = a.V + (long long)i * a.lvec;
+      const float* Vi = a.V + (long long)i * a.lvec + base;
 #pragma unroll
-      for (int r = 0; r < kEigPix; r++) vv[u][r] = (i < j || (i == j && !xj)) ? Vi[qv[r]] : (i == j ? xj[r] : 0.f);
+      for (int r = 0; r < kEigPix; r++) vv[u][r] = (i < j || (i == j && !xj)) ? ldu(Vi, qv[r]) : (i == j ? xj[r] : 0.f);
     }
     float hi[kGrp], lo[kGrp];
 #pragma unroll
@@ -178,38 +234,39 @@ __global__ void __launch_bounds__(kEigThreads, 2) ks_spmv(EigArgs a, int j, cons
   const EigTile t = a.tiles[blockIdx.x];
   if (!a.active[t.patch]) return;
   const PatchDev P = a.patches[t.patch];
+  // the FP64 root and quotient run beside the stencil; read after it
+  __shared__ float inv_s;
+  if (threadIdx.x == 0) inv_s = use_beta ? (float)(1.0 / sqrt(a.beta2[t.patch])) : 1.f;
+  const long long base = uniform(P.vec);
   __shared__ int off[kUpper];
   if (threadIdx.x < kUpper) off[threadIdx.x] = c_up_dy[threadIdx.x] * P.W + c_up_dx[threadIdx.x];
   __syncthreads();
-  __shared__ float inv_s;
-  if (threadIdx.x == 0) inv_s = use_beta ? (float)(1.0 / sqrt(a.beta2[t.patch])) : 1.f;
-  __syncthreads();
-  const float inv = inv_s;
-  const long long base = P.vec;
   // this thread's pixels; a pixel past the tile reads the tile's first one
   // (in bounds) and its results are dropped
-  int qv[kEigPix];
+  uint32_t qv[kEigPix];
   bool okv[kEigPix];
 #pragma unroll
   for (int r = 0; r < kEigPix; r++) {
     const int p = t.p0 + threadIdx.x + r * kEigThreads;
     okv[r] = p < t.p1;
-    qv[r] = (int)(base + (okv[r] ? p : t.p0));
+    qv[r] = 4u * (uint32_t)(okv[r] ? p : t.p0);
   }
   float acc[kEigPix];
 #pragma unroll
   for (int r = 0; r < kEigPix; r++) acc[r] = 0.f;
 #pragma unroll 2
   for (int k = 0; k < kUpper; k++) {
-    const float* au = a.a_up + (long long)k * a.lvec;
+    const float* au = a.a_up + (long long)k * a.lvec + base;
+    const float* xs = src + base;
     const int o = off[k];
     float cu[kEigPix], xu[kEigPix], cl[kEigPix], xl[kEigPix];
 #pragma unroll
     for (int r = 0; r < kEigPix; r++) {
-      cu[r] = au[qv[r]];
-      xu[r] = src[qv[r] + o];
-      cl[r] = au[qv[r] - o];
-      xl[r] = src[qv[r] - o];
+      const int q = (int)(qv[r] >> 2);
+      cu[r] = au[q];
+      xu[r] = xs[q + o];
+      cl[r] = au[q - o];
+      xl[r] = xs[q - o];
     }
 #pragma unroll
     for (int r = 0; r < kEigPix; r++) {
@@ -217,38 +274,39 @@ __global__ void __launch_bounds__(kEigThreads, 2) ks_spmv(EigArgs a, int j, cons
       acc[r] = fmaf(cl[r], xl[r], acc[r]);
     }
   }
+  __syncthreads();
+  const float inv = inv_s;
   float wv[kEigPix], xv[kEigPix];
 #pragma unroll
   for (int r = 0; r < kEigPix; r++) {
-    const float x = src[qv[r]] * inv;
+    const float x = ldu(src + base, qv[r]) * inv;
     xv[r] = okv[r] ? x : 0.f;
-    wv[r] = okv[r] ? fmaf(acc[r], inv, a.a_diag[qv[r]] * x) : 0.f;
+    wv[r] = okv[r] ? fmaf(acc[r], inv, ldu(a.a_diag + base, qv[r]) * x) : 0.f;
   }
-  float* Vj = a.V + (long long)j * a.lvec;
+  float* Vj = a.V + (long long)j * a.lvec + base;
 #pragma unroll
   for (int r = 0; r < kEigPix; r++) {
     if (!okv[r]) continue;
-    Vj[qv[r]] = xv[r];
-    dst[qv[r]] = wv[r];
+    stu(Vj, qv[r], xv[r]);
+    stu(dst + base, qv[r], wv[r]);
   }
   // h_i = v_i . w for i <= j
   __shared__ float2 sred[kEigWarps * kRed];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // the second pass measures what these dots missed (h2 = V^T (w - V h)),
   // and T takes h + h2
-  basis_dots(a, j, qv, wv, xv, sred, warp, lane);
+  basis_dots(a, j, base, qv, wv, xv, sred, warp, lane);
   cta_partials(sred, j + 1, a.part + (long long)blockIdx.x * a.mp1);
   if (last_cta(a.counter + t.patch, a.tile_count[t.patch])) {
     const int tb = a.tile_begin[t.patch], tc = a.tile_count[t.patch];
     double* T = a.T + (long long)t.patch * a.m * a.m;
-    for (int i = warp; i <= j; i += kEigWarps) {
-      const double s = patch_sum(a.part, tb, tc, a.mp1, i, lane);
-      if (lane == 0) {
-        a.hbuf[(long long)t.patch * a.mp1 + i] = s;
-        T[i * a.m + j] = s;
-        T[j * a.m + i] = s;
-      }
-    }
+    patch_sums(
+        a.part, tb, tc, a.mp1, j + 1, warp, lane, [](int) { return 0.0; },
+        [&](int i, double s, double) {
+          a.hbuf[(long long)t.patch * a.mp1 + i] = s;
+          T[i * a.m + j] = s;
+          T[j * a.m + i] = s;
+        });
   }
 }
 
@@ -256,13 +314,17 @@ __global__ void __launch_bounds__(kEigThreads, 2) ks_spmv(EigArgs a, int j, cons
 // MODE 1: w -= V h, then h2 = V^T w;  MODE 2: w -= V h2, then |w|^2.
 // Pass 1 subtracts a projection of about |w|'s size (the cancellation of a
 // converging step), so V h is formed in float-float and subtracted exactly;
-// pass 2's V h2 is of rounding-error size and an FMA chain holds it.
+// pass 2's V h2 is of rounding-error size and an FMA chain holds it.  Both
+// sums run on pairs of pixels (f32x2).  Measured on one 321 x 481 image, whose
+// basis stays in L2: 18.8 us (pass 1) and 9.1 us (pass 2) per launch, from
+// 26.0 and 11.0 us with scalar sums, 64-bit addresses and a one-value-at-a-
+// time tail; ks_restart 49 us from 117 us with one CTA per 2048 pixels.
 template <int MODE>
 __global__ void __launch_bounds__(kEigThreads, 2) ks_orth(EigArgs a, int j, float* __restrict__ w) {
   const EigTile t = a.tiles[blockIdx.x];
   if (!a.active[t.patch]) return;
   const PatchDev P = a.patches[t.patch];
-  const long long base = P.vec;
+  const long long base = uniform(P.vec);
   // projection coefficients as FP32 hi + lo pairs; the sum V h is formed in
   // float-float and subtracted from w before the single rounding to FP32, so
   // the cancellation of a converging step (|w - V h| << |w|) keeps its digits
@@ -273,59 +335,63 @@ __global__ void __launch_bounds__(kEigThreads, 2) ks_orth(EigArgs a, int j, floa
     hl[i] = (float)(h - (double)hs[i]);
   }
   __syncthreads();
-  int qv[kEigPix];
+  uint32_t qv[kEigPix];
   bool okv[kEigPix];
-  float wv[kEigPix], sh[kEigPix], sl[kEigPix];
+  float wv[kEigPix];
+  F2 sh[kEigPix / 2], sl[kEigPix / 2];  // pairs of pixels
 #pragma unroll
   for (int r = 0; r < kEigPix; r++) {
     const int p = t.p0 + threadIdx.x + r * kEigThreads;
     okv[r] = p < t.p1;
-    qv[r] = (int)(base + (okv[r] ? p : t.p0));
-    wv[r] = okv[r] ? w[qv[r]] : 0.f;
-    sh[r] = sl[r] = 0.f;
+    qv[r] = 4u * (uint32_t)(okv[r] ? p : t.p0);
+    wv[r] = okv[r] ? ldu(w + base, qv[r]) : 0.f;
+    sh[r / 2] = sl[r / 2] = f2(0.f, 0.f);
   }
   for (int i0 = 0; i0 <= j; i0 += kGrp) {
     float vv[kGrp][kEigPix];
 #pragma unroll
     for (int u = 0; u < kGrp; u++) {
-      const float* Vi = a.V + (long long)(i0 + u) * a.lvec;
+      const float* Vi = a.V + (long long)(i0 + u) * a.lvec + base;
 #pragma unroll
-      for (int r = 0; r < kEigPix; r++) vv[u][r] = (i0 + u <= j) ? Vi[qv[r]] : 0.f;
+      for (int r = 0; r < kEigPix; r++) vv[u][r] = (i0 + u <= j) ? ldu(Vi, qv[r]) : 0.f;
     }
 #pragma unroll
     for (int u = 0; u < kGrp; u++) {
       if (i0 + u > j) break;
-      const float h = hs[i0 + u], h2 = hl[i0 + u];
+      const F2 h = f2(hs[i0 + u], hs[i0 + u]), h2 = f2(hl[i0 + u], hl[i0 + u]);
 #pragma unroll
-      for (int r = 0; r < kEigPix; r++) {
+      for (int r = 0; r < kEigPix / 2; r++) {
+        const F2 v = f2(vv[u][2 * r], vv[u][2 * r + 1]);
         if constexpr (MODE == 1) {
-          ff_add_prod(sh[r], sl[r], h, vv[u][r]);
-          sl[r] = fmaf(h2, vv[u][r], sl[r]);
+          ff_add_prod2(sh[r], sl[r], h, v);
+          sl[r] = f2_fma(h2, v, sl[r]);
         } else {
-          sh[r] = fmaf(h, vv[u][r], sh[r]);
+          sh[r] = f2_fma(h, v, sh[r]);
         }
       }
     }
   }
 #pragma unroll
   for (int r = 0; r < kEigPix; r++) {
+    const float2 s2 = f2_split(sh[r / 2]), l2 = f2_split(sl[r / 2]);
+    const float sr = r % 2 ? s2.y : s2.x, lr = r % 2 ? l2.y : l2.x;
     if constexpr (MODE == 1) {
-      // w - (sh + sl) with the subtraction of sh exact (two-difference)
-      const float d = wv[r] - sh[r];
+      // w - (sr + lr) with the subtraction of sr exact (two-difference)
+      const float d = wv[r] - sr;
       const float z = d - wv[r];
-      const float e = (wv[r] - (d - z)) - (sh[r] + z);
-      wv[r] = okv[r] ? d + (e - sl[r]) : 0.f;
+      const float e = (wv[r] - (d - z)) - (sr + z);
+      wv[r] = okv[r] ? d + (e - lr) : 0.f;
     } else {
-      wv[r] = okv[r] ? wv[r] - sh[r] : 0.f;
+      wv[r] = okv[r] ? wv[r] - sr : 0.f;
     }
   }
 #pragma unroll
   for (int r = 0; r < kEigPix; r++)
-    if (okv[r]) w[qv[r]] = wv[r];
+    if (okv[r]) stu(w + base, qv[r], wv[r]);
   __shared__ float2 sred[kEigWarps * kRed];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if constexpr (MODE == 1) {
-    basis_dots(a, j, qv, wv, nullptr, sred, warp, lane);
+    basis_dots(a, j, base, qv, wv, nullptr, sred, warp, lane);
     cta_partials(sred, j + 1, a.part + (long long)blockIdx.x * a.mp1);
   } else {
     float hi = 0.f, lo = 0.f;
@@ -340,24 +406,26 @@ __global__ void __launch_bounds__(kEigThreads, 2) ks_orth(EigArgs a, int j, floa
     const int tb = a.tile_begin[t.patch], tc = a.tile_count[t.patch];
     double* T = a.T + (long long)t.patch * a.m * a.m;
     if constexpr (MODE == 1) {
-      for (int i = warp; i <= j; i += kEigWarps) {
-        const double s = patch_sum(a.part, tb, tc, a.mp1, i, lane);
-        if (lane == 0) {
-          a.hbuf[(long long)t.patch * a.mp1 + i] = s;
-          T[i * a.m + j] += s;
-          if (i != j) T[j * a.m + i] += s;
-        }
-      }
+      // T is symmetric, and pass 0 wrote both of its entries
+      patch_sums(
+          a.part, tb, tc, a.mp1, j + 1, warp, lane, [&](int i) { return T[i * a.m + j]; },
+          [&](int i, double s, double was) {
+            a.hbuf[(long long)t.patch * a.mp1 + i] = s;
+            T[i * a.m + j] = was + s;
+            T[j * a.m + i] = was + s;
+          });
     } else if (warp == 0) {
-      double s = patch_sum(a.part, tb, tc, a.mp1, 0, lane);
-      if (lane != 0) return;
-      if (!(s > 1e-60)) s = 1e-60;
-      a.beta2[t.patch] = s;
-      if (j + 1 < a.m) {
-        const double b = sqrt(s);
-        T[(j + 1) * a.m + j] = b;
-        T[j * a.m + (j + 1)] = b;
-      }
+      patch_sums(
+          a.part, tb, tc, a.mp1, 1, warp, lane, [](int) { return 0.0; },
+          [&](int, double s, double) {
+            if (!(s > 1e-60)) s = 1e-60;
+            a.beta2[t.patch] = s;
+            if (j + 1 < a.m) {
+              const double b = sqrt(s);
+              T[(j + 1) * a.m + j] = b;
+              T[j * a.m + (j + 1)] = b;
+            }
+          });
     }
   }
 }
@@ -365,7 +433,9 @@ __global__ void __launch_bounds__(kEigThreads, 2) ks_orth(EigArgs a, int j, floa
 // -------------------------------------------------------------- restart
 // Vout[:, 0..nk) = V[:, 0..m) Y[:, 0..nk) per pixel, then Vout[nk] = w / beta
 // (restart, Vout is the other basis buffer) -- or, for a converged patch
-// (FINAL), the nk = nvec Ritz vectors into evec_out.
+// (FINAL), the nk = nvec Ritz vectors into evec_out.  A CTA per 256 pixels: a
+// restart is one launch between host round trips, so it is spread as wide as
+// it goes.
 // Restart: FMA chains over the m basis vectors; the kept vectors come out
 // orthonormal to a few units of rounding, which the next cycle's two CGS
 // passes keep.  A thread takes one pixel and up to 32 outputs per pass over
@@ -381,7 +451,7 @@ __global__ void __launch_bounds__(kEigThreads, 2) ks_restart(EigArgs a, const fl
                                                             float* __restrict__ vout,
                                                             float* __restrict__ evec_out) {
   constexpr int COLS = 16;  // outputs per pass over V
-  const EigTile t = a.tiles[blockIdx.x];
+  const EigTile t = a.tiles[blockIdx.x / kEigPix];
   const int mode = a.decision[t.patch];  // 0 idle, 1 restart, 2 final
   if (mode != (FINAL ? 2 : 1)) return;
   const PatchDev P = a.patches[t.patch];
@@ -390,6 +460,9 @@ __global__ void __launch_bounds__(kEigThreads, 2) ks_restart(EigArgs a, const fl
   float* ysh = (float*)ysh4;
   const double* Y = a.Y + (long long)t.patch * m * m;
   const int base = (int)P.vec;
+  // 256 pixels of the tile per CTA
+  const int p0 = t.p0 + (int)(blockIdx.x % kEigPix) * kEigThreads, p = p0 + threadIdx.x;
+  if (p0 >= t.p1) return;
   float* out = FINAL ? evec_out : vout;
   for (int c0 = 0; c0 < nk; c0 += COLS) {
     __syncthreads();
@@ -401,14 +474,12 @@ __global__ void __launch_bounds__(kEigThreads, 2) ks_restart(EigArgs a, const fl
       ysh[m * COLS + idx] = (float)(y - (double)yh);
     }
     __syncthreads();
-    for (int r = 0; r < kEigPix; r++) {
-      const int p = t.p0 + threadIdx.x + r * kEigThreads;
-      if (p >= t.p1) break;
+    if (p < t.p1) {
       const int q = base + p;
       float acc[COLS], lo[COLS], g[COLS];
 #pragma unroll
       for (int c = 0; c < COLS; c++) acc[c] = lo[c] = g[c] = 0.f;
-#pragma unroll 4
+#pragma unroll 8
       for (int i = 0; i < m; i++) {
         const float v = a.V[(long long)i * a.lvec + q];
 #pragma unroll
@@ -440,10 +511,7 @@ __global__ void __launch_bounds__(kEigThreads, 2) ks_restart(EigArgs a, const fl
   }
   if constexpr (!FINAL) {
     const float inv = (float)(1.0 / sqrt(a.beta2[t.patch]));
-    for (int r = 0; r < kEigPix; r++) {
-      const int p = t.p0 + threadIdx.x + r * kEigThreads;
-      if (p < t.p1) vout[(long long)nk * a.lvec + base + p] = w[base + p] * inv;
-    }
+    if (p < t.p1) vout[(long long)nk * a.lvec + base + p] = w[base + p] * inv;
   }
 }
 
@@ -477,8 +545,9 @@ __global__ void __launch_bounds__(kEigThreads) ks_init(EigArgs a, float* __restr
   cta_partials(sred, 1, a.part + (long long)blockIdx.x * a.mp1);
   if (last_cta(a.counter + t.patch, a.tile_count[t.patch]) && warp == 0) {
     const int tb = a.tile_begin[t.patch], tc = a.tile_count[t.patch];
-    const double s2 = patch_sum(a.part, tb, tc, a.mp1, 0, lane);
-    if (lane == 0) a.beta2[t.patch] = s2;
+    patch_sums(
+        a.part, tb, tc, a.mp1, 1, warp, lane, [](int) { return 0.0; },
+        [&](int, double s2, double) { a.beta2[t.patch] = s2; });
   }
 }
 
@@ -500,8 +569,8 @@ cudaError_t ks_launch_orth(const EigArgs& a, int ntiles, int j, int mode, float*
 }
 cudaError_t ks_launch_restart(const EigArgs& a, int ntiles, const float* w, float* vout, float* evec,
                               cudaStream_t s, bool any_restart, bool any_final) {
-  if (any_restart) ks_restart<false><<<ntiles, kEigThreads, 2 * a.m * 16 * sizeof(float), s>>>(a, w, vout, evec);
-  if (any_final) ks_restart<true><<<ntiles, kEigThreads, 2 * a.m * 16 * sizeof(float), s>>>(a, w, vout, evec);
+  if (any_restart) ks_restart<false><<<ntiles * kEigPix, kEigThreads, 2 * a.m * 16 * sizeof(float), s>>>(a, w, vout, evec);
+  if (any_final) ks_restart<true><<<ntiles * kEigPix, kEigThreads, 2 * a.m * 16 * sizeof(float), s>>>(a, w, vout, evec);
   return cudaGetLastError();
 }
 
