@@ -14,9 +14,9 @@
 //                Forward (ReLU to BF16, or the head to FP32), and the
 //                data gradient (the masked FP32 output gradient staged as
 //                BF16, convolved with the flipped, transposed weights).
-//   k_ln_wgrad   weight and bias gradients: per (tap, 16-channel chunk) a
-//                CTA accumulates dW = dZ^T X over its share of the tiles on
-//                the tensor cores, then adds it to the FP32 gradient.
+//   k_ln_wgrad   weight and bias gradients: a CTA accumulates dW = dZ^T X of
+//                all taps over its share of the tiles on the tensor cores,
+//                then adds it to the FP32 gradient.
 //   pooling, up-sampling + concatenation and their gradients, the subspace
 //   loss reductions and its gradient, Adam, the weights' BF16 copies.
 #include <cuda_bf16.h>
@@ -186,28 +186,64 @@ __global__ void __launch_bounds__(kConvThreads) k_ln_conv(const LnPatch* __restr
   }
 }
 
-// dW[n][tap][c] += sum over pixels of dZ[p][n] X[p + tap][c] for the CTA's
-// tap and 16-channel chunk c0 (blockIdx.y = chunk * 9 + tap), over the tiles
-// blockIdx.x, + gridDim.x, ...; db[n] += sum dZ[p][n] in the centre-tap,
-// first-chunk CTAs.  dZ = BF16(dA * (mask > 0)).
-template <int CIN, int COUT>
-__global__ void __launch_bounds__(kConvThreads) k_ln_wgrad(const LnPatch* __restrict__ lp,
-                                                           const LnTile* __restrict__ tiles, int ntiles,
-                                                           const float* __restrict__ dA,
-                                                           const bf16* __restrict__ mask, const bf16* __restrict__ X,
-                                                           float* __restrict__ dW, float* __restrict__ db) {
-  constexpr int SP = TH * TW + 8;  // pixels per shared row (+ pad)
-  constexpr int PAIRS = (COUT / 16) * 2, PW = (PAIRS + 3) / 4;
-  __shared__ __align__(16) bf16 dz_s[COUT * SP];
-  __shared__ __align__(16) bf16 x_s[16 * SP];
-  const int tap = blockIdx.y % 9, c0 = (blockIdx.y / 9) * 16, dy = tap / 3 - 1, dx = tap % 3 - 1;
-  const bool bias_cta = (tap == 4 && c0 == 0);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tg = lane & 3;
-  float acc[PW][4];
+__device__ __forceinline__ void ldsm4t(uint32_t (&r)[4], const bf16* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"((uint32_t)__cvta_generic_to_shared(p)));
+}
+__device__ __forceinline__ void ldsm2t(uint32_t (&r)[2], const bf16* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];"
+               : "=r"(r[0]), "=r"(r[1])
+               : "r"((uint32_t)__cvta_generic_to_shared(p)));
+}
+
+// dW[n][tap][c] += sum over pixels of dZ[p][n] X[p + tap][c] for all nine
+// taps and the CTA's CC input channels (from c0 = blockIdx.y * CC), over the
+// tiles blockIdx.x, + gridDim.x, ...; db[n] += sum dZ[p][n] in the first
+// chunk's CTAs.  dZ = BF16(dA * (mask > 0)).
+// A GEMM over pixels, 16 (one tile row) per step: the tile's dZ and its X
+// with the halo are staged once, pixel-major as they lie in memory, and
+// ldmatrix.trans turns them into fragments, so a tap is only another row
+// offset.  Warp (wc, wk) keeps the sums of CC / (8 WC) blocks of 8 input
+// channels x 9 taps x COUT over the tile rows wk, wk + 8 / WC, ... in
+// registers over all its tiles; the row groups are added in shared memory and
+// leave with one atomic per weight and CTA.
+// Bound by reading dA (FP32), mask and X for the thin layers and by the
+// tensor pipe for 64 channels.  Measured for one gradient of 16 patches of
+// 256^2, all 15 layers: 0.99 ms; a CTA per (tap, 16 channels), which
+// staged every tile 9 CIN / 16 times and transposed it with 2-byte stores,
+// took 4.24 ms.
+template <int CIN, int CC, int COUT, int WC>
+struct WgradCfg {
+  static constexpr int WK = 8 / WC, CPW = CC / 8 / WC, NT = COUT / 16;
+  static constexpr int ZP = COUT + 8, XP = CC + 8;  // row pitches: 16-byte rows in distinct banks
+  static constexpr size_t stage = ((size_t)TH * TW * ZP + (size_t)NHALO * XP) * sizeof(bf16);
+  static constexpr size_t sums = WK > 1 ? (size_t)COUT * 9 * CC * sizeof(float) : 0;
+  static constexpr size_t smem = stage > sums ? stage : sums;
+  static_assert(CPW * WC * 8 == CC && CIN % CC == 0, "channel split");
+};
+template <int CIN, int CC, int COUT, int WC>
+__global__ void __launch_bounds__(256) k_ln_wgrad(const LnPatch* __restrict__ lp, const LnTile* __restrict__ tiles,
+                                                  int ntiles, const float* __restrict__ dA,
+                                                  const bf16* __restrict__ mask, const bf16* __restrict__ X,
+                                                  float* __restrict__ dW, float* __restrict__ db) {
+  using G = WgradCfg<CIN, CC, COUT, WC>;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  bf16* dz_s = (bf16*)smem_raw;            // [128][ZP]
+  bf16* x_s = dz_s + TH * TW * G::ZP;      // [NHALO][XP]
+  __shared__ float db_s[256];
+  const int c0 = blockIdx.y * CC;
+  const bool bias_cta = blockIdx.y == 0;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, wc = warp % WC, wk = warp / WC;
+  float acc[G::CPW][9][G::NT][4];
 #pragma unroll
-  for (int i = 0; i < PW; i++)
+  for (int ct = 0; ct < G::CPW; ct++)
 #pragma unroll
-    for (int k = 0; k < 4; k++) acc[i][k] = 0.f;
+    for (int t = 0; t < 9; t++)
+#pragma unroll
+      for (int n = 0; n < G::NT; n++)
+#pragma unroll
+        for (int k = 0; k < 4; k++) acc[ct][t][n][k] = 0.f;
   float dbacc = 0.f;
   for (int ti = blockIdx.x; ti < ntiles; ti += gridDim.x) {
     const LnTile t = tiles[ti];
@@ -216,11 +252,11 @@ __global__ void __launch_bounds__(kConvThreads) k_ln_wgrad(const LnPatch* __rest
     for (int idx = threadIdx.x; idx < TH * TW * (COUT / 8); idx += blockDim.x) {
       const int px = idx / (COUT / 8), q = idx % (COUT / 8);
       const int y = t.y0 + px / TW, x = t.x0 + px % TW;
-      float f[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+      uint4 v = make_uint4(0u, 0u, 0u, 0u);
       if (y < P.H && x < P.W) {
         const long long pix = P.off + (long long)y * P.W + x;
         const float4 g0 = *(const float4*)(dA + pix * COUT + q * 8), g1 = *(const float4*)(dA + pix * COUT + q * 8 + 4);
-        f[0] = g0.x, f[1] = g0.y, f[2] = g0.z, f[3] = g0.w, f[4] = g1.x, f[5] = g1.y, f[6] = g1.z, f[7] = g1.w;
+        float f[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
         if (mask) {
           const uint4 mk = *(const uint4*)(mask + pix * COUT + q * 8);
           const bf16* m = (const bf16*)&mk;
@@ -228,56 +264,77 @@ __global__ void __launch_bounds__(kConvThreads) k_ln_wgrad(const LnPatch* __rest
           for (int k = 0; k < 8; k++)
             if (!(__bfloat162float(m[k]) > 0.f)) f[k] = 0.f;
         }
+        v = make_uint4(pack2(f[0], f[1]), pack2(f[2], f[3]), pack2(f[4], f[5]), pack2(f[6], f[7]));
       }
-#pragma unroll
-      for (int k = 0; k < 8; k++) dz_s[(q * 8 + k) * SP + px] = __float2bfloat16_rn(f[k]);
+      *(uint4*)(dz_s + px * G::ZP + q * 8) = v;
     }
-    for (int idx = threadIdx.x; idx < TH * TW * 2; idx += blockDim.x) {
-      const int px = idx >> 1, q = idx & 1;
-      const int y = t.y0 + px / TW + dy, x = t.x0 + px % TW + dx;
+    // zeros outside the patch; a pixel of the tile outside it has dZ = 0
+    for (int idx = threadIdx.x; idx < NHALO * (CC / 8); idx += blockDim.x) {
+      const int h = idx / (CC / 8), q = idx % (CC / 8);
+      const int y = t.y0 - 1 + h / WP, x = t.x0 - 1 + h % WP;
       uint4 v = make_uint4(0u, 0u, 0u, 0u);
-      // only output pixels inside the patch contribute (their dZ is zero
-      // otherwise); the input pixel must exist too (zero padding)
-      const int yo = t.y0 + px / TW, xo = t.x0 + px % TW;
-      if (yo < P.H && xo < P.W && y >= 0 && y < P.H && x >= 0 && x < P.W)
+      if (y >= 0 && y < P.H && x >= 0 && x < P.W)
         v = *(const uint4*)(X + (P.off + (long long)y * P.W + x) * CIN + c0 + q * 8);
-      const bf16* e = (const bf16*)&v;
-#pragma unroll
-      for (int k = 0; k < 8; k++) x_s[(q * 8 + k) * SP + px] = e[k];
+      *(uint4*)(x_s + h * G::XP + q * 8) = v;
     }
     __syncthreads();
-    if (bias_cta && threadIdx.x < COUT) {
+    if (bias_cta) {  // thread = channel + COUT * share of the pixels
+      const int n = threadIdx.x % COUT, part = threadIdx.x / COUT;
+      constexpr int PER = TH * TW * COUT / 256;
       float s = 0.f;
-      for (int px = 0; px < TH * TW; px++) s += __bfloat162float(dz_s[threadIdx.x * SP + px]);
+#pragma unroll 4
+      for (int px = part * PER; px < (part + 1) * PER; px++) s += __bfloat162float(dz_s[px * G::ZP + n]);
       dbacc += s;
     }
+#pragma unroll 1
+    for (int row = wk; row < TH; row += G::WK) {
+      uint32_t a[G::NT][4];
 #pragma unroll
-    for (int ks = 0; ks < TH * TW / 16; ks++) {
+      for (int n = 0; n < G::NT; n++)
+        ldsm4t(a[n], dz_s + (row * TW + (lane & 7) + ((lane >> 4) & 1) * 8) * G::ZP + n * 16 + ((lane >> 3) & 1) * 8);
 #pragma unroll
-      for (int i = 0; i < PW; i++) {
-        const int pair = warp + 4 * i;
-        if (pair >= PAIRS) break;
-        const int mt = pair >> 1, nt = pair & 1;
-        const bf16* ar = dz_s + (mt * 16 + g) * SP + ks * 16 + 2 * tg;
-        const bf16* br = x_s + (nt * 8 + g) * SP + ks * 16 + 2 * tg;
-        mma_bf16(acc[i], ld32(ar), ld32(ar + 8 * SP), ld32(ar + 8), ld32(ar + 8 * SP + 8), ld32(br), ld32(br + 8));
-      }
+      for (int tap = 0; tap < 9; tap++)
+#pragma unroll
+        for (int ct = 0; ct < G::CPW; ct++) {
+          uint32_t b[2];
+          ldsm2t(b, x_s + ((row + tap / 3) * WP + tap % 3 + (lane & 15)) * G::XP + (wc * G::CPW + ct) * 8);
+#pragma unroll
+          for (int n = 0; n < G::NT; n++) mma_bf16(acc[ct][tap][n], a[n][0], a[n][1], a[n][2], a[n][3], b[0], b[1]);
+        }
     }
   }
-#pragma unroll
-  for (int i = 0; i < PW; i++) {
-    const int pair = warp + 4 * i;
-    if (pair >= PAIRS) break;
-    const int mt = pair >> 1, nt = pair & 1;
-    const int n = mt * 16 + g, c = c0 + nt * 8 + 2 * tg;
-    float* d0 = dW + ((long long)n * 9 + tap) * CIN + c;
-    float* d1 = dW + ((long long)(n + 8) * 9 + tap) * CIN + c;
-    atomicAdd(d0, acc[i][0]);
-    atomicAdd(d0 + 1, acc[i][1]);
-    atomicAdd(d1, acc[i][2]);
-    atomicAdd(d1 + 1, acc[i][3]);
+  __syncthreads();
+  const int g = lane >> 2, tg = lane & 3;
+  float* sums = (float*)smem_raw;  // [COUT][9][CC]
+  if constexpr (G::WK > 1) {
+    for (int i = threadIdx.x; i < COUT * 9 * CC; i += blockDim.x) sums[i] = 0.f;
+    __syncthreads();
   }
-  if (bias_cta && threadIdx.x < COUT) atomicAdd(db + threadIdx.x, dbacc);
+#pragma unroll
+  for (int ct = 0; ct < G::CPW; ct++)
+#pragma unroll
+    for (int tap = 0; tap < 9; tap++)
+#pragma unroll
+      for (int n = 0; n < G::NT; n++)
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+          const int o = n * 16 + g + 8 * (k >> 1), c = (wc * G::CPW + ct) * 8 + 2 * tg + (k & 1);
+          if constexpr (G::WK > 1)
+            atomicAdd(sums + (o * 9 + tap) * CC + c, acc[ct][tap][n][k]);
+          else
+            atomicAdd(dW + ((long long)o * 9 + tap) * CIN + c0 + c, acc[ct][tap][n][k]);
+        }
+  if (bias_cta) db_s[threadIdx.x] = dbacc;
+  __syncthreads();
+  if constexpr (G::WK > 1) {
+    for (int i = threadIdx.x; i < COUT * 9 * CC; i += blockDim.x)
+      atomicAdd(dW + (long long)(i / CC) * CIN + c0 + i % CC, sums[i]);
+  }
+  if (bias_cta && threadIdx.x < COUT) {
+    float s = 0.f;
+    for (int i = threadIdx.x; i < 256; i += COUT) s += db_s[i];
+    atomicAdd(db + threadIdx.x, s);
+  }
 }
 
 // ---------------------------------------------------------- resampling
@@ -286,11 +343,9 @@ __global__ void k_ln_pool(const LnPatch* __restrict__ lo, const LnPatch* __restr
                           const bf16* __restrict__ in, bf16* __restrict__ out) {
   const int p = blockIdx.y;
   const LnPatch S = lo[p], D = hi[p];  // source (fine), destination (coarse)
-  const int nq = C / 8;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < (long long)D.H * D.W * nq;
-       i += (long long)gridDim.x * blockDim.x) {
-    const int q = (int)(i % nq);
-    const long long px = i / nq;
+  const uint32_t nq = C / 8, total = (uint32_t)D.H * D.W * nq;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+    const uint32_t q = i % nq, px = i / nq;
     const int y = (int)(px / D.W), x = (int)(px % D.W);
     float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     int n = 0;
@@ -311,19 +366,28 @@ __global__ void k_ln_pool(const LnPatch* __restrict__ lo, const LnPatch* __restr
   }
 }
 
+// The resampling gradients move 4 channels (16 bytes) per thread with 32-bit
+// indices (a level of a patch has at most 2^26 pixels and 2^31 / 4 groups of
+// channels); one channel per thread with 64-bit divisions took 300 us of
+// one gradient of 16 patches of 256^2, against 153 us.
 // dS[y][x] += dP[y/2][x/2] / count(y/2, x/2), FP32
 __global__ void k_ln_pool_bwd(const LnPatch* __restrict__ lo, const LnPatch* __restrict__ hi, int C,
                               const float* __restrict__ dP, float* __restrict__ dS) {
   const int p = blockIdx.y;
   const LnPatch S = lo[p], D = hi[p];
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < (long long)S.H * S.W * C;
-       i += (long long)gridDim.x * blockDim.x) {
-    const int c = (int)(i % C);
-    const long long px = i / C;
-    const int y = (int)(px / S.W), x = (int)(px % S.W);
-    const int cy = y >> 1, cx = x >> 1;
-    const int n = (min(2 * cy + 2, S.H) - 2 * cy) * (min(2 * cx + 2, S.W) - 2 * cx);
-    dS[(S.off + px) * C + c] += dP[(D.off + (long long)cy * D.W + cx) * C + c] / (float)n;
+  const uint32_t nq = C / 4, total = (uint32_t)S.H * S.W * nq;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+    const uint32_t q = i % nq, px = i / nq;
+    const int y = (int)(px / S.W), x = (int)(px % S.W), cy = y >> 1, cx = x >> 1;
+    const float n = (float)((min(2 * cy + 2, S.H) - 2 * cy) * (min(2 * cx + 2, S.W) - 2 * cx));
+    float4* d = (float4*)(dS + (S.off + px) * C) + q;
+    const float4 g = *((const float4*)(dP + (D.off + (long long)cy * D.W + cx) * C) + q);
+    float4 v = *d;
+    v.x += g.x / n;
+    v.y += g.y / n;
+    v.z += g.z / n;
+    v.w += g.w / n;
+    *d = v;
   }
 }
 
@@ -332,14 +396,13 @@ __global__ void k_ln_upcat(const LnPatch* __restrict__ lo, const LnPatch* __rest
                            const bf16* __restrict__ coarse, const bf16* __restrict__ skip, bf16* __restrict__ out) {
   const int p = blockIdx.y;
   const LnPatch F = lo[p], Q = hi[p];
-  const int C = C1 + C2, nq = C / 8;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < (long long)F.H * F.W * nq;
-       i += (long long)gridDim.x * blockDim.x) {
-    const int q = (int)(i % nq);
-    const long long px = i / nq;
+  const int C = C1 + C2;
+  const uint32_t nq = C / 8, total = (uint32_t)F.H * F.W * nq;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+    const uint32_t q = i % nq, px = i / nq;
     const int y = (int)(px / F.W), x = (int)(px % F.W);
     uint4 v;
-    if (q * 8 < C1)
+    if ((int)q * 8 < C1)
       v = *(const uint4*)(coarse + (Q.off + (long long)(y >> 1) * Q.W + (x >> 1)) * C1 + q * 8);
     else
       v = *(const uint4*)(skip + (F.off + px) * C2 + (q * 8 - C1));
@@ -354,18 +417,24 @@ __global__ void k_ln_upcat_bwd_coarse(const LnPatch* __restrict__ lo, const LnPa
   const int p = blockIdx.y;
   const LnPatch F = lo[p], Q = hi[p];
   const int C = C1 + C2;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < (long long)Q.H * Q.W * C1;
-       i += (long long)gridDim.x * blockDim.x) {
-    const int c = (int)(i % C1);
-    const long long px = i / C1;
+  const uint32_t nq = C1 / 4, total = (uint32_t)Q.H * Q.W * nq;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+    const uint32_t q = i % nq, px = i / nq;
     const int y = (int)(px / Q.W), x = (int)(px % Q.W);
-    float s = 0.f;
+    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
     for (int a = 0; a < 2; a++)
+#pragma unroll
       for (int b = 0; b < 2; b++) {
         const int yy = 2 * y + a, xx = 2 * x + b;
-        if (yy < F.H && xx < F.W) s += dC[(F.off + (long long)yy * F.W + xx) * C + c];
+        if (yy >= F.H || xx >= F.W) continue;
+        const float4 v = *((const float4*)(dC + (F.off + (long long)yy * F.W + xx) * C) + q);
+        s.x += v.x;
+        s.y += v.y;
+        s.z += v.z;
+        s.w += v.w;
       }
-    dcoarse[(Q.off + px) * C1 + c] = s;
+    *((float4*)(dcoarse + (Q.off + px) * C1) + q) = s;
   }
 }
 __global__ void k_ln_upcat_bwd_skip(const LnPatch* __restrict__ lo, int C1, int C2, const float* __restrict__ dC,
@@ -373,11 +442,10 @@ __global__ void k_ln_upcat_bwd_skip(const LnPatch* __restrict__ lo, int C1, int 
   const int p = blockIdx.y;
   const LnPatch F = lo[p];
   const int C = C1 + C2;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < (long long)F.H * F.W * C2;
-       i += (long long)gridDim.x * blockDim.x) {
-    const int c = (int)(i % C2);
-    const long long px = i / C2;
-    dskip[(F.off + px) * C2 + c] = dC[(F.off + px) * C + C1 + c];
+  const uint32_t nq = C2 / 4, total = (uint32_t)F.H * F.W * nq;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+    const uint32_t q = i % nq, px = i / nq;
+    *((float4*)(dskip + (F.off + px) * C2) + q) = *((const float4*)(dC + (F.off + px) * C + C1) + q);
   }
 }
 
@@ -407,44 +475,193 @@ __global__ void k_ln_features_from(const LnPatch* __restrict__ lp, const PatchDe
 }
 
 // ------------------------------------------------------------------ loss
-// per patch: G = Y^T Y (32 x 32) and B = V^T Y (9 x 32), FP64 sums of FP32
-// per-warp partials; lane j owns column j
+// Rows of 4 consecutive pixels per warp pass through shared memory, so a
+// pixel's 32 fields and 9 targets reach every lane as 16-byte broadcasts
+// instead of 41 shuffles.
 constexpr int kGramLen = kLnOut * kLnOut + kLnTargets * kLnOut;
+constexpr int kVPitch = 12;
+struct LnRows {
+  float y[4][kLnOut];
+  float v[4][kVPitch];
+};
+// a lane's share of 4 pixels q, q + step, .. (zeros from the n-th on), held in
+// registers while the warp works on the previous 4
+struct LnShare {
+  float4 y;
+  float v[2];
+};
+__device__ __forceinline__ LnShare ln_fetch(const float* __restrict__ y, const float* __restrict__ v, long long q,
+                                            long long step, int n, int lane) {
+  LnShare f;
+  const int px = lane >> 3;
+  f.y = px < n ? *(const float4*)(y + (q + px * step) * kLnOut + 4 * (lane & 7)) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+  for (int h = 0; h < 2; h++) {
+    const int i = lane + 32 * h, p = i / kLnTargets;
+    f.v[h] = i < 4 * kLnTargets && p < n ? v[(q + p * step) * kLnTargets + i % kLnTargets] : 0.f;
+  }
+  return f;
+}
+__device__ __forceinline__ void ln_store(LnRows& r, const LnShare& f, int lane) {
+  __syncwarp();
+  *(float4*)&r.y[lane >> 3][4 * (lane & 7)] = f.y;
+  r.v[lane / kLnTargets][lane % kLnTargets] = f.v[0];
+  if (lane + 32 < 4 * kLnTargets) r.v[(lane + 32) / kLnTargets][(lane + 32) % kLnTargets] = f.v[1];
+  __syncwarp();
+}
+__device__ __forceinline__ void ln_row(const LnRows& r, int p, float (&yk)[kLnOut], float (&vi)[kVPitch]) {
+#pragma unroll
+  for (int k = 0; k < kLnOut; k += 4) {
+    const float4 f = *(const float4*)&r.y[p][k];
+    yk[k] = f.x, yk[k + 1] = f.y, yk[k + 2] = f.z, yk[k + 3] = f.w;
+  }
+#pragma unroll
+  for (int k = 0; k < kVPitch; k += 4) {
+    const float4 f = *(const float4*)&r.v[p][k];
+    vi[k] = f.x, vi[k + 1] = f.y, vi[k + 2] = f.z, vi[k + 3] = f.w;
+  }
+}
+
+// per patch: G = Y^T Y (32 x 32) and B = V^T Y (9 x 32), FP64 sums of FP32
+// per-warp partials; lane j owns column j.  The warps of a CTA are summed in
+// shared memory before the atomics: 138 us for 16 patches of 256^2, from 358
+// us with 5.5 M FP64 atomics and 41 shuffles per pixel.
 __global__ void __launch_bounds__(256) k_ln_gram(const LnPatch* __restrict__ lp, const float* __restrict__ y,
                                                  const float* __restrict__ v, double* __restrict__ gb) {
+  __shared__ __align__(16) LnRows rows[8];
+  __shared__ float part[8][kGramLen];
   const LnPatch P = lp[blockIdx.y];
   const long long N = (long long)P.H * P.W;
-  const int lane = threadIdx.x & 31;
-  const long long w0 = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
-  const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const long long w0 = (long long)blockIdx.x * 8 + warp, nw = (long long)gridDim.x * 8;
+  LnRows& r = rows[warp];
+  if (lane < 4 * (kVPitch - kLnTargets)) r.v[lane / 3][kLnTargets + lane % 3] = 0.f;
   float G[kLnOut], B[kLnTargets];
 #pragma unroll
   for (int k = 0; k < kLnOut; k++) G[k] = 0.f;
 #pragma unroll
   for (int i = 0; i < kLnTargets; i++) B[i] = 0.f;
-  for (long long p = w0; p < N; p += nw) {
-    const long long q = P.off + p;
-    const float yj = y[q * kLnOut + lane];
-    const float vl = lane < kLnTargets ? v[q * kLnTargets + lane] : 0.f;
+  auto count = [&](long long p) { return p < N ? (int)min((N - p + nw - 1) / nw, 4LL) : 0; };
+  LnShare next = ln_fetch(y, v, P.off + w0, nw, count(w0), lane);
+  for (long long p = w0; p < N; p += 4 * nw) {
+    ln_store(r, next, lane);
+    next = ln_fetch(y, v, P.off + p + 4 * nw, nw, count(p + 4 * nw), lane);
 #pragma unroll
-    for (int k = 0; k < kLnOut; k++) G[k] = fmaf(yj, __shfl_sync(0xffffffffu, yj, k), G[k]);
+    for (int k4 = 0; k4 < 4; k4++) {
+      float yk[kLnOut], vi[kVPitch];
+      ln_row(r, k4, yk, vi);
+      const float yj = r.y[k4][lane];
 #pragma unroll
-    for (int i = 0; i < kLnTargets; i++) B[i] = fmaf(__shfl_sync(0xffffffffu, vl, i), yj, B[i]);
+      for (int k = 0; k < kLnOut; k++) G[k] = fmaf(yj, yk[k], G[k]);
+#pragma unroll
+      for (int i = 0; i < kLnTargets; i++) B[i] = fmaf(vi[i], yj, B[i]);
+    }
   }
+#pragma unroll
+  for (int k = 0; k < kLnOut; k++) part[warp][k * kLnOut + lane] = G[k];  // G is symmetric
+#pragma unroll
+  for (int i = 0; i < kLnTargets; i++) part[warp][kLnOut * kLnOut + i * kLnOut + lane] = B[i];
+  __syncthreads();
   double* o = gb + (long long)blockIdx.y * kGramLen;
+  for (int e = threadIdx.x; e < kGramLen; e += blockDim.x) {
+    double s = 0;
 #pragma unroll
-  for (int k = 0; k < kLnOut; k++) atomicAdd(o + lane * kLnOut + k, (double)G[k]);
-#pragma unroll
-  for (int i = 0; i < kLnTargets; i++) atomicAdd(o + kLnOut * kLnOut + i * kLnOut + lane, (double)B[i]);
+    for (int w = 0; w < 8; w++) s += (double)part[w][e];
+    atomicAdd(o + e, s);
+  }
+}
+
+// per patch, from G and B: C1 = B (G + eps I)^-1 (9 x 32) and C2 = C1^T C1
+// (32 x 32) into cm, and the loss 9 - <C1, B>; bad is set where the
+// regularised G is not positive definite.  One CTA per patch in FP64 with
+// unfused operations in the order of a sequential Cholesky inverse, so the
+// values are those of host code.  Bound by the FP64 roots, quotients and
+// subtraction chains: 147 us for any number of patches up to the SMs, against
+// 0.77 ms for the host round trip of 16.
+__global__ void __launch_bounds__(256) k_ln_solve(const double* __restrict__ gb, float* __restrict__ cm,
+                                                  double* __restrict__ loss, int* __restrict__ bad) {
+  constexpr int K = kLnOut, T = kLnTargets, LP = K + 1;
+  __shared__ double A[K * LP], Gi[K * LP], Bs[T * K], C1[T * K], red[T * K];
+  const double* g = gb + (long long)blockIdx.x * kGramLen;
+  const int tid = threadIdx.x, lane = tid & 31;
+  double tr = 0;
+  for (int i = 0; i < K; i++) tr = __dadd_rn(tr, g[i * K + i]);
+  const double eps = __dadd_rn(__ddiv_rn(__dmul_rn(1e-4, tr), (double)K), 1e-30);
+  for (int i = tid; i < K * K; i += 256) A[(i / K) * LP + i % K] = i / K == i % K ? __dadd_rn(g[i], eps) : g[i];
+  for (int i = tid; i < T * K; i += 256) Bs[i] = g[K * K + i];
+  __syncthreads();
+  // Each element's products are subtracted in ascending k, as a dot product
+  // would; the columns advance together.  A becomes L; Gi starts as I and
+  // becomes L^-1, then (L L^T)^-1.
+  __shared__ int fail;
+  if (tid == 0) fail = 0;
+  for (int e = tid; e < K * K; e += 256) Gi[(e / K) * LP + e % K] = e / K == e % K ? 1.0 : 0.0;
+  __syncthreads();
+  for (int j = 0; j < K; j++) {
+    const double d = A[j * LP + j];
+    if (tid == 0 && !(d > 0)) fail = 1;
+    const double s = __dsqrt_rn(d > 0 ? d : 1.0);
+    double l = 0;
+    if (tid < 32) {
+      if (lane > j) l = __ddiv_rn(A[lane * LP + j], s);
+    } else if (tid < 64) {
+      l = __ddiv_rn(Gi[j * LP + lane], s);  // row j of L^-1, column = lane
+    }
+    __syncthreads();
+    if (tid < 32) {
+      if (lane >= j) A[lane * LP + j] = lane == j ? s : l;
+    } else if (tid < 64) {
+      Gi[j * LP + lane] = l;
+    }
+    __syncthreads();
+    for (int e = tid; e < K * K; e += 256) {
+      const int r = e / K, q = e % K;
+      if (r <= j) continue;
+      const double lr = A[r * LP + j];
+      if (q > j && q <= r) A[r * LP + q] = __dsub_rn(A[r * LP + q], __dmul_rn(lr, A[q * LP + j]));
+      Gi[r * LP + q] = __dsub_rn(Gi[r * LP + q], __dmul_rn(lr, Gi[j * LP + q]));
+    }
+    __syncthreads();
+  }
+  if (tid < 32) {  // L^T x = z, lane = column
+    for (int i = K - 1; i >= 0; i--) {
+      double v = Gi[i * LP + lane];
+#pragma unroll 8
+      for (int k = i + 1; k < K; k++) v = __dsub_rn(v, __dmul_rn(A[k * LP + i], Gi[k * LP + lane]));
+      Gi[i * LP + lane] = __ddiv_rn(v, A[i * LP + i]);
+    }
+    if (fail && lane == 0) *bad = 1;
+  }
+  __syncthreads();
+  float* c = cm + (long long)blockIdx.x * kGramLen;
+  for (int e = tid; e < T * K; e += 256) {
+    double v = 0;
+    for (int k = 0; k < K; k++) v = __dadd_rn(v, __dmul_rn(Bs[e / K * K + k], Gi[k * LP + e % K]));
+    C1[e] = v;
+    c[e] = (float)v;
+    red[e] = __dmul_rn(v, Bs[e]);
+  }
+  __syncthreads();
+  for (int e = tid; e < K * K; e += 256) {
+    double v = 0;
+    for (int i = 0; i < T; i++) v = __dadd_rn(v, __dmul_rn(C1[i * K + e / K], C1[i * K + e % K]));
+    c[T * K + e] = (float)v;
+  }
+  if (tid == 0) {
+    double cap = 0;
+    for (int i = 0; i < T * K; i++) cap = __dadd_rn(cap, red[i]);
+    loss[blockIdx.x] = T - cap;
+  }
 }
 
 // dY[p][j] = -2 (sum_i V[p][i] C1[i][j] - sum_k Y[p][k] C2[k][j])
 __global__ void __launch_bounds__(256) k_ln_dy(const LnPatch* __restrict__ lp, const float* __restrict__ y,
                                                const float* __restrict__ v, const float* __restrict__ cm,
                                                float* __restrict__ dy) {
+  __shared__ __align__(16) LnRows rows[8];
   const LnPatch P = lp[blockIdx.y];
   const long long N = (long long)P.H * P.W;
-  const int lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const float* C1 = cm + (long long)blockIdx.y * kGramLen;  // [9][32]
   const float* C2 = C1 + kLnTargets * kLnOut;                  // [32][32]
   float c1[kLnTargets], c2[kLnOut];
@@ -452,18 +669,26 @@ __global__ void __launch_bounds__(256) k_ln_dy(const LnPatch* __restrict__ lp, c
   for (int i = 0; i < kLnTargets; i++) c1[i] = C1[i * kLnOut + lane];
 #pragma unroll
   for (int k = 0; k < kLnOut; k++) c2[k] = C2[k * kLnOut + lane];
-  const long long w0 = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
-  const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
-  for (long long p = w0; p < N; p += nw) {
-    const long long q = P.off + p;
-    const float yj = y[q * kLnOut + lane];
-    const float vl = lane < kLnTargets ? v[q * kLnTargets + lane] : 0.f;
-    float s = 0.f;
+  const long long w0 = (long long)blockIdx.x * 8 + warp, nw = (long long)gridDim.x * 8;
+  LnRows& r = rows[warp];
+  auto count = [&](long long p) { return p < N ? (int)min(N - p, 4LL) : 0; };
+  LnShare next = ln_fetch(y, v, P.off + 4 * w0, 1, count(4 * w0), lane);
+  for (long long p = 4 * w0; p < N; p += 4 * nw) {
+    const int n = count(p);
+    ln_store(r, next, lane);
+    next = ln_fetch(y, v, P.off + p + 4 * nw, 1, count(p + 4 * nw), lane);
 #pragma unroll
-    for (int i = 0; i < kLnTargets; i++) s = fmaf(__shfl_sync(0xffffffffu, vl, i), c1[i], s);
+    for (int k4 = 0; k4 < 4; k4++) {
+      if (k4 >= n) break;
+      float yk[kLnOut], vi[kVPitch];
+      ln_row(r, k4, yk, vi);
+      float s = 0.f;
 #pragma unroll
-    for (int k = 0; k < kLnOut; k++) s = fmaf(-__shfl_sync(0xffffffffu, yj, k), c2[k], s);
-    dy[q * kLnOut + lane] = -2.f * s;
+      for (int i = 0; i < kLnTargets; i++) s = fmaf(vi[i], c1[i], s);
+#pragma unroll
+      for (int k = 0; k < kLnOut; k++) s = fmaf(-yk[k], c2[k], s);
+      dy[(P.off + p + k4) * kLnOut + lane] = -2.f * s;
+    }
   }
 }
 
@@ -573,23 +798,34 @@ cudaError_t conv_launch(int cin, int cout, int mode, const LnPatch* lp, const Ln
   return cudaErrorInvalidValue;
 }
 
+template <int CIN, int CC, int COUT, int WC>
+cudaError_t wgrad_go(const LnPatch* lp, const LnTile* tiles, int ntiles, const float* dA, const bf16* mask,
+                     const bf16* X, float* dW, float* db, cudaStream_t s) {
+  using G = WgradCfg<CIN, CC, COUT, WC>;
+  static bool attr = false;
+  if (!attr) {
+    cudaFuncSetAttribute(k_ln_wgrad<CIN, CC, COUT, WC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G::smem);
+    attr = true;
+  }
+  // about two CTAs per SM over the channel chunks; one where a thread's sums
+  // take most of its registers
+  constexpr int chunks = CIN / CC, per_sm = G::CPW * G::NT >= 4 ? 1 : 2;
+  const dim3 grid(std::max(1, std::min(ntiles, 152 * per_sm / chunks)), chunks);
+  k_ln_wgrad<CIN, CC, COUT, WC><<<grid, 256, G::smem, s>>>(lp, tiles, ntiles, dA, mask, X, dW, db);
+  return cudaGetLastError();
+}
 cudaError_t wgrad_launch(int cin, int cout, const LnPatch* lp, const LnTile* tiles, int ntiles, const float* dA,
                          const bf16* mask, const bf16* X, float* dW, float* db, cudaStream_t s) {
   if (ntiles == 0) return cudaSuccess;
-  const dim3 grid(std::min(ntiles, 64), 9 * (cin / 16));
-#define GO(CI, CO)                                                                                \
-  do {                                                                                            \
-    k_ln_wgrad<CI, CO><<<grid, kConvThreads, 0, s>>>(lp, tiles, ntiles, dA, mask, X, dW, db); \
-    return cudaGetLastError();                                                                    \
-  } while (0)
-  if (cin == 16 && cout == 16) GO(16, 16);
-  if (cin == 16 && cout == 32) GO(16, 32);
-  if (cin == 32 && cout == 32) GO(32, 32);
-  if (cin == 32 && cout == 64) GO(32, 64);
-  if (cin == 64 && cout == 64) GO(64, 64);
-  if (cin == 128 && cout == 64) GO(128, 64);
-  if (cin == 96 && cout == 32) GO(96, 32);
-  if (cin == 48 && cout == 16) GO(48, 16);
+#define GO(CI, CC, CO, WC) return wgrad_go<CI, CC, CO, WC>(lp, tiles, ntiles, dA, mask, X, dW, db, s)
+  if (cin == 16 && cout == 16) GO(16, 16, 16, 2);
+  if (cin == 16 && cout == 32) GO(16, 16, 32, 2);
+  if (cin == 32 && cout == 32) GO(32, 32, 32, 4);
+  if (cin == 32 && cout == 64) GO(32, 32, 64, 4);
+  if (cin == 64 && cout == 64) GO(64, 64, 64, 8);
+  if (cin == 128 && cout == 64) GO(128, 64, 64, 8);
+  if (cin == 96 && cout == 32) GO(96, 32, 32, 4);
+  if (cin == 48 && cout == 16) GO(48, 48, 16, 2);
 #undef GO
   return cudaErrorInvalidValue;
 }
@@ -623,9 +859,10 @@ struct LearnedNet::Impl {
   size_t cap_y = 0;
   double* gram = nullptr;
   float* cm = nullptr;
-  size_t cap_gram = 0, cap_cm = 0;
-  std::vector<double> h_gram;
-  std::vector<float> h_cm;
+  double* ploss = nullptr;  // loss per patch
+  int* bad = nullptr;
+  size_t cap_gram = 0, cap_cm = 0, cap_ploss = 0, cap_bad = 0;
+  std::vector<double> h_loss;
   // named tensors
   bf16 *X0, *A0a, *S0, *C0, *A0c, *A0d, *P0, *A1a, *S1, *C1, *A1c, *A1d, *P1, *A2a, *S2, *C2, *A2c, *A2d, *P2,
       *A3a, *A3b;
@@ -635,7 +872,7 @@ struct LearnedNet::Impl {
 
   Impl() { conv_offsets(wo, bo, &np); }
   ~Impl() {
-    void* ps[] = {w32, grad, am, av, wb, wt, act, gr, y, gram, cm};
+    void* ps[] = {w32, grad, am, av, wb, wt, act, gr, y, gram, cm, ploss, bad};
     for (void* p : ps)
       if (p) cudaFree(p);
     for (int l = 0; l < kLnLevels; l++) {
@@ -771,6 +1008,8 @@ cudaError_t LearnedNet::layout(const std::vector<int>& H, const std::vector<int>
   if ((e = grow_buf(m.y, m.cap_y, (size_t)N0 * kLnOut)) != cudaSuccess) return e;
   if ((e = grow_buf(m.gram, m.cap_gram, (size_t)n * kGramLen)) != cudaSuccess) return e;
   if ((e = grow_buf(m.cm, m.cap_cm, (size_t)n * kGramLen)) != cudaSuccess) return e;
+  if ((e = grow_buf(m.ploss, m.cap_ploss, (size_t)n)) != cudaSuccess) return e;
+  if ((e = grow_buf(m.bad, m.cap_bad, 1)) != cudaSuccess) return e;
   bf16* a = m.act;
   auto A = [&](long long N, int C) {
     bf16* r = a;
@@ -854,36 +1093,6 @@ cudaError_t LearnedNet::forward(cudaStream_t s) {
   return cudaSuccess;
 }
 
-// dense symmetric positive definite inverse by Cholesky (n <= 32)
-static bool spd_inverse(const double* A, int n, double* X) {
-  std::vector<double> L((size_t)n * n, 0.0);
-  for (int j = 0; j < n; j++) {
-    double d = A[j * n + j];
-    for (int k = 0; k < j; k++) d -= L[j * n + k] * L[j * n + k];
-    if (!(d > 0)) return false;
-    L[j * n + j] = std::sqrt(d);
-    for (int i = j + 1; i < n; i++) {
-      double v = A[i * n + j];
-      for (int k = 0; k < j; k++) v -= L[i * n + k] * L[j * n + k];
-      L[i * n + j] = v / L[j * n + j];
-    }
-  }
-  for (int c = 0; c < n; c++) {  // solve L L^T x = e_c
-    std::vector<double> z(n, 0.0);
-    for (int i = 0; i < n; i++) {
-      double v = (i == c) ? 1.0 : 0.0;
-      for (int k = 0; k < i; k++) v -= L[i * n + k] * z[k];
-      z[i] = v / L[i * n + i];
-    }
-    for (int i = n - 1; i >= 0; i--) {
-      double v = z[i];
-      for (int k = i + 1; k < n; k++) v -= L[k * n + i] * X[k * n + c];
-      X[i * n + c] = v / L[i * n + i];
-    }
-  }
-  return true;
-}
-
 cudaError_t LearnedNet::loss_backward(const float* d_v, double* loss, cudaStream_t s) {
   Impl& m = *im_;
   if (!m.have) return cudaErrorInvalidValue;
@@ -895,44 +1104,11 @@ cudaError_t LearnedNet::loss_backward(const float* d_v, double* loss, cudaStream
       m.d_lp[0], m.y, d_v, m.gram);
   m.launches++;
   CKE(cudaGetLastError());
-  m.h_gram.resize((size_t)np * kGramLen);
-  CKE(cudaMemcpyAsync(m.h_gram.data(), m.gram, m.h_gram.size() * sizeof(double), cudaMemcpyDeviceToHost, s));
-  CKE(cudaStreamSynchronize(s));
-  m.h_cm.assign((size_t)np * kGramLen, 0.f);
-  double total = 0;
-  constexpr int K = kLnOut, T = kLnTargets;
-  std::vector<double> Gm(K * K), Gi(K * K), C1(T * K), Bt(T * K);
-  for (int p = 0; p < np; p++) {
-    const double* g = m.h_gram.data() + (size_t)p * kGramLen;
-    double tr = 0;
-    for (int i = 0; i < K; i++) tr += g[i * K + i];
-    for (int i = 0; i < K * K; i++) Gm[i] = g[i];
-    for (int i = 0; i < K; i++) Gm[i * K + i] += 1e-4 * tr / K + 1e-30;
-    const double* B = g + K * K;  // [9][32]
-    if (!spd_inverse(Gm.data(), K, Gi.data())) return cudaErrorInvalidValue;
-    for (int i = 0; i < T; i++)
-      for (int j = 0; j < K; j++) {
-        double v = 0;
-        for (int k = 0; k < K; k++) v += B[i * K + k] * Gi[k * K + j];
-        C1[i * K + j] = v;
-      }
-    double cap = 0;
-    for (int i = 0; i < T; i++)
-      for (int j = 0; j < K; j++) cap += C1[i * K + j] * B[i * K + j];
-    total += T - cap;
-    // C2 = C1^T C1' where C2 = Gi B^T B Gi = (B Gi)^T (B Gi) = C1^T C1
-    float* cm = m.h_cm.data() + (size_t)p * kGramLen;
-    for (int i = 0; i < T * K; i++) cm[i] = (float)C1[i];
-    for (int a = 0; a < K; a++)
-      for (int b = 0; b < K; b++) {
-        double v = 0;
-        for (int i = 0; i < T; i++) v += C1[i * K + a] * C1[i * K + b];
-        cm[T * K + a * K + b] = (float)v;
-      }
-  }
-  *loss = total;
-  CKE(cudaMemcpyAsync(m.cm, m.h_cm.data(), m.h_cm.size() * sizeof(float), cudaMemcpyHostToDevice, s));
-  k_ln_dy<<<dim3((unsigned)std::max(1LL, std::min(m.maxpix[0] / 2048 + 1, 512LL)), np), 256, 0, s>>>(
+  CKE(cudaMemsetAsync(m.bad, 0, sizeof(int), s));
+  k_ln_solve<<<np, 256, 0, s>>>(m.gram, m.cm, m.ploss, m.bad);
+  m.launches++;
+  CKE(cudaGetLastError());
+  k_ln_dy<<<dim3((unsigned)std::max(1LL, std::min(m.maxpix[0] / 512 + 1, 1024LL)), np), 256, 0, s>>>(
       m.d_lp[0], m.y, d_v, m.cm, m.dY);
   m.launches++;
   CKE(cudaGetLastError());
@@ -971,6 +1147,14 @@ cudaError_t LearnedNet::loss_backward(const float* d_v, double* loss, cudaStream
   CKE(pool_bwd(0, 16, m.dP0, m.dS0));
   CKE(m.conv_bwd(1, 0, m.dS0, m.S0, m.A0a, m.dA0a, s));
   CKE(m.conv_bwd(0, 0, m.dA0a, m.A0a, m.X0, nullptr, s));
+  int bad = 0;
+  m.h_loss.resize(np);
+  CKE(cudaMemcpyAsync(m.h_loss.data(), m.ploss, np * sizeof(double), cudaMemcpyDeviceToHost, s));
+  CKE(cudaMemcpyAsync(&bad, m.bad, sizeof(int), cudaMemcpyDeviceToHost, s));
+  CKE(cudaStreamSynchronize(s));
+  if (bad) return cudaErrorInvalidValue;  // a patch's Gram matrix is not positive definite
+  *loss = 0;
+  for (double l : m.h_loss) *loss += l;
 #undef CKE
   return cudaSuccess;
 }
