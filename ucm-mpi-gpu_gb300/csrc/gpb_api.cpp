@@ -1914,9 +1914,12 @@ extern "C" gpb_status gpb_learned_forward_device(gpb_ctx* ctx, size_t n, const u
     if (st != GPB_OK) return st;
     cudaStream_t s = ctx->st;
     CK(ctx->net->features(d_mpb, d_deg, s));
-    CK(ctx->net->forward(s));
-    CK(cudaMemcpyAsync(d_y, ctx->net->y(), (size_t)ctx->net->npix0() * kLnOut * sizeof(float),
-                       cudaMemcpyDeviceToDevice, s));
+    // the head writes pairs of fields: straight to the caller where those are aligned
+    const bool direct = ((uintptr_t)d_y & 7u) == 0;
+    CK(ctx->net->forward(s, direct ? d_y : nullptr));
+    if (!direct)
+      CK(cudaMemcpyAsync(d_y, ctx->net->y(), (size_t)ctx->net->npix0() * kLnOut * sizeof(float),
+                         cudaMemcpyDeviceToDevice, s));
     CK(cudaStreamSynchronize(s));
     return GPB_OK;
   });

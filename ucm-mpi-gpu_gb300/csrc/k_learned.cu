@@ -17,7 +17,7 @@
 //   k_ln_wgrad   weight and bias gradients: a CTA accumulates dW = dZ^T X of
 //                all taps over its share of the tiles on the tensor cores,
 //                then adds it to the FP32 gradient.
-//   pooling, up-sampling + concatenation and their gradients, the subspace
+//   pooling, the gradients of pooling, up-sampling and concatenation, the subspace
 //   loss reductions and its gradient, Adam, the weights' BF16 copies.
 #include <cuda_bf16.h>
 #include <math.h>
@@ -60,8 +60,6 @@ typedef __nv_bfloat16 bf16;
 constexpr int TH = 8, TW = 16, HP = TH + 2, WP = TW + 2, NHALO = HP * WP;  // tile, halo tile
 constexpr int kConvThreads = 128;
 
-__device__ __forceinline__ uint32_t ld32(const bf16* p) { return *(const uint32_t*)p; }
-
 __device__ __forceinline__ void mma_bf16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
                                          uint32_t b0, uint32_t b1) {
   asm volatile(
@@ -76,15 +74,42 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
   return *(const uint32_t*)&v;
 }
 
+__device__ __forceinline__ void ldsm4(uint32_t (&r)[4], const bf16* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"((uint32_t)__cvta_generic_to_shared(p)));
+}
+
+// A convolution's BF16 input, CIN channels of pixel (y, x) of a patch: with
+// C1 = 0 one tensor; with C1 > 0 the concatenation of an up-sampled coarser
+// tensor (C1 channels, nearest) and a skip tensor, read where they lie.
+struct LnIn {
+  const bf16* x;        // the tensor, or the skip tensor
+  const bf16* coarse;   // C1 channels at the next coarser level
+  const LnPatch* cp;    // that level's patches
+};
+template <int CIN, int C1>
+__device__ __forceinline__ uint4 ln_in8(const LnIn& in, const LnPatch& P, const LnPatch& Q, int y, int x, int c) {
+  if (C1 > 0 && c < C1)
+    return *(const uint4*)(in.coarse + (Q.off + (long long)(y >> 1) * Q.W + (x >> 1)) * C1 + c);
+  return *(const uint4*)(in.x + (P.off + (long long)y * P.W + x) * (CIN - C1) + c - C1);
+}
+
 // MODE 0: forward, ReLU, BF16 out.  1: forward head, FP32 out.
-// 2: data gradient: `in` is the FP32 output gradient of the layer being
+// 2: data gradient: dA is the FP32 output gradient of the layer being
 //    differentiated (CIN = its channels), masked by its BF16 activation
 //    (mask, may be null) and rounded to BF16; w is the flipped, transposed
 //    weight; FP32 out, no bias.
-template <int CIN, int CO, int MODE>
+// A persistent CTA stages its weights once and walks the tiles blockIdx.x,
+// + gridDim.x, ...; fragments come by ldmatrix, one instruction for the four
+// registers that plain loads took four for.  Bound by the staging (memory)
+// for the thin layers, by fragment loads and mma.sync for the wide ones.
+// Measured, forward of 617 kpx, all 15: 357 us, from 392 us with the weights
+// staged per tile and 4-byte fragment loads.
+template <int CIN, int CO, int MODE, int C1>
 __global__ void __launch_bounds__(kConvThreads) k_ln_conv(const LnPatch* __restrict__ lp,
-                                                          const LnTile* __restrict__ tiles,
-                                                          const void* __restrict__ in,
+                                                          const LnTile* __restrict__ tiles, int ntiles, LnIn in,
+                                                          const float* __restrict__ dA,
                                                           const bf16* __restrict__ mask,
                                                           const bf16* __restrict__ w, const float* __restrict__ bias,
                                                           void* __restrict__ out, int cout_total) {
@@ -92,94 +117,105 @@ __global__ void __launch_bounds__(kConvThreads) k_ln_conv(const LnPatch* __restr
   extern __shared__ __align__(16) unsigned char smem_raw[];
   bf16* in_s = (bf16*)smem_raw;
   bf16* w_s = in_s + NHALO * SI;
-  const LnTile t = tiles[blockIdx.x];
-  const LnPatch P = lp[t.patch];
   const int co0 = blockIdx.y * CO;
-  // stage the input tile with its halo (zeros outside the patch)
-  for (int idx = threadIdx.x; idx < NHALO * (CIN / 8); idx += blockDim.x) {
-    const int h = idx / (CIN / 8), q = idx % (CIN / 8);
-    const int y = t.y0 - 1 + h / WP, x = t.x0 - 1 + h % WP;
-    uint4 v = make_uint4(0u, 0u, 0u, 0u);
-    if (y >= 0 && y < P.H && x >= 0 && x < P.W) {
-      const long long pix = P.off + (long long)y * P.W + x;
-      if constexpr (MODE == 2) {
-        const float* g = (const float*)in + pix * CIN + q * 8;
-        const float4 g0 = *(const float4*)g, g1 = *(const float4*)(g + 4);
-        float f[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
-        if (mask) {
-          const uint4 mk = *(const uint4*)(mask + pix * CIN + q * 8);
-          const bf16* m = (const bf16*)&mk;
-#pragma unroll
-          for (int k = 0; k < 8; k++)
-            if (!(__bfloat162float(m[k]) > 0.f)) f[k] = 0.f;
-        }
-        v = make_uint4(pack2(f[0], f[1]), pack2(f[2], f[3]), pack2(f[4], f[5]), pack2(f[6], f[7]));
-      } else {
-        v = *(const uint4*)((const bf16*)in + pix * CIN + q * 8);
-      }
-    }
-    *(uint4*)(in_s + h * SI + q * 8) = v;
-  }
-  // stage this CTA's output channels of the weights
+  // this CTA's output channels of the weights
   for (int idx = threadIdx.x; idx < CO * (9 * CIN / 8); idx += blockDim.x) {
     const int r = idx / (9 * CIN / 8), q = idx % (9 * CIN / 8);
     *(uint4*)(w_s + r * SW + q * 8) = *(const uint4*)(w + (long long)(co0 + r) * 9 * CIN + q * 8);
   }
-  __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tg = lane & 3;
-  float acc[2][CO / 8][4];
+  float bs[CO / 8][2];
 #pragma unroll
-  for (int mt = 0; mt < 2; mt++)
+  for (int nt = 0; nt < CO / 8; nt++) {
+    bs[nt][0] = MODE < 2 ? bias[co0 + nt * 8 + 2 * tg] : 0.f;
+    bs[nt][1] = MODE < 2 ? bias[co0 + nt * 8 + 2 * tg + 1] : 0.f;
+  }
+  // ldmatrix rows: A: tile pixel (lane & 15) at channel half lane >> 4;
+  // B: output channel (lane & 7) + 8 (lane >> 4) at channel half (lane >> 3) & 1
+  const bf16* arow = in_s + (2 * warp * WP + (lane & 15)) * SI + 8 * (lane >> 4);
+  const bf16* brow = w_s + ((lane & 7) + 8 * (lane >> 4)) * SW + 8 * ((lane >> 3) & 1);
+  for (int ti = blockIdx.x; ti < ntiles; ti += gridDim.x) {
+    const LnTile t = tiles[ti];
+    const LnPatch P = lp[t.patch], Q = C1 > 0 ? in.cp[t.patch] : P;
+    __syncthreads();
+    // the input tile with its halo (zeros outside the patch)
+    for (int idx = threadIdx.x; idx < NHALO * (CIN / 8); idx += blockDim.x) {
+      const int h = idx / (CIN / 8), q = idx % (CIN / 8);
+      const int y = t.y0 - 1 + h / WP, x = t.x0 - 1 + h % WP;
+      uint4 v = make_uint4(0u, 0u, 0u, 0u);
+      if (y >= 0 && y < P.H && x >= 0 && x < P.W) {
+        if constexpr (MODE == 2) {
+          const long long pix = P.off + (long long)y * P.W + x;
+          const float* gp = dA + pix * CIN + q * 8;
+          const float4 g0 = *(const float4*)gp, g1 = *(const float4*)(gp + 4);
+          float f[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
+          if (mask) {
+            const uint4 mk = *(const uint4*)(mask + pix * CIN + q * 8);
+            const bf16* m = (const bf16*)&mk;
 #pragma unroll
-    for (int nt = 0; nt < CO / 8; nt++)
-#pragma unroll
-      for (int k = 0; k < 4; k++) acc[mt][nt][k] = 0.f;
-#pragma unroll 1
-  for (int tap = 0; tap < 9; tap++) {
-    const int dy = tap / 3, dx = tap % 3;
-#pragma unroll
-    for (int kc = 0; kc < CIN / 16; kc++) {
-      uint32_t a[2][4];
-#pragma unroll
-      for (int mt = 0; mt < 2; mt++) {
-        const bf16* r0 = in_s + ((2 * warp + mt + dy) * WP + dx + g) * SI + kc * 16 + 2 * tg;
-        a[mt][0] = ld32(r0);
-        a[mt][1] = ld32(r0 + 8 * SI);
-        a[mt][2] = ld32(r0 + 8);
-        a[mt][3] = ld32(r0 + 8 * SI + 8);
+            for (int k = 0; k < 8; k++)
+              if (!(__bfloat162float(m[k]) > 0.f)) f[k] = 0.f;
+          }
+          v = make_uint4(pack2(f[0], f[1]), pack2(f[2], f[3]), pack2(f[4], f[5]), pack2(f[6], f[7]));
+        } else {
+          v = ln_in8<CIN, C1>(in, P, Q, y, x, q * 8);
+        }
       }
+      *(uint4*)(in_s + h * SI + q * 8) = v;
+    }
+    __syncthreads();
+    float acc[2][CO / 8][4];
 #pragma unroll
-      for (int nt = 0; nt < CO / 8; nt++) {
-        const bf16* wr = w_s + (nt * 8 + g) * SW + tap * CIN + kc * 16 + 2 * tg;
-        const uint32_t b0 = ld32(wr), b1 = ld32(wr + 8);
+    for (int mt = 0; mt < 2; mt++)
 #pragma unroll
-        for (int mt = 0; mt < 2; mt++) mma_bf16(acc[mt][nt], a[mt][0], a[mt][1], a[mt][2], a[mt][3], b0, b1);
+      for (int nt = 0; nt < CO / 8; nt++)
+#pragma unroll
+        for (int k = 0; k < 4; k++) acc[mt][nt][k] = 0.f;
+#pragma unroll 1
+    for (int tap = 0; tap < 9; tap++) {
+      const bf16* at = arow + ((tap / 3) * WP + tap % 3) * SI;
+      const bf16* bt = brow + tap * CIN;
+#pragma unroll
+      for (int kc = 0; kc < CIN / 16; kc++) {
+        uint32_t a[2][4];
+        ldsm4(a[0], at + kc * 16);
+        ldsm4(a[1], at + WP * SI + kc * 16);
+#pragma unroll
+        for (int nt = 0; nt < CO / 8; nt += 2) {
+          uint32_t b[4];
+          ldsm4(b, bt + nt * 8 * SW + kc * 16);
+#pragma unroll
+          for (int mt = 0; mt < 2; mt++) {
+            mma_bf16(acc[mt][nt], a[mt][0], a[mt][1], a[mt][2], a[mt][3], b[0], b[1]);
+            mma_bf16(acc[mt][nt + 1], a[mt][0], a[mt][1], a[mt][2], a[mt][3], b[2], b[3]);
+          }
+        }
       }
     }
-  }
-  // epilogue: accumulator rows are tile pixels x = g (c0, c1) and g + 8
-  // (c2, c3) of tile row 2 warp + mt; columns are channels 2 tg, 2 tg + 1
+    // accumulator rows are tile pixels x = g (c0, c1) and g + 8 (c2, c3) of
+    // tile row 2 warp + mt; columns are channels 2 tg, 2 tg + 1
 #pragma unroll
-  for (int mt = 0; mt < 2; mt++) {
-    const int y = t.y0 + 2 * warp + mt;
-    if (y >= P.H) continue;
+    for (int mt = 0; mt < 2; mt++) {
+      const int y = t.y0 + 2 * warp + mt;
+      if (y >= P.H) continue;
 #pragma unroll
-    for (int half = 0; half < 2; half++) {
-      const int x = t.x0 + g + 8 * half;
-      if (x >= P.W) continue;
-      const long long pix = P.off + (long long)y * P.W + x;
+      for (int half = 0; half < 2; half++) {
+        const int x = t.x0 + g + 8 * half;
+        if (x >= P.W) continue;
+        const long long pix = P.off + (long long)y * P.W + x;
 #pragma unroll
-      for (int nt = 0; nt < CO / 8; nt++) {
-        const int ch = co0 + nt * 8 + 2 * tg;
-        float v0 = acc[mt][nt][2 * half], v1 = acc[mt][nt][2 * half + 1];
-        if constexpr (MODE == 0) {
-          v0 = fmaxf(v0 + bias[ch], 0.f);
-          v1 = fmaxf(v1 + bias[ch + 1], 0.f);
-          *(uint32_t*)((bf16*)out + pix * cout_total + ch) = pack2(v0, v1);
-        } else if constexpr (MODE == 1) {
-          *(float2*)((float*)out + pix * cout_total + ch) = make_float2(v0 + bias[ch], v1 + bias[ch + 1]);
-        } else {
-          *(float2*)((float*)out + pix * cout_total + ch) = make_float2(v0, v1);
+        for (int nt = 0; nt < CO / 8; nt++) {
+          const int ch = co0 + nt * 8 + 2 * tg;
+          float v0 = acc[mt][nt][2 * half], v1 = acc[mt][nt][2 * half + 1];
+          if constexpr (MODE == 0) {
+            v0 = fmaxf(v0 + bs[nt][0], 0.f);
+            v1 = fmaxf(v1 + bs[nt][1], 0.f);
+            *(uint32_t*)((bf16*)out + pix * cout_total + ch) = pack2(v0, v1);
+          } else if constexpr (MODE == 1) {
+            *(float2*)((float*)out + pix * cout_total + ch) = make_float2(v0 + bs[nt][0], v1 + bs[nt][1]);
+          } else {
+            *(float2*)((float*)out + pix * cout_total + ch) = make_float2(v0, v1);
+          }
         }
       }
     }
@@ -222,11 +258,11 @@ struct WgradCfg {
   static constexpr size_t smem = stage > sums ? stage : sums;
   static_assert(CPW * WC * 8 == CC && CIN % CC == 0, "channel split");
 };
-template <int CIN, int CC, int COUT, int WC>
+template <int CIN, int CC, int COUT, int WC, int C1>
 __global__ void __launch_bounds__(256) k_ln_wgrad(const LnPatch* __restrict__ lp, const LnTile* __restrict__ tiles,
                                                   int ntiles, const float* __restrict__ dA,
-                                                  const bf16* __restrict__ mask, const bf16* __restrict__ X,
-                                                  float* __restrict__ dW, float* __restrict__ db) {
+                                                  const bf16* __restrict__ mask, LnIn X, float* __restrict__ dW,
+                                                  float* __restrict__ db) {
   using G = WgradCfg<CIN, CC, COUT, WC>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   bf16* dz_s = (bf16*)smem_raw;            // [128][ZP]
@@ -247,7 +283,7 @@ __global__ void __launch_bounds__(256) k_ln_wgrad(const LnPatch* __restrict__ lp
   float dbacc = 0.f;
   for (int ti = blockIdx.x; ti < ntiles; ti += gridDim.x) {
     const LnTile t = tiles[ti];
-    const LnPatch P = lp[t.patch];
+    const LnPatch P = lp[t.patch], Q = C1 > 0 ? X.cp[t.patch] : P;
     __syncthreads();
     for (int idx = threadIdx.x; idx < TH * TW * (COUT / 8); idx += blockDim.x) {
       const int px = idx / (COUT / 8), q = idx % (COUT / 8);
@@ -274,7 +310,7 @@ __global__ void __launch_bounds__(256) k_ln_wgrad(const LnPatch* __restrict__ lp
       const int y = t.y0 - 1 + h / WP, x = t.x0 - 1 + h % WP;
       uint4 v = make_uint4(0u, 0u, 0u, 0u);
       if (y >= 0 && y < P.H && x >= 0 && x < P.W)
-        v = *(const uint4*)(X + (P.off + (long long)y * P.W + x) * CIN + c0 + q * 8);
+        v = ln_in8<CIN, C1>(X, P, Q, y, x, c0 + q * 8);
       *(uint4*)(x_s + h * G::XP + q * 8) = v;
     }
     __syncthreads();
@@ -391,26 +427,7 @@ __global__ void k_ln_pool_bwd(const LnPatch* __restrict__ lo, const LnPatch* __r
   }
 }
 
-// concatenation [up(coarse), skip] at the fine level, BF16
-__global__ void k_ln_upcat(const LnPatch* __restrict__ lo, const LnPatch* __restrict__ hi, int C1, int C2,
-                           const bf16* __restrict__ coarse, const bf16* __restrict__ skip, bf16* __restrict__ out) {
-  const int p = blockIdx.y;
-  const LnPatch F = lo[p], Q = hi[p];
-  const int C = C1 + C2;
-  const uint32_t nq = C / 8, total = (uint32_t)F.H * F.W * nq;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
-    const uint32_t q = i % nq, px = i / nq;
-    const int y = (int)(px / F.W), x = (int)(px % F.W);
-    uint4 v;
-    if ((int)q * 8 < C1)
-      v = *(const uint4*)(coarse + (Q.off + (long long)(y >> 1) * Q.W + (x >> 1)) * C1 + q * 8);
-    else
-      v = *(const uint4*)(skip + (F.off + px) * C2 + (q * 8 - C1));
-    *(uint4*)(out + (F.off + px) * C + q * 8) = v;
-  }
-}
-
-// gradient of k_ln_upcat: the coarse part summed over each 2 x 2 block, the
+// gradient of the concatenation [up(coarse), skip]: the coarse part summed over each 2 x 2 block, the
 // skip part copied, FP32
 __global__ void k_ln_upcat_bwd_coarse(const LnPatch* __restrict__ lo, const LnPatch* __restrict__ hi, int C1,
                                       int C2, const float* __restrict__ dC, float* __restrict__ dcoarse) {
@@ -750,82 +767,90 @@ __global__ void k_ln_start(const LnPatch* __restrict__ lp, const PatchDev* __res
   }
 }
 
-template <int CIN, int CO, int MODE>
-cudaError_t conv_go(const LnPatch* lp, const LnTile* tiles, int ntiles, int cout, const void* in, const bf16* mask,
-                    const bf16* w, const float* bias, void* out, cudaStream_t s) {
+template <int CIN, int CO, int MODE, int C1>
+cudaError_t conv_go(const LnPatch* lp, const LnTile* tiles, int ntiles, int cout, const LnIn& in, const float* dA,
+                    const bf16* mask, const bf16* w, const float* bias, void* out, cudaStream_t s) {
   constexpr size_t smem = ((size_t)NHALO * (CIN + 8) + (size_t)CO * (9 * CIN + 8)) * sizeof(bf16);
   static bool attr = false;
   if (!attr) {
-    cudaFuncSetAttribute(k_ln_conv<CIN, CO, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaFuncSetAttribute(k_ln_conv<CIN, CO, MODE, C1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     attr = true;
   }
   if (ntiles == 0) return cudaSuccess;
-  k_ln_conv<CIN, CO, MODE><<<dim3(ntiles, cout / CO), kConvThreads, smem, s>>>(lp, tiles, in, mask, w, bias, out,
-                                                                               cout);
+  // Up to 16 input channels a tile per CTA: the weights are under 10 KB, and
+  // 12-16 CTAs per SM overlap one another's staging (62 us for the three of
+  // a forward of 617 kpx against 67 us persistent).  Wider layers: as many
+  // CTAs as fit the SMs together, in equal shares of the tiles, so the
+  // weights (up to 74 KB) are staged once (128 channels: 47 us against 69).
+  const int chunks = cout / CO;
+  const int fit = std::max(1, 152 * (int)std::min<size_t>(12, 227 * 1024 / (smem + 1024)) / chunks);
+  const int per = CIN <= 16 ? 1 : (ntiles + fit - 1) / fit;
+  k_ln_conv<CIN, CO, MODE, C1><<<dim3((ntiles + per - 1) / per, chunks), kConvThreads, smem, s>>>(
+      lp, tiles, ntiles, in, dA, mask, w, bias, out, cout);
   return cudaGetLastError();
 }
 
 // the instantiations the network uses: forward (mode 0 / 1) and data
 // gradient (mode 2, cin = the layer's cout, cout = its cin)
 cudaError_t conv_launch(int cin, int cout, int mode, const LnPatch* lp, const LnTile* tiles, int ntiles,
-                        const void* in, const bf16* mask, const bf16* w, const float* bias, void* out,
-                        cudaStream_t s) {
+                        const LnIn& in, const float* dA, const bf16* mask, const bf16* w, const float* bias,
+                        void* out, cudaStream_t s) {
   const bool c16 = (cout % 32) != 0;
-#define GO(CI, CO, M) return conv_go<CI, CO, M>(lp, tiles, ntiles, cout, in, mask, w, bias, out, s)
+#define GO(CI, CO, M, C1) return conv_go<CI, CO, M, C1>(lp, tiles, ntiles, cout, in, dA, mask, w, bias, out, s)
   if (mode == 0) {
     if (c16) {
-      if (cin == 16) GO(16, 16, 0);
-      if (cin == 48) GO(48, 16, 0);
+      if (cin == 16) GO(16, 16, 0, 0);
+      if (cin == 48) GO(48, 16, 0, 32);
     } else {
-      if (cin == 16) GO(16, 32, 0);
-      if (cin == 32) GO(32, 32, 0);
-      if (cin == 64) GO(64, 32, 0);
-      if (cin == 96) GO(96, 32, 0);
-      if (cin == 128) GO(128, 32, 0);
+      if (cin == 16) GO(16, 32, 0, 0);
+      if (cin == 32) GO(32, 32, 0, 0);
+      if (cin == 64) GO(64, 32, 0, 0);
+      if (cin == 96) GO(96, 32, 0, 64);
+      if (cin == 128) GO(128, 32, 0, 64);
     }
   } else if (mode == 1) {
-    if (cin == 16 && !c16) GO(16, 32, 1);
+    if (cin == 16 && !c16) GO(16, 32, 1, 0);
   } else {
     if (c16) {
-      if (cin == 16) GO(16, 16, 2);
-      if (cin == 32) GO(32, 16, 2);
+      if (cin == 16) GO(16, 16, 2, 0);
+      if (cin == 32) GO(32, 16, 2, 0);
     } else {
-      if (cin == 32) GO(32, 32, 2);
-      if (cin == 64) GO(64, 32, 2);
+      if (cin == 32) GO(32, 32, 2, 0);
+      if (cin == 64) GO(64, 32, 2, 0);
     }
   }
 #undef GO
   return cudaErrorInvalidValue;
 }
 
-template <int CIN, int CC, int COUT, int WC>
+template <int CIN, int CC, int COUT, int WC, int C1>
 cudaError_t wgrad_go(const LnPatch* lp, const LnTile* tiles, int ntiles, const float* dA, const bf16* mask,
-                     const bf16* X, float* dW, float* db, cudaStream_t s) {
+                     const LnIn& X, float* dW, float* db, cudaStream_t s) {
   using G = WgradCfg<CIN, CC, COUT, WC>;
   static bool attr = false;
   if (!attr) {
-    cudaFuncSetAttribute(k_ln_wgrad<CIN, CC, COUT, WC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G::smem);
+    cudaFuncSetAttribute(k_ln_wgrad<CIN, CC, COUT, WC, C1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G::smem);
     attr = true;
   }
   // about two CTAs per SM over the channel chunks; one where a thread's sums
   // take most of its registers
   constexpr int chunks = CIN / CC, per_sm = G::CPW * G::NT >= 4 ? 1 : 2;
   const dim3 grid(std::max(1, std::min(ntiles, 152 * per_sm / chunks)), chunks);
-  k_ln_wgrad<CIN, CC, COUT, WC><<<grid, 256, G::smem, s>>>(lp, tiles, ntiles, dA, mask, X, dW, db);
+  k_ln_wgrad<CIN, CC, COUT, WC, C1><<<grid, 256, G::smem, s>>>(lp, tiles, ntiles, dA, mask, X, dW, db);
   return cudaGetLastError();
 }
 cudaError_t wgrad_launch(int cin, int cout, const LnPatch* lp, const LnTile* tiles, int ntiles, const float* dA,
-                         const bf16* mask, const bf16* X, float* dW, float* db, cudaStream_t s) {
+                         const bf16* mask, const LnIn& X, float* dW, float* db, cudaStream_t s) {
   if (ntiles == 0) return cudaSuccess;
-#define GO(CI, CC, CO, WC) return wgrad_go<CI, CC, CO, WC>(lp, tiles, ntiles, dA, mask, X, dW, db, s)
-  if (cin == 16 && cout == 16) GO(16, 16, 16, 2);
-  if (cin == 16 && cout == 32) GO(16, 16, 32, 2);
-  if (cin == 32 && cout == 32) GO(32, 32, 32, 4);
-  if (cin == 32 && cout == 64) GO(32, 32, 64, 4);
-  if (cin == 64 && cout == 64) GO(64, 64, 64, 8);
-  if (cin == 128 && cout == 64) GO(128, 64, 64, 8);
-  if (cin == 96 && cout == 32) GO(96, 32, 32, 4);
-  if (cin == 48 && cout == 16) GO(48, 48, 16, 2);
+#define GO(CI, CC, CO, WC, C1) return wgrad_go<CI, CC, CO, WC, C1>(lp, tiles, ntiles, dA, mask, X, dW, db, s)
+  if (cin == 16 && cout == 16) GO(16, 16, 16, 2, 0);
+  if (cin == 16 && cout == 32) GO(16, 16, 32, 2, 0);
+  if (cin == 32 && cout == 32) GO(32, 32, 32, 4, 0);
+  if (cin == 32 && cout == 64) GO(32, 32, 64, 4, 0);
+  if (cin == 64 && cout == 64) GO(64, 64, 64, 8, 0);
+  if (cin == 128 && cout == 64) GO(128, 64, 64, 8, 64);
+  if (cin == 96 && cout == 32) GO(96, 32, 32, 4, 64);
+  if (cin == 48 && cout == 16) GO(48, 48, 16, 2, 32);
 #undef GO
   return cudaErrorInvalidValue;
 }
@@ -844,6 +869,7 @@ struct LearnedNet::Impl {
   float *am = nullptr, *av = nullptr;  // Adam moments
   bf16 *wb = nullptr, *wt = nullptr;   // BF16 weights, flipped-transposed BF16 weights
   bool have = false;
+  std::vector<int> h, w;  // the sizes that the layout below was built for
   std::vector<LnPatch> lp[kLnLevels];
   std::vector<LnTile> lt[kLnLevels];
   long long npix[kLnLevels] = {0, 0, 0, 0}, maxpix[kLnLevels] = {0, 0, 0, 0};
@@ -864,7 +890,7 @@ struct LearnedNet::Impl {
   size_t cap_gram = 0, cap_cm = 0, cap_ploss = 0, cap_bad = 0;
   std::vector<double> h_loss;
   // named tensors
-  bf16 *X0, *A0a, *S0, *C0, *A0c, *A0d, *P0, *A1a, *S1, *C1, *A1c, *A1d, *P1, *A2a, *S2, *C2, *A2c, *A2d, *P2,
+  bf16 *X0, *A0a, *S0, *A0c, *A0d, *P0, *A1a, *S1, *A1c, *A1d, *P1, *A2a, *S2, *A2c, *A2d, *P2,
       *A3a, *A3b;
   float *dY, *dA0d, *dA0c, *dC0, *dS0, *dA0a, *dA1d, *dA1c, *dC1, *dS1, *dA1a, *dP0, *dA2d, *dA2c, *dC2, *dS2,
       *dA2a, *dP1, *dA3b, *dA3a, *dP2;
@@ -891,23 +917,26 @@ struct LearnedNet::Impl {
     launches++;
     return cudaGetLastError();
   }
-  cudaError_t conv(int l, int level, const void* in, void* out, cudaStream_t s) {
+  LnIn one(const bf16* x) const { return {x, nullptr, nullptr}; }
+  // [up-sampled coarse, skip] at a level
+  LnIn cat(int level, const bf16* coarse, const bf16* skip) const { return {skip, coarse, d_lp[level + 1]}; }
+  cudaError_t conv(int l, int level, const LnIn& in, void* out, cudaStream_t s) {
     launches++;
     return conv_launch(kLnNet[l].cin, kLnNet[l].cout, kLnNet[l].relu ? 0 : 1, d_lp[level], d_lt[level],
-                       (int)lt[level].size(), in, nullptr, wb + wo[l], w32 + bo[l], out, s);
+                       (int)lt[level].size(), in, nullptr, nullptr, wb + wo[l], w32 + bo[l], out, s);
   }
   // backward of convolution l: dA (FP32 gradient of its output), mask (its
   // BF16 output; null for the head), X (its input); the data gradient into
   // dX unless null
-  cudaError_t conv_bwd(int l, int level, const float* dA, const bf16* mask, const bf16* X, float* dX,
+  cudaError_t conv_bwd(int l, int level, const float* dA, const bf16* mask, const LnIn& X, float* dX,
                        cudaStream_t s) {
     cudaError_t e = wgrad_launch(kLnNet[l].cin, kLnNet[l].cout, d_lp[level], d_lt[level], (int)lt[level].size(), dA,
                                  mask, X, grad + wo[l], grad + bo[l], s);
     launches++;
     if (e != cudaSuccess || !dX) return e;
     launches++;
-    return conv_launch(kLnNet[l].cout, kLnNet[l].cin, 2, d_lp[level], d_lt[level], (int)lt[level].size(), dA, mask,
-                       wt + wo[l], nullptr, dX, s);
+    return conv_launch(kLnNet[l].cout, kLnNet[l].cin, 2, d_lp[level], d_lt[level], (int)lt[level].size(), LnIn{},
+                       dA, mask, wt + wo[l], nullptr, dX, s);
   }
 };
 
@@ -967,6 +996,8 @@ cudaError_t LearnedNet::get_params(float* hp, cudaStream_t s) {
 cudaError_t LearnedNet::layout(const std::vector<int>& H, const std::vector<int>& W, cudaStream_t s) {
   Impl& m = *im_;
   const int n = (int)H.size();
+  if (H == m.h && W == m.w) return cudaSuccess;  // the tables and tensors of these sizes are in place
+  m.h.clear();  // until all of it is
   for (int l = 0; l < kLnLevels; l++) {
     m.lp[l].clear();
     m.lt[l].clear();
@@ -998,8 +1029,8 @@ cudaError_t LearnedNet::layout(const std::vector<int>& H, const std::vector<int>
   // channel counts of the BF16 activations per level, then of the FP32
   // gradients; each tensor is its level's pixel count times its channels
   const long long N0 = m.npix[0], N1 = m.npix[1], N2 = m.npix[2], N3 = m.npix[3];
-  const size_t act_need = N0 * (16 + 16 + 16 + 48 + 16 + 16) + N1 * (16 + 32 + 32 + 96 + 32 + 32) +
-                          N2 * (32 + 64 + 64 + 128 + 64 + 64) + N3 * (64 + 64 + 64);
+  const size_t act_need = N0 * (16 + 16 + 16 + 16 + 16) + N1 * (16 + 32 + 32 + 32 + 32) +
+                          N2 * (32 + 64 + 64 + 64 + 64) + N3 * (64 + 64 + 64);
   const size_t gr_need = N0 * (32 + 16 + 16 + 48 + 16 + 16) + N1 * (32 + 32 + 96 + 32 + 32 + 16) +
                          N2 * (64 + 64 + 128 + 64 + 64 + 32) + N3 * (64 + 64 + 64);
   cudaError_t e;
@@ -1016,9 +1047,9 @@ cudaError_t LearnedNet::layout(const std::vector<int>& H, const std::vector<int>
     a += N * C;
     return r;
   };
-  m.X0 = A(N0, 16), m.A0a = A(N0, 16), m.S0 = A(N0, 16), m.C0 = A(N0, 48), m.A0c = A(N0, 16), m.A0d = A(N0, 16);
-  m.P0 = A(N1, 16), m.A1a = A(N1, 32), m.S1 = A(N1, 32), m.C1 = A(N1, 96), m.A1c = A(N1, 32), m.A1d = A(N1, 32);
-  m.P1 = A(N2, 32), m.A2a = A(N2, 64), m.S2 = A(N2, 64), m.C2 = A(N2, 128), m.A2c = A(N2, 64), m.A2d = A(N2, 64);
+  m.X0 = A(N0, 16), m.A0a = A(N0, 16), m.S0 = A(N0, 16), m.A0c = A(N0, 16), m.A0d = A(N0, 16);
+  m.P0 = A(N1, 16), m.A1a = A(N1, 32), m.S1 = A(N1, 32), m.A1c = A(N1, 32), m.A1d = A(N1, 32);
+  m.P1 = A(N2, 32), m.A2a = A(N2, 64), m.S2 = A(N2, 64), m.A2c = A(N2, 64), m.A2d = A(N2, 64);
   m.P2 = A(N3, 64), m.A3a = A(N3, 64), m.A3b = A(N3, 64);
   float* g = m.gr;
   auto G = [&](long long N, int C) {
@@ -1030,6 +1061,8 @@ cudaError_t LearnedNet::layout(const std::vector<int>& H, const std::vector<int>
   m.dA1d = G(N1, 32), m.dA1c = G(N1, 32), m.dC1 = G(N1, 96), m.dS1 = G(N1, 32), m.dA1a = G(N1, 32), m.dP0 = G(N1, 16);
   m.dA2d = G(N2, 64), m.dA2c = G(N2, 64), m.dC2 = G(N2, 128), m.dS2 = G(N2, 64), m.dA2a = G(N2, 64), m.dP1 = G(N2, 32);
   m.dA3b = G(N3, 64), m.dA3a = G(N3, 64), m.dP2 = G(N3, 64);
+  m.h = H;
+  m.w = W;
   return cudaSuccess;
 }
 
@@ -1049,7 +1082,7 @@ cudaError_t LearnedNet::features_from(const PatchDev* patches, const float* d_mp
   return cudaGetLastError();
 }
 
-cudaError_t LearnedNet::forward(cudaStream_t s) {
+cudaError_t LearnedNet::forward(cudaStream_t s, float* out) {
   Impl& m = *im_;
   if (!m.have) return cudaErrorInvalidValue;
   const int np = (int)m.lp[0].size();
@@ -1063,33 +1096,24 @@ cudaError_t LearnedNet::forward(cudaStream_t s) {
     m.launches++;
     return cudaGetLastError();
   };
-  auto upcat = [&](int l, int C1, int C2, const bf16* coarse, const bf16* skip, bf16* out) {
-    k_ln_upcat<<<pix_grid(m.maxpix[l] * ((C1 + C2) / 8), np), 256, 0, s>>>(m.d_lp[l], m.d_lp[l + 1], C1, C2, coarse,
-                                                                           skip, out);
-    m.launches++;
-    return cudaGetLastError();
-  };
-  CKE(m.conv(0, 0, m.X0, m.A0a, s));
-  CKE(m.conv(1, 0, m.A0a, m.S0, s));
+  CKE(m.conv(0, 0, m.one(m.X0), m.A0a, s));
+  CKE(m.conv(1, 0, m.one(m.A0a), m.S0, s));
   CKE(pool(0, 16, m.S0, m.P0));
-  CKE(m.conv(2, 1, m.P0, m.A1a, s));
-  CKE(m.conv(3, 1, m.A1a, m.S1, s));
+  CKE(m.conv(2, 1, m.one(m.P0), m.A1a, s));
+  CKE(m.conv(3, 1, m.one(m.A1a), m.S1, s));
   CKE(pool(1, 32, m.S1, m.P1));
-  CKE(m.conv(4, 2, m.P1, m.A2a, s));
-  CKE(m.conv(5, 2, m.A2a, m.S2, s));
+  CKE(m.conv(4, 2, m.one(m.P1), m.A2a, s));
+  CKE(m.conv(5, 2, m.one(m.A2a), m.S2, s));
   CKE(pool(2, 64, m.S2, m.P2));
-  CKE(m.conv(6, 3, m.P2, m.A3a, s));
-  CKE(m.conv(7, 3, m.A3a, m.A3b, s));
-  CKE(upcat(2, 64, 64, m.A3b, m.S2, m.C2));
-  CKE(m.conv(8, 2, m.C2, m.A2c, s));
-  CKE(m.conv(9, 2, m.A2c, m.A2d, s));
-  CKE(upcat(1, 64, 32, m.A2d, m.S1, m.C1));
-  CKE(m.conv(10, 1, m.C1, m.A1c, s));
-  CKE(m.conv(11, 1, m.A1c, m.A1d, s));
-  CKE(upcat(0, 32, 16, m.A1d, m.S0, m.C0));
-  CKE(m.conv(12, 0, m.C0, m.A0c, s));
-  CKE(m.conv(13, 0, m.A0c, m.A0d, s));
-  CKE(m.conv(14, 0, m.A0d, m.y, s));
+  CKE(m.conv(6, 3, m.one(m.P2), m.A3a, s));
+  CKE(m.conv(7, 3, m.one(m.A3a), m.A3b, s));
+  CKE(m.conv(8, 2, m.cat(2, m.A3b, m.S2), m.A2c, s));
+  CKE(m.conv(9, 2, m.one(m.A2c), m.A2d, s));
+  CKE(m.conv(10, 1, m.cat(1, m.A2d, m.S1), m.A1c, s));
+  CKE(m.conv(11, 1, m.one(m.A1c), m.A1d, s));
+  CKE(m.conv(12, 0, m.cat(0, m.A1d, m.S0), m.A0c, s));
+  CKE(m.conv(13, 0, m.one(m.A0c), m.A0d, s));
+  CKE(m.conv(14, 0, m.one(m.A0d), out ? out : m.y, s));
   return cudaSuccess;
 }
 
@@ -1126,27 +1150,27 @@ cudaError_t LearnedNet::loss_backward(const float* d_v, double* loss, cudaStream
     m.launches += 2;
     return cudaGetLastError();
   };
-  CKE(m.conv_bwd(14, 0, m.dY, nullptr, m.A0d, m.dA0d, s));
-  CKE(m.conv_bwd(13, 0, m.dA0d, m.A0d, m.A0c, m.dA0c, s));
-  CKE(m.conv_bwd(12, 0, m.dA0c, m.A0c, m.C0, m.dC0, s));
+  CKE(m.conv_bwd(14, 0, m.dY, nullptr, m.one(m.A0d), m.dA0d, s));
+  CKE(m.conv_bwd(13, 0, m.dA0d, m.A0d, m.one(m.A0c), m.dA0c, s));
+  CKE(m.conv_bwd(12, 0, m.dA0c, m.A0c, m.cat(0, m.A1d, m.S0), m.dC0, s));
   CKE(upcat_bwd(0, 32, 16, m.dC0, m.dA1d, m.dS0));
-  CKE(m.conv_bwd(11, 1, m.dA1d, m.A1d, m.A1c, m.dA1c, s));
-  CKE(m.conv_bwd(10, 1, m.dA1c, m.A1c, m.C1, m.dC1, s));
+  CKE(m.conv_bwd(11, 1, m.dA1d, m.A1d, m.one(m.A1c), m.dA1c, s));
+  CKE(m.conv_bwd(10, 1, m.dA1c, m.A1c, m.cat(1, m.A2d, m.S1), m.dC1, s));
   CKE(upcat_bwd(1, 64, 32, m.dC1, m.dA2d, m.dS1));
-  CKE(m.conv_bwd(9, 2, m.dA2d, m.A2d, m.A2c, m.dA2c, s));
-  CKE(m.conv_bwd(8, 2, m.dA2c, m.A2c, m.C2, m.dC2, s));
+  CKE(m.conv_bwd(9, 2, m.dA2d, m.A2d, m.one(m.A2c), m.dA2c, s));
+  CKE(m.conv_bwd(8, 2, m.dA2c, m.A2c, m.cat(2, m.A3b, m.S2), m.dC2, s));
   CKE(upcat_bwd(2, 64, 64, m.dC2, m.dA3b, m.dS2));
-  CKE(m.conv_bwd(7, 3, m.dA3b, m.A3b, m.A3a, m.dA3a, s));
-  CKE(m.conv_bwd(6, 3, m.dA3a, m.A3a, m.P2, m.dP2, s));
+  CKE(m.conv_bwd(7, 3, m.dA3b, m.A3b, m.one(m.A3a), m.dA3a, s));
+  CKE(m.conv_bwd(6, 3, m.dA3a, m.A3a, m.one(m.P2), m.dP2, s));
   CKE(pool_bwd(2, 64, m.dP2, m.dS2));
-  CKE(m.conv_bwd(5, 2, m.dS2, m.S2, m.A2a, m.dA2a, s));
-  CKE(m.conv_bwd(4, 2, m.dA2a, m.A2a, m.P1, m.dP1, s));
+  CKE(m.conv_bwd(5, 2, m.dS2, m.S2, m.one(m.A2a), m.dA2a, s));
+  CKE(m.conv_bwd(4, 2, m.dA2a, m.A2a, m.one(m.P1), m.dP1, s));
   CKE(pool_bwd(1, 32, m.dP1, m.dS1));
-  CKE(m.conv_bwd(3, 1, m.dS1, m.S1, m.A1a, m.dA1a, s));
-  CKE(m.conv_bwd(2, 1, m.dA1a, m.A1a, m.P0, m.dP0, s));
+  CKE(m.conv_bwd(3, 1, m.dS1, m.S1, m.one(m.A1a), m.dA1a, s));
+  CKE(m.conv_bwd(2, 1, m.dA1a, m.A1a, m.one(m.P0), m.dP0, s));
   CKE(pool_bwd(0, 16, m.dP0, m.dS0));
-  CKE(m.conv_bwd(1, 0, m.dS0, m.S0, m.A0a, m.dA0a, s));
-  CKE(m.conv_bwd(0, 0, m.dA0a, m.A0a, m.X0, nullptr, s));
+  CKE(m.conv_bwd(1, 0, m.dS0, m.S0, m.one(m.A0a), m.dA0a, s));
+  CKE(m.conv_bwd(0, 0, m.dA0a, m.A0a, m.one(m.X0), nullptr, s));
   int bad = 0;
   m.h_loss.resize(np);
   CKE(cudaMemcpyAsync(m.h_loss.data(), m.ploss, np * sizeof(double), cudaMemcpyDeviceToHost, s));

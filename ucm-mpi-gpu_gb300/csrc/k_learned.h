@@ -52,8 +52,9 @@ class LearnedNet {
   // the same from the pipeline's buffers: mPb at each patch's pixel offset,
   // degree at its vector offset
   cudaError_t features_from(const PatchDev* patches, const float* d_mpb, const float* d_deg, cudaStream_t s);
-  // forward pass; the 32 fields land in y() (FP32, [pixel][32], level-0 offsets)
-  cudaError_t forward(cudaStream_t s);
+  // forward pass; the 32 fields (FP32, [pixel][32], level-0 offsets) land in
+  // out (8-byte aligned), or in y() without it
+  cudaError_t forward(cudaStream_t s, float* out = nullptr);
   float* y();
   // the subspace loss of y() against the 9 orthonormal target fields of each
   // patch (d_v: [pixel][9] FP32 at the level-0 offsets), and the gradient of
