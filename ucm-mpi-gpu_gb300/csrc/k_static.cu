@@ -94,7 +94,11 @@ cudaError_t launch_texton_static(const uint32_t* packed, int W, int H, uint32_t*
   k_static_setup<<<(ntiles + 255) / 256, 256, 0, s>>>(P, tiles_x, ntiles, base);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   if ((e = launch_convert(packed, N, grey, lab4, s)) != cudaSuccess) return e;
-  if ((e = launch_texton(dP, work, ntiles, grey, lab4, repair, count, (int)N, s)) != cudaSuccess) return e;
+  // Split each tile's groups until the tiles fill the SMs.  Whole calls, in us,
+  // with 1 / 2 / 4 sets of threads per tile: 100 tiles 126 / 100 / 83, 256 tiles
+  // 128 / 108 / 114, 1600 tiles 324 / 315 / 406, 2500 tiles 454 / 467 / 618.
+  const int variant = ntiles <= 152 ? 2 : ntiles < 2048 ? 1 : 0;
+  if ((e = launch_texton(dP, work, ntiles, grey, lab4, repair, count, (int)N, s, variant)) != cudaSuccess) return e;
   return launch_texton_repair(dP, grey, lab4, repair, count, (int)N, k32_ring, ring_of, n_rings, s);
 }
 

@@ -18,7 +18,7 @@ cudaError_t launch_convert(const uint32_t* packed, long long n, uint8_t* grey, u
 cudaError_t launch_lab_table(uint32_t* table, cudaStream_t s);
 cudaError_t launch_convert_lut(const uint32_t* packed, long long n, const uint32_t* table, uint8_t* grey,
                                uint32_t* lab4, cudaStream_t s);
-// variant 0, 1, 2: 32, 64 or 128 threads per 16 x 16 tile (identical labels)
+// variant 0, 1, 2: 64, 128 or 256 threads per 16 x 16 tile (identical labels)
 constexpr int kTextonVariants = 3;
 cudaError_t launch_texton(const PatchDev* patches, const int4* work, int nwork, const uint8_t* grey,
                           uint32_t* lab4, int* repair_list, int* repair_count, int repair_cap,
