@@ -196,8 +196,7 @@ typedef struct {
  * order.  d_nmax (width*height floats) and d_orient (8*width*height, plane
  * after plane) receive row-major image planes in the patch output's plane
  * order; pixels no patch covers are left as they were.  Device pointers;
- * synchronous on the context's stream.  BLEND uses a context buffer of
- * 10*width*height floats. */
+ * synchronous on the context's stream. */
 gpb_status gpb_stitch_device(gpb_ctx* ctx, int mode, uint32_t width, uint32_t height, const gpb_place* places,
                              size_t n, int ramp, float* d_nmax, float* d_orient);
 

@@ -134,9 +134,8 @@ struct Buf {
   float* cblk[4] = {nullptr, nullptr, nullptr, nullptr}; size_t c_cblk[4] = {0, 0, 0, 0};
   float* afull = nullptr; size_t c_afull = 0;  // fine stencil rows in the block step's tile layout
   int4* work_act = nullptr; size_t c_wact = 0;  // 16 x 16 tiles of the still active patches
-  float* stitch = nullptr; size_t c_stitch = 0;  // BLEND accumulators [10][image]
-  uint32_t* spcount = nullptr; size_t c_spcount = 0;          // superpixel histograms
-  unsigned long long* spcsum = nullptr; size_t c_spcsum = 0;  // superpixel colour sums
+  StitchBox* stitch = nullptr; size_t c_stitch = 0;  // the boxes of a stitch
+  unsigned long long* spsum = nullptr; size_t c_spsum = 0;  // superpixel colour sums, then histograms
   int* berr = nullptr; size_t c_berr = 0;
 };
 
@@ -534,7 +533,7 @@ extern "C" void gpb_destroy(gpb_ctx* ctx) {
                   b.tiles, b.tile_begin, b.tile_count, ctx->d_ic, ctx->d_k32_ring, ctx->d_ring_of,
                   b.blk[0], b.blk[1], b.blk[2], b.blk[3], b.bpart, b.bgram, b.bgram2, b.bmat, b.btheta, b.bres,
                   b.bcoef, b.bdone, b.cpatches, b.ctiles, b.ctile_begin, b.ctile_count,
-                  b.cwork16, b.cwc, b.cdeg, b.cdis, b.cblk[0], b.cblk[1], b.cblk[2], b.cblk[3], b.afull, b.berr, b.work_act, b.stitch, b.spcount, b.spcsum};
+                  b.cwork16, b.cwc, b.cdeg, b.cdis, b.cblk[0], b.cblk[1], b.cblk[2], b.cblk[3], b.afull, b.berr, b.work_act, b.stitch, b.spsum};
   for (void* q : ptrs)
     if (q) cudaFree(q);
   if (ctx->h_packed) cudaFreeHost(ctx->h_packed);
@@ -1771,37 +1770,20 @@ extern "C" gpb_status gpb_stitch_device(gpb_ctx* ctx, int mode, uint32_t width, 
     cudaStream_t s = ctx->st;
     Buf& b = ctx->b;
     const int colmajor = ctx->prm.compat == GPB_COMPAT_DAMASCENE;
-    const long long plane = (long long)width * height;
-    if (mode == GPB_STITCH_BLEND) {
-      CK(grow(b.stitch, b.c_stitch, 10 * (size_t)plane));
-      CK(cudaMemsetAsync(b.stitch, 0, 10 * (size_t)plane * sizeof(float), s));
-    }
     const float rmp = (float)(ramp > 0 ? ramp : 10);
+    std::vector<StitchBox> boxes(n);
     for (size_t i = 0; i < n; i++) {
       const gpb_place& q = places[i];
       const PatchDev& P = ctx->patches[i];
-      StitchBox bx;
-      bx.ox = q.x0;
-      bx.oy = q.y0;
-      if (mode == GPB_STITCH_INTERIOR) {
-        bx.x = q.ix;
-        bx.y = q.iy;
-        bx.w = q.iw;
-        bx.h = q.ih;
-      } else {
-        bx.x = 0;
-        bx.y = 0;
-        bx.w = P.W;
-        bx.h = P.H;
-      }
-      if (mode == GPB_STITCH_BLEND)
-        CK(launch_stitch_acc(b.patches, (int)i, P.N, b.nmax, b.orient, colmajor, bx, (int)width, (int)height, rmp,
-                             b.stitch, s));
+      if (mode == GPB_STITCH_INTERIOR)
+        boxes[i] = {q.x0, q.y0, q.ix, q.iy, q.iw, q.ih};
       else
-        CK(launch_stitch_copy(b.patches, (int)i, b.nmax, b.orient, colmajor, bx, (int)width, (int)height, d_nmax,
-                              d_orient, s));
+        boxes[i] = {q.x0, q.y0, 0, 0, P.W, P.H};
     }
-    if (mode == GPB_STITCH_BLEND) CK(launch_stitch_norm(b.stitch, plane, d_nmax, d_orient, s));
+    CK(grow(b.stitch, b.c_stitch, n));
+    CK(cudaMemcpyAsync(b.stitch, boxes.data(), n * sizeof(StitchBox), cudaMemcpyHostToDevice, s));
+    CK(launch_stitch(b.patches, b.stitch, (int)n, mode == GPB_STITCH_BLEND, b.nmax, b.orient, colmajor, (int)width,
+                     (int)height, rmp, d_nmax, d_orient, s));
     CK(cudaStreamSynchronize(s));
     return GPB_OK;
   });
@@ -1818,10 +1800,10 @@ extern "C" gpb_status gpb_superpixel_features(gpb_ctx* ctx, size_t patch, const 
     cudaStream_t s = ctx->st;
     Buf& b = ctx->b;
     const int K = with_textons ? ctx->K : 0, nbins = 255 / bin_step + 1;
-    CK(grow(b.spcount, b.c_spcount, (size_t)n_labels * (K + nbins + 1)));
-    CK(grow(b.spcsum, b.c_spcsum, (size_t)n_labels * 3));
+    const size_t nsum = (size_t)n_labels * 3, ncount = (size_t)n_labels * (K + nbins + 1);
+    CK(grow(b.spsum, b.c_spsum, nsum + (ncount + 1) / 2));
     CK(launch_sp_features(b.patches, (int)patch, ctx->patches[patch].N, d_labels, n_labels, b.lab4, b.grey, b.packed,
-                          bin_step, K, nbins, b.spcount, b.spcsum, d_out, s));
+                          bin_step, K, nbins, b.spsum, (uint32_t*)(b.spsum + nsum), d_out, s));
     CK(cudaStreamSynchronize(s));
     return GPB_OK;
   });

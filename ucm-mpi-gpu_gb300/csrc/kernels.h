@@ -61,18 +61,16 @@ cudaError_t launch_spb(const PatchDev* patches, const int4* work, int nwork, con
 struct StitchBox {
   int ox, oy, x, y, w, h;
 };
-cudaError_t launch_stitch_copy(const PatchDev* patches, int pi, const float* nmax, const float* orient, int colmajor,
-                               const StitchBox& bx, int img_w, int img_h, float* out_nmax, float* out_orient,
-                               cudaStream_t s);
-cudaError_t launch_stitch_acc(const PatchDev* patches, int pi, long long npix, const float* nmax, const float* orient,
-                              int colmajor, const StitchBox& bx, int img_w, int img_h, float ramp, float* acc,
-                              cudaStream_t s);
-cudaError_t launch_stitch_norm(const float* acc, long long plane, float* out_nmax, float* out_orient, cudaStream_t s);
+// whole-image planes from n patches' boxes (device arrays, patch order): the
+// last covering box's values, or (blend) their weighted mean
+cudaError_t launch_stitch(const PatchDev* patches, const StitchBox* boxes, int n, bool blend, const float* nmax,
+                          const float* orient, int colmajor, int img_w, int img_h, float ramp, float* out_nmax,
+                          float* out_orient, cudaStream_t s);
 
 // k_spfeat.cu
 cudaError_t launch_sp_features(const PatchDev* patches, int pi, long long npix, const int32_t* labels, int n,
                                const uint32_t* lab4, const uint8_t* grey, const uint32_t* packed, int bin_step,
-                               int K, int nbins, uint32_t* counts, unsigned long long* csum, double* out,
+                               int K, int nbins, unsigned long long* csum, uint32_t* counts, double* out,
                                cudaStream_t s);
 
 }  // namespace gpb
