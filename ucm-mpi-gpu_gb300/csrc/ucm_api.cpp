@@ -5,8 +5,8 @@
 // A call takes a batch of images, the pieces that the reference gives to
 // one MPI rank each (src/main.cpp:456-459): the images are flooded together
 // (one CTA each), their contour fitting and merging run on the context's
-// host thread pool, one image per thread, and the data-parallel stages run
-// image after image on the context's stream.
+// host thread pool, one image per thread, and each data-parallel stage is one
+// launch over all images.
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <string.h>
@@ -28,7 +28,7 @@ size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
 
 // where image i's slices start in the batch's concatenated arrays
 struct Offsets {
-  size_t pix, pix4, rows, rows2, grid2, bsum;
+  size_t pix, pix4, rows, rows2, grid2, bsum, border;
 };
 
 struct UcmState {
@@ -41,6 +41,7 @@ struct UcmState {
   float* orient = nullptr;  // staging of host planes
   size_t cap_orient = 0;
   std::vector<UcmScratch> views;  // image i's slices of the batch arrays
+  UcmView* d_views = nullptr;     // in base: the images as the kernels see them
   std::vector<int> H, W;          // the last call's images
 };
 
@@ -70,7 +71,7 @@ cudaError_t grow_dev(T*& p, size_t& cap, size_t need) {
 cudaError_t ucm_reserve(UcmState& u, const std::vector<int>& H, const std::vector<int>& W) {
   const size_t n = H.size();
   std::vector<Offsets> off(n + 1);
-  off[0] = {0, 0, 0, 0, 0, 0};
+  off[0] = {0, 0, 0, 0, 0, 0, 0};
   for (size_t i = 0; i < n; i++) {
     const size_t N = (size_t)H[i] * W[i];
     off[i + 1].pix = off[i].pix + N;
@@ -79,12 +80,13 @@ cudaError_t ucm_reserve(UcmState& u, const std::vector<int>& H, const std::vecto
     off[i + 1].rows2 = off[i].rows2 + 2 * H[i] + 1;
     off[i + 1].grid2 = off[i].grid2 + (size_t)(2 * H[i] + 1) * (2 * W[i] + 1);
     off[i + 1].bsum = off[i].bsum + 4 * N / 4096 + 2;
+    off[i + 1].border = off[i].border + (size_t)(H[i] + 2) * (W[i] + 2);
   }
   const Offsets& T = off[n];
-  // slots: mm, pb, q, off, cols, img, ws, bw, wswt, pb2, rowcnt, nart, art, par, rank, bsum, nreg, labels, wswt2
-  const size_t sizes[] = {2 * n * 4, T.pix * 4, T.pix, T.rows * 257 * 4, T.pix * 2, n * sizeof(UcmImage), T.pix * 4,
+  // slots: mm, pb, q, off, cols, img, ws, bw, wswt, pb2, rowcnt, nart, art, par, rank, bsum, nreg, labels, wswt2, views
+  const size_t sizes[] = {2 * n * 4, T.pix * 4, T.pix, T.rows * 257 * 4, T.pix * 2, n * sizeof(UcmImage), T.border * 4,
                           T.pix, T.pix * 4, T.pix4 * 4, T.rows2 * 4, n * 4, T.pix4 * 4, T.pix4 * 4, T.pix4 * 4,
-                          T.bsum * 4, n * 4, T.pix * 4, T.grid2 * 4};
+                          T.bsum * 4, n * 4, T.pix * 4, T.grid2 * 4, n * sizeof(UcmView)};
   constexpr size_t kSlots = sizeof(sizes) / sizeof(sizes[0]);
   size_t need = 0;
   for (size_t b : sizes) need += align256(b);
@@ -102,6 +104,7 @@ cudaError_t ucm_reserve(UcmState& u, const std::vector<int>& H, const std::vecto
     base[k] = p;
     p += align256(sizes[k]);
   }
+  u.d_views = (UcmView*)base[19];
   u.views.assign(n, UcmScratch{});
   for (size_t i = 0; i < n; i++) {
     const Offsets& o = off[i];
@@ -112,7 +115,7 @@ cudaError_t ucm_reserve(UcmState& u, const std::vector<int>& H, const std::vecto
     v.off = (int32_t*)base[3] + o.rows * 257;
     v.cols = (uint16_t*)base[4] + o.pix;
     v.img = (UcmImage*)base[5] + i;
-    v.ws = (int32_t*)base[6] + o.pix;
+    v.ws = (int32_t*)base[6];
     v.bw = (uint8_t*)base[7] + o.pix;
     v.wswt = (float*)base[8] + o.pix;
     v.pb2 = (float*)base[9] + o.pix4;
@@ -185,12 +188,23 @@ extern "C" gpb_status gpb_ucm_batch(gpb_ctx* ctx, size_t n, const uint32_t* widt
       }
     }
     std::vector<UcmImage> imgs(n);
-    for (size_t i = 0; i < n; i++)
-      imgs[i] = {H[i], W[i], (long long)pix[i], (int)((u.views[i].off - u.views[0].off) / 257)};
+    long long ws_cells = 0;
+    for (size_t i = 0; i < n; i++) {
+      imgs[i] = {H[i], W[i], (long long)pix[i], (int)((u.views[i].off - u.views[0].off) / 257), ws_cells};
+      ws_cells += (long long)(H[i] + 2) * (W[i] + 2);
+    }
     UCK(cudaMemcpyAsync(u.views[0].img, imgs.data(), n * sizeof(UcmImage), cudaMemcpyHostToDevice, st));
-    // device: orientation max, quantisation and row sort per image, then one flooding launch for all
-    for (size_t i = 0; i < n; i++) UCK(ucm_prepare(d_orient[i], H[i], W[i], u.views[i], st));
-    UCK(ucm_flood(ni, (long long)pix[n], u.views[0], st));
+    // device: orientation max, quantisation, row sort and flooding
+    std::vector<UcmView> views(n);
+    UcmBatch batch = {u.d_views, ni, 0, 0, (long long)pix[n], 0, ws_cells};
+    for (size_t i = 0; i < n; i++) {
+      views[i] = {u.views[i], d_orient[i], H[i], W[i], 0};
+      batch.max_h = std::max(batch.max_h, H[i]);
+      batch.max_pix = std::max(batch.max_pix, (long long)N[i]);
+    }
+    UCK(cudaMemcpyAsync(u.d_views, views.data(), n * sizeof(UcmView), cudaMemcpyHostToDevice, st));
+    UCK(ucm_prepare(batch, u.views[0], st));
+    UCK(ucm_flood(batch, u.views[0], st));
     std::vector<uint8_t> bw(pix[n]);
     UCK(cudaMemcpyAsync(bw.data(), u.views[0].bw, pix[n], cudaMemcpyDeviceToHost, st));
     UCK(cudaStreamSynchronize(st));
@@ -211,25 +225,35 @@ extern "C" gpb_status gpb_ucm_batch(gpb_ctx* ctx, size_t n, const uint32_t* widt
       ms_fit_i[i] = ms_since(ti);
     });
     const double ms_fit = ms_since(t1);
-    // device: painting, super contour, cleaning, labelling, image after image
+    // device: painting, super contour, cleaning, labelling
     const auto t2 = std::chrono::steady_clock::now();
     std::vector<size_t> poff(n + 1, 0);
     for (size_t i = 0; i < n; i++) poff[i + 1] = poff[i] + ppix[i].size();
     UCK(grow_dev(u.paint_pix, u.cap_pix, poff[n]));
     UCK(grow_dev(u.paint_ori, u.cap_ori, poff[n]));
-    for (size_t i = 0; i < n; i++) {
-      const int np = (int)ppix[i].size();
-      if (np) {
-        UCK(cudaMemcpyAsync(u.paint_pix + poff[i], ppix[i].data(), (size_t)np * sizeof(int32_t),
-                            cudaMemcpyHostToDevice, st));
-        UCK(cudaMemcpyAsync(u.paint_ori + poff[i], pori[i].data(), (size_t)np, cudaMemcpyHostToDevice, st));
-      }
-      UcmScratch v = u.views[i];
-      v.paint_pix = u.paint_pix + poff[i];
-      v.paint_ori = u.paint_ori + poff[i];
-      UCK(ucm_paint(d_orient[i], H[i], W[i], np, v, st));
-      UCK(ucm_mid(H[i], W[i], v, st));
+    if (n > 1) {  // one list for all images: one copy each of pixels and planes
+      std::vector<int32_t> all_pix(poff[n]);
+      std::vector<uint8_t> all_ori(poff[n]);
+      ctx_parallel_for(ctx, ni, [&](int i) {
+        std::copy(ppix[i].begin(), ppix[i].end(), all_pix.begin() + poff[i]);
+        std::copy(pori[i].begin(), pori[i].end(), all_ori.begin() + poff[i]);
+      });
+      ppix[0].swap(all_pix);
+      pori[0].swap(all_ori);
     }
+    if (poff[n]) {
+      UCK(cudaMemcpyAsync(u.paint_pix, ppix[0].data(), poff[n] * sizeof(int32_t), cudaMemcpyHostToDevice, st));
+      UCK(cudaMemcpyAsync(u.paint_ori, pori[0].data(), poff[n], cudaMemcpyHostToDevice, st));
+    }
+    for (size_t i = 0; i < n; i++) {
+      views[i].s.paint_pix = u.paint_pix + poff[i];
+      views[i].s.paint_ori = u.paint_ori + poff[i];
+      views[i].np = (int)(poff[i + 1] - poff[i]);
+      batch.max_paint = std::max(batch.max_paint, views[i].np);
+    }
+    UCK(cudaMemcpyAsync(u.d_views, views.data(), n * sizeof(UcmView), cudaMemcpyHostToDevice, st));
+    UCK(ucm_paint(batch, u.views[0], st));
+    UCK(ucm_mid(batch, st));
     std::vector<size_t> g2(n + 1, 0);
     for (size_t i = 0; i < n; i++) g2[i + 1] = g2[i] + (size_t)(2 * H[i] + 1) * (2 * W[i] + 1);
     std::vector<float> w2(g2[n]);

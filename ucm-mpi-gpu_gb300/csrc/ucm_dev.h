@@ -9,16 +9,17 @@ struct UcmImage {
   int H, W;
   long long pix;  // first pixel of the image in the per-pixel arrays
   int row0;       // first row in the per-row arrays
+  long long wpix; // first cell in the flooding's labels, which have a border of one pixel
 };
 
 struct UcmScratch {
-  unsigned* mm;        // ordered min, max of pb
+  unsigned* mm;        // complement of the ordered min, ordered max of pb
   float* pb;           // N
   uint8_t* q;          // N
   int32_t* off;        // H x 257
   uint16_t* cols;      // N
   UcmImage* img;       // this image's entry of the batch's image table
-  int32_t* ws;         // N
+  int32_t* ws;         // all images' flooding labels, (H+2)(W+2) each
   uint8_t* bw;         // N
   float* wswt;         // N
   int32_t* paint_pix;  // painted pixels
@@ -35,12 +36,27 @@ struct UcmScratch {
   float* wswt2;        // (2H+1)(2W+1)
 };
 
-// per image: max over orientations, quantisation, per-row level sort
-cudaError_t ucm_prepare(const float* d_orient, int H, int W, UcmScratch& s, cudaStream_t st);
-// all images of a batch: flooding (one CTA each) and the watershed-pixel map;
-// base is image 0's view, whose arrays start the batch's concatenated ones
-cudaError_t ucm_flood(int nimg, long long total_pix, const UcmScratch& base, cudaStream_t st);
-cudaError_t ucm_paint(const float* d_orient, int H, int W, int npaint, UcmScratch& s, cudaStream_t st);
-cudaError_t ucm_mid(int H, int W, UcmScratch& s, cudaStream_t st);
+// one image of a batch, as the kernels see it (blockIdx.y)
+struct UcmView {
+  UcmScratch s;
+  const float* orient;  // 8 planes
+  int H, W, np;         // np: painted pixels
+};
+// what sizes the launches of a batch
+struct UcmBatch {
+  const UcmView* views;  // device, n entries
+  int n, max_h;
+  long long max_pix, total_pix;
+  int max_paint;
+  long long ws_cells;    // of all images' flooding labels
+};
+
+// max over orientations, quantisation, per-row level sort; base is image 0's
+// view, whose arrays start the batch's concatenated ones
+cudaError_t ucm_prepare(const UcmBatch& b, const UcmScratch& base, cudaStream_t st);
+// flooding (one CTA per image) and the watershed-pixel map
+cudaError_t ucm_flood(const UcmBatch& b, const UcmScratch& base, cudaStream_t st);
+cudaError_t ucm_paint(const UcmBatch& b, const UcmScratch& base, cudaStream_t st);
+cudaError_t ucm_mid(const UcmBatch& b, cudaStream_t st);
 
 }  // namespace gpb
