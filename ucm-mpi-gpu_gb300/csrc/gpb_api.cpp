@@ -1230,7 +1230,8 @@ static gpb_status solve_block(gpb_ctx* ctx, const Level& lv, bool have_start, do
         bool trial = false;
         const int v = decided ? chosen : ctx->tuner.pick(step_key(nwb), kStepVariants, 3, chosen, &trial);
         if (trial) ctx->tuner.begin(step_key(nwb), v, s);
-        const cudaError_t e = cf_launch_step(a, work_blk, nwb, buf[c], buf[prv], buf[nxt], k, s, false, v);
+        const bool overlap = k > 0 && decided && !ctx->profile;  // no event between it and the step before
+        const cudaError_t e = cf_launch_step(a, work_blk, nwb, buf[c], buf[prv], buf[nxt], k, s, false, v, overlap);
         if (trial) ctx->tuner.end(s);
         if (e != cudaSuccess) return e;
         prof_end(ctx);

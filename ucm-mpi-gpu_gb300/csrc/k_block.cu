@@ -29,6 +29,7 @@
 #include "gpb_internal.h"
 #include "k_block.h"
 #include "k_eig.h"
+#include "overlap.h"
 
 namespace gpb {
 
@@ -335,8 +336,11 @@ __global__ void __launch_bounds__((WARPS + 2) * 32, 1) cf_step_t(BlkArgs a, cons
     }
   }
   __syncthreads();
+  // the next step's CTAs may set up and fetch coefficients as this one's end
+  overlap_release();
   if (warp >= WARPS) {  // ------------------------------------- producers
     if (lane != 0) return;
+    if (warp == WARPS) overlap_wait();  // Y; the operator does not change within a chain of steps
     int i = 0;
     for (int t = blockIdx.x; t < nwork * SUB; t += gridDim.x) {
       const int4 w = work[t / SUB];
@@ -412,6 +416,7 @@ __global__ void __launch_bounds__((WARPS + 2) * 32, 1) cf_step_t(BlkArgs a, cons
   ring.empty = cempty;
   ring.n0 = 0;
   ring.bad = false;
+  overlap_wait();  // X, and the readers of out
   for (int i = 0;; i++, ring.n0 += SM::NG) {
     const int st = i & 1;
     if (!mbar_wait(yfull + st, (i >> 1) & 1)) {
@@ -1031,18 +1036,18 @@ static void step_attrs() {
 }
 
 template <class S, bool C>
-static void step_go(const BlkArgs& a, const int4* work, int nwork, const float* Y, const float* X, float* out,
-                    int step, int nsm, int variant, cudaStream_t s) {
+static cudaError_t step_go(const BlkArgs& a, const int4* work, int nwork, const float* Y, const float* X, float* out,
+                           int step, int nsm, int variant, bool overlap, cudaStream_t s) {
   // one persistent CTA per SM
   if (variant == 0)
-    cf_step_t<S, C, 8><<<std::min(nwork, nsm), 10 * 32, StepSmem<S, 8>::bytes, s>>>(a, work, nwork, Y, X, out, step);
-  else
-    cf_step_t<S, C, 4><<<std::min(2 * nwork, nsm), 6 * 32, StepSmem<S, 4>::bytes, s>>>(a, work, nwork, Y, X, out,
-                                                                                       step);
+    return launch_overlap(cf_step_t<S, C, 8>, std::min(nwork, nsm), 10 * 32, StepSmem<S, 8>::bytes, s, overlap, a, work,
+                          nwork, Y, X, out, step);
+  return launch_overlap(cf_step_t<S, C, 4>, std::min(2 * nwork, nsm), 6 * 32, StepSmem<S, 4>::bytes, s, overlap, a, work,
+                        nwork, Y, X, out, step);
 }
 
 cudaError_t cf_launch_step(const BlkArgs& a, const int4* work, int nwork, const float* Y, const float* X, float* out,
-                           int step, cudaStream_t s, bool comp, int variant) {
+                           int step, cudaStream_t s, bool comp, int variant, bool overlap) {
   static int nsm = 0;
   if (!nsm) {
     int dev = 0;
@@ -1053,14 +1058,14 @@ cudaError_t cf_launch_step(const BlkArgs& a, const int4* work, int nwork, const 
     if (nsm <= 0) nsm = 1;
   }
   if (nwork <= 0) return cudaSuccess;
-  if (a.coarse) {
-    if (comp) step_go<SquareStencil, true>(a, work, nwork, Y, X, out, step, nsm, variant, s);
-    else step_go<SquareStencil, false>(a, work, nwork, Y, X, out, step, nsm, variant, s);
-  } else {
-    if (comp) step_go<DiskStencil, true>(a, work, nwork, Y, X, out, step, nsm, variant, s);
-    else step_go<DiskStencil, false>(a, work, nwork, Y, X, out, step, nsm, variant, s);
-  }
-  return cudaGetLastError();
+  cudaError_t e;
+  if (a.coarse)
+    e = comp ? step_go<SquareStencil, true>(a, work, nwork, Y, X, out, step, nsm, variant, overlap, s)
+             : step_go<SquareStencil, false>(a, work, nwork, Y, X, out, step, nsm, variant, overlap, s);
+  else
+    e = comp ? step_go<DiskStencil, true>(a, work, nwork, Y, X, out, step, nsm, variant, overlap, s)
+             : step_go<DiskStencil, false>(a, work, nwork, Y, X, out, step, nsm, variant, overlap, s);
+  return e != cudaSuccess ? e : cudaGetLastError();
 }
 cudaError_t cf_launch_full(const PatchDev* patches, const int4* work16, int nwork, const float* a_up,
                            const float* a_diag, long long lvec, float* afull, cudaStream_t s) {

@@ -62,8 +62,11 @@ constexpr int kBlkSplit = 4;  // CTAs per eigensolver tile in cf_gram / cf_rotat
 // variant (bit-identical results, chosen by the autotuner): 0 computes 16 x 16
 // pixels per CTA and pass, 1 halves them (for launches of few tiles)
 constexpr int kStepVariants = 2, kStepDefault = 0;
+// overlap: the launch before it on the stream is a step with the same active
+// patches, tiles and operator, whose tail this one's set-up may overlap
 cudaError_t cf_launch_step(const BlkArgs& a, const int4* work, int nwork, const float* Y, const float* X, float* out,
-                           int step, cudaStream_t s, bool comp = false, int variant = kStepDefault);
+                           int step, cudaStream_t s, bool comp = false, int variant = kStepDefault,
+                           bool overlap = false);
 // out = U^T V per patch; with out2, out2 = U^T U in the same pass
 cudaError_t cf_launch_gram(const BlkArgs& a, int ntiles, const float* U, const float* V, double* out,
                            cudaStream_t s, double* out2 = nullptr);

@@ -1,0 +1,42 @@
+// overlap.h -- programmatic dependent launch: a kernel of a fixed chain starts
+// its set-up while the one before it finishes.
+//
+// The kernel calls overlap_release() when its successor may be scheduled (its
+// CTAs then start as resources allow) and overlap_wait() before it touches
+// anything that an earlier kernel of the chain writes, or writes anything that
+// one reads: the wait returns when the kernel before it has completed, and that
+// one had waited for its own predecessor.  Both do nothing in a kernel that was
+// launched without `overlap`.
+//
+// Measured: 4.63 ms for one 64 x 80 image through the warm solver, 4.95 ms
+// without it (217 block steps of about 6 us); nothing at 16 patches of 266^2,
+// whose steps fill every SM until they end, nor for the three kernels of a
+// Lanczos step, whose tail is one CTA's reduction.
+#pragma once
+
+#include <cuda_runtime.h>
+
+namespace gpb {
+
+__device__ __forceinline__ void overlap_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void overlap_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// overlap: the launch before it on the stream is a kernel that calls
+// overlap_release()
+template <class... P, class... A>
+cudaError_t launch_overlap(void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t s, bool overlap,
+                           A... args) {
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = at;
+  cfg.numAttrs = overlap ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
+}  // namespace gpb
