@@ -1082,7 +1082,7 @@ static gpb_status solve_block(gpb_ctx* ctx, const Level& lv, bool have_start, do
   // orthonormalisation into the same host step; AF receives A F.
   // comp: compensated Rayleigh-Ritz product and rotation (see cf_step_t, cf_rotate)
   auto rr = [&](float* F, float* AF, bool comp) -> gpb_status {
-    CK(cf_launch_gram(a, nt, F, F, b.bgram, s));
+    CK(cf_launch_gram(a, np, nt, F, F, b.bgram, s));
     CK(cudaMemcpyAsync(G.data(), b.bgram, np * BB * sizeof(double), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
     ctx->tuner.collect();
@@ -1096,11 +1096,11 @@ static gpb_status solve_block(gpb_ctx* ctx, const Level& lv, bool have_start, do
     CK(cf_launch_rotate(a, nt, F, nullptr, kBlk, s));
     CK(upload_unit());
     CK(cf_launch_step(a, work_blk, nwb, F, F, AF, 0, s, comp, step_variant(nwb)));
-    CK(cf_launch_gram(a, nt, F, AF, b.bgram, s, b.bgram2));  // G = F^T AF and G2 = F^T F in one pass
+    CK(cf_launch_gram(a, np, nt, F, AF, b.bgram, s, b.bgram2));  // G = F^T AF and G2 = F^T F in one pass
     CK(cudaMemcpyAsync(G2.data(), b.bgram2, np * BB * sizeof(double), cudaMemcpyDeviceToHost, s));
     CK(cudaMemcpyAsync(G.data(), b.bgram, np * BB * sizeof(double), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
-    ctx->launches += 4;
+    ctx->launches += 6;
     ctx->host_pool().run(np, [&](int i) {
       if (!active[i]) return;
       mv[i] += kBlk;

@@ -11,7 +11,7 @@
 //              recurrence, Zhou & Saad 2007; with alpha=1, beta=gamma=0 it
 //              is the plain block SpMV)
 //   cf_gram    G = U^T V per patch (32 x 32), FP32 FMA runs folded into
-//              float-float sums, summed across CTAs by the patch's last CTA
+//              float-float sums, summed across CTAs by cf_gram_sum
 //   cf_rotate  U <- U M (32 x 32 per patch), optionally V <- V M too
 //   cf_resid   |A x_c - theta_c x_c|^2 per column
 //   cf_extract the first nvec columns into separate vectors (sPb layout)
@@ -552,20 +552,20 @@ __device__ __forceinline__ void ffp(float& hi, float& lo, float a, float b) {
 // accurate as a compensated one at about the cost of plain FMAs; the four
 // groups and then the tiles are summed in FP64.
 constexpr int GR_CH = 256;  // pixels per staged chunk
-__device__ __forceinline__ void two_sum_into(float& hi, float& lo, float x) {
-  const float s = hi + x;
-  const float bb = s - hi;
-  lo += (hi - (s - bb)) + (x - bb);
+__device__ __forceinline__ void two_sum_into(F2& hi, F2& lo, F2 x) {
+  const F2 s = f2_add(hi, x);
+  const F2 bb = f2_sub(s, hi);
+  lo = f2_add(lo, f2_add(f2_sub(hi, f2_sub(s, bb)), f2_sub(x, bb)));
   hi = s;
 }
 
 // The reductions and the rotation split each eigensolver tile (kEigTile
 // pixels) into kBlkSplit runs, one CTA each, so a launch has several CTAs
 // per SM and no near-empty last wave.  A CTA's partial sums are float-float
-// pairs in slot blockIdx.x of a.part; the last CTA of a patch adds the
-// slots [tile_begin, tile_begin + tile_count) x kBlkSplit in order, in
-// float-float on the FP32 pipes (one SM adding them in FP64 would take tens
-// of microseconds at GB300's FP64 rate).
+// pairs in slot blockIdx.x of a.part; the slots [tile_begin, tile_begin +
+// tile_count) x kBlkSplit of a patch are added in order, in float-float on the
+// FP32 pipes (FP64 would take tens of microseconds at GB300's rate): by
+// cf_gram_sum, or for cf_resid by the patch's last CTA.
 __device__ __forceinline__ void ff2_add(float2& s, float2 b) {
   const float t = s.x + b.x;
   const float z = t - s.x;
@@ -598,12 +598,20 @@ __device__ __forceinline__ bool blk_last(const BlkArgs& a, int patch) {
   if (is_last) __threadfence();
   return is_last;
 }
-// sum of element e over the patch's CTA slots (stride floats2 per slot)
+// sum of element e over the patch's CTA slots (stride floats2 per slot), in
+// order; the loads of 32 slots are in flight together
 __device__ __forceinline__ double blk_sum(const BlkArgs& a, int patch, int e, int stride) {
-  const float2* part = (const float2*)a.part;
+  constexpr int NB = 32;
   const int b0 = a.tile_begin[patch] * kBlkSplit, b1 = b0 + a.tile_count[patch] * kBlkSplit;
+  const float2* part = (const float2*)a.part + (long long)b0 * stride + e;
   float2 acc = make_float2(0.f, 0.f);
-  for (int b = b0; b < b1; b++) ff2_add(acc, part[(long long)b * stride + e]);
+  for (int b = b0; b < b1; b += NB, part += (long long)NB * stride) {
+    float2 v[NB];
+#pragma unroll
+    for (int i = 0; i < NB; i++) v[i] = b + i < b1 ? part[(long long)i * stride] : make_float2(0.f, 0.f);
+#pragma unroll
+    for (int i = 0; i < NB; i++) ff2_add(acc, v[i]);  // a pair of zeros changes nothing
+  }
   return (double)acc.x + (double)acc.y;
 }
 
@@ -612,8 +620,7 @@ __device__ __forceinline__ double blk_sum(const BlkArgs& a, int patch, int e, in
 // same order as a pass of its own, so the results are the same to the bit.
 template <bool TWO>
 __global__ void __launch_bounds__(256, TWO ? 2 : 3) cf_gram(BlkArgs a, const float* __restrict__ U,
-                                                            const float* __restrict__ V, double* __restrict__ out,
-                                                            double* __restrict__ out2) {
+                                                            const float* __restrict__ V) {
   const BlkRun run = blk_run(a);
   const EigTile t = run.t;
   if (!a.active[t.patch]) return;
@@ -624,11 +631,11 @@ __global__ void __launch_bounds__(256, TWO ? 2 : 3) cf_gram(BlkArgs a, const flo
   const int grp = threadIdx.x >> 6, lt = threadIdx.x & 63;
   const int i0 = (lt >> 3) * 4, j0 = (lt & 7) * 4;
   constexpr int NG = TWO ? 2 : 1;  // Gram matrices formed
-  float hi[NG][16], lo[NG][16];
+  F2 hi[NG][8], lo[NG][8];         // pairs of columns: [row of the 4 x 4 block][pair]
 #pragma unroll
   for (int g = 0; g < NG; g++)
 #pragma unroll
-    for (int k = 0; k < 16; k++) hi[g][k] = lo[g][k] = 0.f;
+    for (int k = 0; k < 8; k++) hi[g][k] = lo[g][k] = f2(0.f, 0.f);
   for (int p0 = run.p0; p0 < run.p1; p0 += GR_CH) {
     __syncthreads();
     for (int f = threadIdx.x; f < GR_CH * kBlk / 4; f += blockDim.x) {
@@ -643,34 +650,35 @@ __global__ void __launch_bounds__(256, TWO ? 2 : 3) cf_gram(BlkArgs a, const flo
       ((float4*)vs)[f] = v;
     }
     __syncthreads();
-    float acc[NG][16];
+    F2 acc[NG][8];
 #pragma unroll
     for (int g = 0; g < NG; g++)
 #pragma unroll
-      for (int k = 0; k < 16; k++) acc[g][k] = 0.f;
+      for (int k = 0; k < 8; k++) acc[g][k] = f2(0.f, 0.f);
     const int pbeg = grp * (GR_CH / 4);
 #pragma unroll(TWO ? 2 : 4)
     for (int pp = pbeg; pp < pbeg + GR_CH / 4; pp++) {
       const float4 u4 = *(const float4*)(us + pp * kBlk + i0);
       const float4 v4 = *(const float4*)(vs + pp * kBlk + j0);
-      const float uu[4] = {u4.x, u4.y, u4.z, u4.w}, vv[4] = {v4.x, v4.y, v4.z, v4.w};
+      const F2 uu[4] = {f2(u4.x, u4.x), f2(u4.y, u4.y), f2(u4.z, u4.z), f2(u4.w, u4.w)};
+      const F2 vv[2] = {f2(v4.x, v4.y), f2(v4.z, v4.w)};
 #pragma unroll
       for (int r = 0; r < 4; r++)
 #pragma unroll
-        for (int c = 0; c < 4; c++) acc[0][r * 4 + c] = fmaf(uu[r], vv[c], acc[0][r * 4 + c]);
+        for (int c = 0; c < 2; c++) acc[0][r * 2 + c] = f2_fma(uu[r], vv[c], acc[0][r * 2 + c]);
       if constexpr (TWO) {
         const float4 w4 = *(const float4*)(us + pp * kBlk + j0);
-        const float ww[4] = {w4.x, w4.y, w4.z, w4.w};
+        const F2 ww[2] = {f2(w4.x, w4.y), f2(w4.z, w4.w)};
 #pragma unroll
         for (int r = 0; r < 4; r++)
 #pragma unroll
-          for (int c = 0; c < 4; c++) acc[NG - 1][r * 4 + c] = fmaf(uu[r], ww[c], acc[NG - 1][r * 4 + c]);
+          for (int c = 0; c < 2; c++) acc[NG - 1][r * 2 + c] = f2_fma(uu[r], ww[c], acc[NG - 1][r * 2 + c]);
       }
     }
 #pragma unroll
     for (int g = 0; g < NG; g++)
 #pragma unroll
-      for (int k = 0; k < 16; k++) two_sum_into(hi[g][k], lo[g][k], acc[g][k]);
+      for (int k = 0; k < 8; k++) two_sum_into(hi[g][k], lo[g][k], acc[g][k]);
   }
   // the four groups' blocks, summed in float-float
   __syncthreads();
@@ -678,8 +686,12 @@ __global__ void __launch_bounds__(256, TWO ? 2 : 3) cf_gram(BlkArgs a, const flo
 #pragma unroll
   for (int g = 0; g < NG; g++)
 #pragma unroll
-    for (int k = 0; k < 16; k++)
-      red[(g * 4 + grp) * kBlk * kBlk + (i0 + k / 4) * kBlk + j0 + k % 4] = make_float2(hi[g][k], lo[g][k]);
+    for (int k = 0; k < 8; k++) {
+      const float2 h = f2_split(hi[g][k]), l = f2_split(lo[g][k]);
+      float2* at = red + (g * 4 + grp) * kBlk * kBlk + (i0 + k / 2) * kBlk + j0 + 2 * (k % 2);
+      at[0] = make_float2(h.x, l.x);
+      at[1] = make_float2(h.y, l.y);
+    }
   __syncthreads();
   float2* part = (float2*)a.part + (long long)blockIdx.x * NG * kBlk * kBlk;
   for (int e = threadIdx.x; e < NG * kBlk * kBlk; e += blockDim.x) {
@@ -688,11 +700,18 @@ __global__ void __launch_bounds__(256, TWO ? 2 : 3) cf_gram(BlkArgs a, const flo
     for (int q = 1; q < 4; q++) ff2_add(sum, red[(g * 4 + q) * kBlk * kBlk + el]);
     part[e] = sum;
   }
-  if (!blk_last(a, t.patch)) return;
-  for (int e = threadIdx.x; e < NG * kBlk * kBlk; e += blockDim.x) {
-    const int g = e / (kBlk * kBlk), el = e % (kBlk * kBlk);
-    (g ? out2 : out)[(long long)t.patch * kBlk * kBlk + el] = blk_sum(a, t.patch, e, NG * kBlk * kBlk);
-  }
+}
+
+// The Gram matrices' sums over a patch's CTA slots, 128 elements per CTA: a
+// patch of 0.4 Mpx has 800 slots (13 MB for two matrices), which its last
+// cf_gram CTA alone took longer to add than the others to form.
+constexpr int kSumThreads = 128;
+__global__ void __launch_bounds__(kSumThreads) cf_gram_sum(BlkArgs a, int ngram, double* __restrict__ out,
+                                                           double* __restrict__ out2) {
+  const int patch = blockIdx.x, e = blockIdx.y * kSumThreads + threadIdx.x;
+  if (!a.active[patch]) return;
+  const int g = e / (kBlk * kBlk), el = e % (kBlk * kBlk);
+  (g ? out2 : out)[(long long)patch * kBlk * kBlk + el] = blk_sum(a, patch, e, ngram * kBlk * kBlk);
 }
 
 // U <- U M (and V <- V M if V), M = a.mat[patch] (32 x 32, FP64 on the
@@ -757,47 +776,48 @@ __global__ void __launch_bounds__(256) cf_rotate(BlkArgs a, float* __restrict__ 
         }
 #pragma unroll 1
       for (int c0 = 0; c0 < kBlk; c0 += 4) {
-        float hi[2][4], lo[2][4], g[2][4];
+        F2 hi[2][2], lo[2][2], g[2][2];  // pairs of columns
 #pragma unroll
         for (int k = 0; k < 2; k++)
 #pragma unroll
-          for (int j = 0; j < 4; j++) hi[k][j] = lo[k][j] = g[k][j] = 0.f;
+          for (int j = 0; j < 2; j++) hi[k][j] = lo[k][j] = g[k][j] = f2(0.f, 0.f);
 #pragma unroll
         for (int r = 0; r < kBlk; r++) {
           const float4 h4 = *(const float4*)&mh[r][c0];  // broadcast: every thread reads the same row
-          const float hh[4] = {h4.x, h4.y, h4.z, h4.w};
-          float ll[4] = {0.f, 0.f, 0.f, 0.f};
+          const F2 hh[2] = {f2(h4.x, h4.y), f2(h4.z, h4.w)};
+          F2 ll[2] = {f2(0.f, 0.f), f2(0.f, 0.f)};
           if constexpr (C) {
             const float4 l4 = *(const float4*)&ml[r][c0];
-            ll[0] = l4.x;
-            ll[1] = l4.y;
-            ll[2] = l4.z;
-            ll[3] = l4.w;
+            ll[0] = f2(l4.x, l4.y);
+            ll[1] = f2(l4.z, l4.w);
           }
 #pragma unroll
-          for (int k = 0; k < 2; k++)
+          for (int k = 0; k < 2; k++) {
+            const F2 xr = f2(x[k][r], x[k][r]);
 #pragma unroll
-            for (int j = 0; j < 4; j++) {
+            for (int j = 0; j < 2; j++) {
               if constexpr (C) {
-                g[k][j] = fmaf(x[k][r], hh[j], g[k][j]);
-                lo[k][j] = fmaf(x[k][r], ll[j], lo[k][j]);
+                g[k][j] = f2_fma(xr, hh[j], g[k][j]);
+                lo[k][j] = f2_fma(xr, ll[j], lo[k][j]);
                 if ((r & 3) == 3) {  // r is a compile-time constant here
-                  const float sum = hi[k][j] + g[k][j], z = sum - hi[k][j];
-                  lo[k][j] += (hi[k][j] - (sum - z)) + (g[k][j] - z);
+                  const F2 sum = f2_add(hi[k][j], g[k][j]), z = f2_sub(sum, hi[k][j]);
+                  lo[k][j] = f2_add(lo[k][j], f2_add(f2_sub(hi[k][j], f2_sub(sum, z)), f2_sub(g[k][j], z)));
                   hi[k][j] = sum;
-                  g[k][j] = 0.f;
+                  g[k][j] = f2(0.f, 0.f);
                 }
               } else {
-                hi[k][j] = fmaf(x[k][r], hh[j], hi[k][j]);
+                hi[k][j] = f2_fma(xr, hh[j], hi[k][j]);
               }
             }
+          }
         }
         if (c0 < ncols) {
-          *(float4*)(rows[0] + c0) = make_float4(hi[0][0] + lo[0][0], hi[0][1] + lo[0][1], hi[0][2] + lo[0][2],
-                                                 hi[0][3] + lo[0][3]);
-          if (ok1)
-            *(float4*)(rows[1] + c0) = make_float4(hi[1][0] + lo[1][0], hi[1][1] + lo[1][1], hi[1][2] + lo[1][2],
-                                                   hi[1][3] + lo[1][3]);
+#pragma unroll
+          for (int k = 0; k < 2; k++) {
+            if (k && !ok1) break;
+            const float2 a0 = f2_split(f2_add(hi[k][0], lo[k][0])), a1 = f2_split(f2_add(hi[k][1], lo[k][1]));
+            *(float4*)(rows[k] + c0) = make_float4(a0.x, a0.y, a1.x, a1.y);
+          }
         }
       }
     }
@@ -1072,7 +1092,7 @@ cudaError_t cf_launch_full(const PatchDev* patches, const int4* work16, int nwor
   cf_full<<<nwork, kTilePx, 0, s>>>(patches, work16, a_up, a_diag, lvec, afull);
   return cudaGetLastError();
 }
-cudaError_t cf_launch_gram(const BlkArgs& a, int ntiles, const float* U, const float* V, double* out,
+cudaError_t cf_launch_gram(const BlkArgs& a, int npatch, int ntiles, const float* U, const float* V, double* out,
                            cudaStream_t s, double* out2) {
   constexpr int smem = 2 * GR_CH * kBlk * sizeof(float);  // 64 KB; the group sums (32 or 64 KB) reuse it
   static bool attr = false;
@@ -1082,9 +1102,11 @@ cudaError_t cf_launch_gram(const BlkArgs& a, int ntiles, const float* U, const f
     attr = true;
   }
   if (out2)
-    cf_gram<true><<<ntiles * kBlkSplit, 256, smem, s>>>(a, U, V, out, out2);
+    cf_gram<true><<<ntiles * kBlkSplit, 256, smem, s>>>(a, U, V);
   else
-    cf_gram<false><<<ntiles * kBlkSplit, 256, smem, s>>>(a, U, V, out, nullptr);
+    cf_gram<false><<<ntiles * kBlkSplit, 256, smem, s>>>(a, U, V);
+  const int ngram = out2 ? 2 : 1;
+  cf_gram_sum<<<dim3(npatch, ngram * kBlk * kBlk / kSumThreads), kSumThreads, 0, s>>>(a, ngram, out, out2);
   return cudaGetLastError();
 }
 cudaError_t cf_launch_rotate(const BlkArgs& a, int ntiles, float* U, float* V, int ncols, cudaStream_t s,

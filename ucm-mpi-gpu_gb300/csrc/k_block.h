@@ -68,7 +68,7 @@ cudaError_t cf_launch_step(const BlkArgs& a, const int4* work, int nwork, const 
                            int step, cudaStream_t s, bool comp = false, int variant = kStepDefault,
                            bool overlap = false);
 // out = U^T V per patch; with out2, out2 = U^T U in the same pass
-cudaError_t cf_launch_gram(const BlkArgs& a, int ntiles, const float* U, const float* V, double* out,
+cudaError_t cf_launch_gram(const BlkArgs& a, int npatch, int ntiles, const float* U, const float* V, double* out,
                            cudaStream_t s, double* out2 = nullptr);
 cudaError_t cf_launch_rotate(const BlkArgs& a, int ntiles, float* U, float* V, int ncols, cudaStream_t s,
                              bool comp = false);
