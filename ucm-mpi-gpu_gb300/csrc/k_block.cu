@@ -110,15 +110,16 @@ static_assert(DiskStencil::index(0, 0) == kStencilN / 2 && DiskStencil::index(kS
 static_assert(SquareStencil::index(kCR, kCR) == kCN - 1, "square numbering");
 static_assert(DiskStencil::NC == kFullNC && SquareStencil::NC == kCoarseNC, "row widths");
 
-// Shared memory of the step for WARPS consumer warps (2 WARPS tile rows):
+// Shared memory of the step for WARPS consumer warps of SBR tile rows each:
 // two stages of Y rows with their halo, and a ring of coefficient groups.
-template <class S, int WARPS>
+template <class S, int WARPS, int SBR>
 struct StepSmem {
-  static constexpr int PH = 2 * WARPS + 2 * S::R, PW = kStepTile + 2 * S::R;
+  static constexpr int ROWS = WARPS * SBR;
+  static constexpr int PH = ROWS + 2 * S::R, PW = kStepTile + 2 * S::R;
   static constexpr int NCH = S::NC / 4, GC = 3, NG = (NCH + GC - 1) / GC;  // chunks, chunks per group, groups
   static constexpr int RING = 4;
   static constexpr size_t y_bytes = (size_t)PH * PW * kBlk * sizeof(float);
-  static constexpr size_t chunk = (size_t)WARPS * 32 * 16;
+  static constexpr size_t chunk = (size_t)ROWS * kStepTile * 16;
   static constexpr size_t group = GC * chunk;
   static constexpr size_t bars = 2 * y_bytes + RING * group;  // tile records, mbarriers
   static constexpr size_t bytes = bars + 256;
@@ -190,7 +191,7 @@ struct StepRing {
   bool bad;              // a wait gave up: no further waits, the results are dropped
 };
 
-constexpr int SB_R = 2, SB_C = 4, SB_N = SB_R * SB_C;  // a quarter-warp's pixels
+constexpr int SB_C = 4;  // a quarter-warp's pixels: SBR rows of 4
 
 // one staged position (RY, DX) relative to the quarter's block origin: the
 // value of this lane's columns there, times the coefficient of every block
@@ -202,18 +203,18 @@ constexpr int SB_R = 2, SB_C = 4, SB_N = SB_R * SB_C;  // a quarter-warp's pixel
 // sum nearly cancel -- down to the groups' own four-term rounding, at about
 // a third of the cost of a TwoSum per term; used for the Rayleigh-Ritz
 // products and residuals, not the filter
-template <class S, int WARPS, bool C, int RY, int DX, int I>
-__device__ __forceinline__ void step_pixels(StepRing& ring, const unsigned char* (&gb)[StepSmem<S, WARPS>::NG],
-                                            const F2 (&v)[2], float4 (&cw)[SB_N], F2 (&acc)[SB_N][2],
-                                            F2 (&lo)[SB_N][2], F2 (&grp)[SB_N][2]) {
-  using SM = StepSmem<S, WARPS>;
-  if constexpr (I < SB_N) {
+template <class S, int WARPS, int SBR, bool C, int RY, int DX, int I>
+__device__ __forceinline__ void step_pixels(StepRing& ring, const unsigned char* (&gb)[StepSmem<S, WARPS, SBR>::NG],
+                                            const F2 (&v)[2], float4 (&cw)[SBR * SB_C], F2 (&acc)[SBR * SB_C][2],
+                                            F2 (&lo)[SBR * SB_C][2], F2 (&grp)[SBR * SB_C][2]) {
+  using SM = StepSmem<S, WARPS, SBR>;
+  if constexpr (I < SBR * SB_C) {
     constexpr int bi = I / SB_C, bj = I % SB_C;
     if constexpr (S::in(RY - bi, DX - bj)) {
       constexpr int idx = S::index(RY - bi, DX - bj), ch = idx / 4, g = ch / SM::GC;
       // a pixel meets its offsets in scanline order, so chunk idx / 4 is
       // first needed at idx % 4 == 0; pixel 0 is the first to get there
-      // (smallest row and column), pixel SB_N - 1 the last
+      // (smallest row and column), pixel SBR * SB_C - 1 the last
       if constexpr (idx % 4 == 0) {
         if constexpr (I == 0 && ch % SM::GC == 0) {
           const unsigned n = ring.n0 + g;
@@ -221,7 +222,7 @@ __device__ __forceinline__ void step_pixels(StepRing& ring, const unsigned char*
           gb[g] = ring.base + (n % SM::RING) * SM::group;
         }
         cw[I] = *(const float4*)(gb[g] + (ch % SM::GC) * SM::chunk + I * 64);
-        if constexpr (I == SB_N - 1 && (ch % SM::GC == SM::GC - 1 || ch == SM::NCH - 1)) {
+        if constexpr (I == SBR * SB_C - 1 && (ch % SM::GC == SM::GC - 1 || ch == SM::NCH - 1)) {
           __syncwarp();
           if ((threadIdx.x & 31) == 0) mbar_arrive(ring.empty + (ring.n0 + g) % SM::RING);
         }
@@ -244,44 +245,44 @@ __device__ __forceinline__ void step_pixels(StepRing& ring, const unsigned char*
         }
       }
     }
-    step_pixels<S, WARPS, C, RY, DX, I + 1>(ring, gb, v, cw, acc, lo, grp);
+    step_pixels<S, WARPS, SBR, C, RY, DX, I + 1>(ring, gb, v, cw, acc, lo, grp);
   }
 }
 
 // whether position P of the block's window feeds any of its pixels
-template <class S>
+template <class S, int SBR>
 __host__ __device__ constexpr bool step_used(int P) {
   const int NX = SB_C + 2 * S::R, RY = P / NX - S::R, DX = P % NX - S::R;
-  for (int i = 0; i < SB_R; i++)
+  for (int i = 0; i < SBR; i++)
     for (int j = 0; j < SB_C; j++)
       if (S::in(RY - i, DX - j)) return true;
   return false;
 }
-template <class S>
+template <class S, int SBR>
 __host__ __device__ constexpr int step_next(int P) {  // the first used position from P on
-  const int n = (SB_R + 2 * S::R) * (SB_C + 2 * S::R);
-  while (P < n && !step_used<S>(P)) P++;
+  const int n = (SBR + 2 * S::R) * (SB_C + 2 * S::R);
+  while (P < n && !step_used<S, SBR>(P)) P++;
   return P;
 }
-template <class S, int WARPS, int P>
+template <class S, int WARPS, int SBR, int P>
 __device__ __forceinline__ float4 step_value(const float* __restrict__ ys) {
   constexpr int NX = SB_C + 2 * S::R;
-  return *(const float4*)(ys + (P / NX * StepSmem<S, WARPS>::PW + P % NX) * kBlk);
+  return *(const float4*)(ys + (P / NX * StepSmem<S, WARPS, SBR>::PW + P % NX) * kBlk);
 }
 // positions P, ... in scanline order; v is P's value, loaded one position ahead
-template <class S, int WARPS, bool C, int P>
+template <class S, int WARPS, int SBR, bool C, int P>
 __device__ __forceinline__ void step_positions(const float* __restrict__ ys, float4 v4, StepRing& ring,
-                                               const unsigned char* (&gb)[StepSmem<S, WARPS>::NG],
-                                               float4 (&cw)[SB_N], F2 (&acc)[SB_N][2], F2 (&lo)[SB_N][2],
-                                               F2 (&grp)[SB_N][2]) {
-  constexpr int NY = SB_R + 2 * S::R, NX = SB_C + 2 * S::R;
+                                               const unsigned char* (&gb)[StepSmem<S, WARPS, SBR>::NG],
+                                               float4 (&cw)[SBR * SB_C], F2 (&acc)[SBR * SB_C][2], F2 (&lo)[SBR * SB_C][2],
+                                               F2 (&grp)[SBR * SB_C][2]) {
+  constexpr int NY = SBR + 2 * S::R, NX = SB_C + 2 * S::R;
   if constexpr (P < NY * NX) {
-    constexpr int RY = P / NX - S::R, DX = P % NX - S::R, PN = step_next<S>(P + 1);
+    constexpr int RY = P / NX - S::R, DX = P % NX - S::R, PN = step_next<S, SBR>(P + 1);
     float4 vn = v4;
-    if constexpr (PN < NY * NX) vn = step_value<S, WARPS, PN>(ys);
+    if constexpr (PN < NY * NX) vn = step_value<S, WARPS, SBR, PN>(ys);
     const F2 v[2] = {f2(v4.x, v4.y), f2(v4.z, v4.w)};
-    step_pixels<S, WARPS, C, RY, DX, 0>(ring, gb, v, cw, acc, lo, grp);
-    step_positions<S, WARPS, C, PN>(ys, vn, ring, gb, cw, acc, lo, grp);
+    step_pixels<S, WARPS, SBR, C, RY, DX, 0>(ring, gb, v, cw, acc, lo, grp);
+    step_positions<S, WARPS, SBR, C, PN>(ys, vn, ring, gb, cw, acc, lo, grp);
   }
 }
 
@@ -307,17 +308,18 @@ __device__ __forceinline__ void step_positions(const float* __restrict__ ys, flo
 // Measured, 16 patches of 266^2: 171 us per launch over all patches, 4.8 TB/s
 // of DRAM traffic, from 203 us with 8 x 16 tiles, half-warps and scalar FMAs
 // (187 us with scalar FMAs in this layout); same results to the bit.
-// WARPS = 8 (16 x 16 tiles) reads a third less halo than WARPS = 4 (8 x 16)
-// and has twice the warps to cover latency: 174 against 213 us there, 29
-// against 35 us at 600 tiles.  WARPS = 4 is for launches whose tiles do not
-// fill the SMs: 10 against 12 us at 20 tiles.
-template <class S, bool C, int WARPS>
+// SBR = 2 (16 x 16 tiles) reads a third less halo than SBR = 1 (8 x 16) and
+// loads each value for twice the pixels.  SBR = 1 is for launches whose tiles
+// do not fill the SMs: half the work in each warp's chain (10 against 12.5 us a
+// launch at 20 tiles, 202 against 175 us at 4624, 33 against 29 at 600).
+constexpr int kStepWarps = 8;
+template <class S, bool C, int WARPS, int SBR>
 __global__ void __launch_bounds__((WARPS + 2) * 32, 1) cf_step_t(BlkArgs a, const int4* __restrict__ work, int nwork,
                                                                  const float* __restrict__ Y,
                                                                  const float* __restrict__ X,
                                                                  float* __restrict__ out, int step) {
-  using SM = StepSmem<S, WARPS>;
-  constexpr int SUB = kStepTile / (2 * WARPS);  // launches' tiles per work entry
+  using SM = StepSmem<S, WARPS, SBR>;
+  constexpr int SB_N = SBR * SB_C, SUB = kStepTile / SM::ROWS;  // SUB: this kernel's tiles per work entry
   extern __shared__ __align__(128) unsigned char smem[];
   StepMeta* meta = (StepMeta*)(smem + SM::bars);  // [2]
   uint64_t* yfull = (uint64_t*)(smem + SM::bars + 128);
@@ -344,7 +346,7 @@ __global__ void __launch_bounds__((WARPS + 2) * 32, 1) cf_step_t(BlkArgs a, cons
     int i = 0;
     for (int t = blockIdx.x; t < nwork * SUB; t += gridDim.x) {
       const int4 w = work[t / SUB];
-      const int sub = t % SUB, y0 = w.y + sub * 2 * WARPS;
+      const int sub = t % SUB, y0 = w.y + sub * SM::ROWS;
       if (!a.active[w.x]) continue;
       const PatchDev P = a.patches[w.x];
       if (y0 >= P.H) continue;
@@ -366,7 +368,7 @@ __global__ void __launch_bounds__((WARPS + 2) * 32, 1) cf_step_t(BlkArgs a, cons
         m.cy = co.y;
         m.cz = co.z;
         // rows past the patch's last row (+ the radius) feed no in-patch pixel
-        const int ny = min(2 * WARPS, P.H - y0) + 2 * S::R;
+        const int ny = min(SM::ROWS, P.H - y0) + 2 * S::R;
         constexpr uint32_t yrow = SM::PW * kBlk * sizeof(float);
         unsigned char* ys = smem + st * SM::y_bytes;
         mbar_expect_tx(yfull + st, (uint32_t)ny * yrow);
@@ -374,7 +376,7 @@ __global__ void __launch_bounds__((WARPS + 2) * 32, 1) cf_step_t(BlkArgs a, cons
           bulk_g2s(ys + (size_t)r * yrow, Y + (P.vec + (long long)(y0 - S::R + r) * P.W + (w.z - S::R)) * kBlk, yrow,
                    yfull + st);
       } else {
-        const float4* src = (const float4*)a.afull + (long long)w.w * SM::NCH * kTilePx + sub * WARPS * 32;
+        const float4* src = (const float4*)a.afull + (long long)w.w * SM::NCH * kTilePx + sub * SM::ROWS * kStepTile;
         for (int g = 0; g < SM::NG; g++) {
           const int n = i * SM::NG + g, pl = n % SM::RING;
           if (n >= SM::RING && !mbar_wait(cempty + pl, (n / SM::RING - 1) & 1)) {
@@ -407,11 +409,12 @@ __global__ void __launch_bounds__((WARPS + 2) * 32, 1) cf_step_t(BlkArgs a, cons
     return;
   }
   // ------------------------------------------------------------ consumers
-  // warp: tile rows 2 warp, 2 warp + 1; quarter: columns 4 quarter .. + 3;
-  // lane: block columns col .. col + 3
-  const int quarter = lane >> 3, by = 2 * warp, bx = SB_C * quarter, col = 4 * (lane & 7);
+  // warp: tile rows SBR warp ..; quarter: columns 4 quarter .. + 3; lane:
+  // block columns col .. col + 3
+  const int quarter = lane >> 3, by = SBR * warp, bx = SB_C * quarter, col = 4 * (lane & 7);
   StepRing ring;
-  ring.base = smem + 2 * SM::y_bytes + (32 * warp + quarter) * 16;
+  // the slot of the quarter's first pixel, which is pixel 0 or 4 of its row pair
+  ring.base = smem + 2 * SM::y_bytes + (32 * (by >> 1) + 16 * (by & 1) + quarter) * 16;
   ring.full = cfull;
   ring.empty = cempty;
   ring.n0 = 0;
@@ -460,8 +463,8 @@ __global__ void __launch_bounds__((WARPS + 2) * 32, 1) cf_step_t(BlkArgs a, cons
     for (int k = 0; k < SB_N; k++)
 #pragma unroll
       for (int h = 0; h < 2; h++) acc[k][h] = lo[k][h] = grp[k][h] = f2(0.f, 0.f);
-    constexpr int P0 = step_next<S>(0);
-    step_positions<S, WARPS, C, P0>(ys, step_value<S, WARPS, P0>(ys), ring, gb, cw, acc, lo, grp);
+    constexpr int P0 = step_next<S, SBR>(0);
+    step_positions<S, WARPS, SBR, C, P0>(ys, step_value<S, WARPS, SBR, P0>(ys), ring, gb, cw, acc, lo, grp);
     if (ring.bad) {
       if (lane == 0) atomicExch(a.err, 1);
       return;
@@ -1042,28 +1045,32 @@ cudaError_t cf_launch_prolong(const CoarseArgs& c, int nwork_f, const float* xc,
   return cudaGetLastError();
 }
 
-template <class S, bool C, int WARPS>
+template <class S, bool C, int SBR>
 static cudaError_t step_attr() {
-  return cudaFuncSetAttribute(cf_step_t<S, C, WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)StepSmem<S, WARPS>::bytes);
+  return cudaFuncSetAttribute(cf_step_t<S, C, kStepWarps, SBR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)StepSmem<S, kStepWarps, SBR>::bytes);
 }
 template <class S>
 static void step_attrs() {
-  step_attr<S, false, 8>();
-  step_attr<S, true, 8>();
-  step_attr<S, false, 4>();
-  step_attr<S, true, 4>();
+  step_attr<S, false, 2>();
+  step_attr<S, true, 2>();
+  step_attr<S, false, 1>();
+  step_attr<S, true, 1>();
 }
 
+template <class S, bool C, int SBR>
+static cudaError_t step_go(const BlkArgs& a, const int4* work, int nwork, const float* Y, const float* X, float* out,
+                           int step, int nsm, bool overlap, cudaStream_t s) {
+  using SM = StepSmem<S, kStepWarps, SBR>;
+  // one persistent CTA per SM
+  return launch_overlap(cf_step_t<S, C, kStepWarps, SBR>, std::min(nwork * (kStepTile / SM::ROWS), nsm),
+                        (kStepWarps + 2) * 32, SM::bytes, s, overlap, a, work, nwork, Y, X, out, step);
+}
 template <class S, bool C>
 static cudaError_t step_go(const BlkArgs& a, const int4* work, int nwork, const float* Y, const float* X, float* out,
                            int step, int nsm, int variant, bool overlap, cudaStream_t s) {
-  // one persistent CTA per SM
-  if (variant == 0)
-    return launch_overlap(cf_step_t<S, C, 8>, std::min(nwork, nsm), 10 * 32, StepSmem<S, 8>::bytes, s, overlap, a, work,
-                          nwork, Y, X, out, step);
-  return launch_overlap(cf_step_t<S, C, 4>, std::min(2 * nwork, nsm), 6 * 32, StepSmem<S, 4>::bytes, s, overlap, a, work,
-                        nwork, Y, X, out, step);
+  return variant == 0 ? step_go<S, C, 2>(a, work, nwork, Y, X, out, step, nsm, overlap, s)
+                      : step_go<S, C, 1>(a, work, nwork, Y, X, out, step, nsm, overlap, s);
 }
 
 cudaError_t cf_launch_step(const BlkArgs& a, const int4* work, int nwork, const float* Y, const float* X, float* out,
