@@ -171,7 +171,7 @@ void mat_mul(const double* A, const double* B, double* C, int n, bool at) {
 // M = G^-1/2 (Loewdin; eigenvalues clamped at 1e-15 of the largest), so that
 // U M has orthonormal columns.  M(i, j) = sum_k Z(i, k) Z(j, k) / sqrt(w_k),
 // k ascending; M(j, i) has the same terms, so only j >= i is formed (half of
-// the divisions: 79 -> 68 us for n = 32).
+// the divisions: 76 -> 64 us for n = 32).
 void lowdin(const double* G, int n, double* M) {
   std::vector<double> A((size_t)n * n), w(n), Z((size_t)n * n), Zt((size_t)n * n), sq(n);
   for (int i = 0; i < n; i++)
