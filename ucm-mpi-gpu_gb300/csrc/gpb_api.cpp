@@ -827,7 +827,7 @@ static gpb_status solve_lanczos(gpb_ctx* ctx, const Layout& L) {
     long long active_px = 0;
     for (int i = 0; i < np; i++)
       if (active[i]) active_px += L.patches[i].N;
-    // one restart cycle: Lanczos steps k .. m-1, three launches each
+    // one restart cycle: Lanczos steps k .. m-1, three or five launches each
     auto cycle = [&]() -> cudaError_t {
       float* c = cur;
       float* nx = nxt;
@@ -849,7 +849,7 @@ static gpb_status solve_lanczos(gpb_ctx* ctx, const Layout& L) {
         prof_begin(ctx, 1, npx * 4.0 * (j + 1 + 2));
         if ((e = ks_launch_orth(a, nt, j, 2, nx, s)) != cudaSuccess) return e;
         prof_end(ctx);
-        ctx->launches += 3;
+        ctx->launches += nt > kEigSplitTiles ? 3 : 5;
         std::swap(c, nx);
       }
       return cudaSuccess;

@@ -6,12 +6,15 @@
 // damascene/src/stencilMatrixMultiply/stencilMVM.cu:129-182; the CPU path's
 // Spectra SymGEigsSolver (src/spectralPb.cpp:221-245) defines the problem.
 //
-// One Lanczos step for every active patch of the batch is three launches:
+// One Lanczos step for every active patch of the batch is three launches
 //   ks_spmv   w = A v_j (FP32 symmetric stencil SpMV, the lower triangle read
 //             as the upper array shifted by the offset), v_j = w_prev / beta
 //             written on the fly, h = V^T w
 //   ks_orth   w -= V h, h2 = V^T w          (classical Gram-Schmidt, pass 1)
 //   ks_orth   w -= V h2, beta^2 = |w|^2     (pass 2)
+// or, where the tiles of the batch leave SMs idle, five: ks_mult and
+// ks_project form the first two w with a pixel or two per thread, and ks_dots
+// takes the dots with the basis vectors dealt over several CTAs per tile.
 // Dot products are FMA chains over a thread's pixels, summed across the
 // warp and the CTA in float-float (a compensated FP32 pair; FP64 runs at
 // 1/64 of the FP32 rate on this part); the first CGS pass's projection V h,
@@ -23,6 +26,8 @@
 // cycle the host solves it (eig_host.cpp) and ks_restart assembles the kept
 // Ritz vectors.
 #include <stdint.h>
+
+#include <algorithm>
 
 #include "gpb_internal.h"
 #include "kernels.h"
@@ -99,12 +104,15 @@ __device__ __forceinline__ bool last_cta(int* counter, int ntiles) {
   return is_last;
 }
 
+// basis vectors loaded together
+constexpr int kGrp = 8;
 // per-warp partial sums (sred[warp][i], written by lane 0) -> one partial per
-// CTA in part[cta][i]
+// tile in part[tile][i], for the values i of the groups g, g + ng, ..
 constexpr int kRed = kMaxKrylov + 1;
-__device__ __forceinline__ void cta_partials(const float2* sred, int nvals, double* part_row) {
+__device__ __forceinline__ void cta_partials(const float2* sred, int nvals, double* part_row, int g = 0, int ng = 1) {
   __syncthreads();
   for (int i = threadIdx.x; i < nvals; i += blockDim.x) {
+    if (i / kGrp % ng != g) continue;
     float hi = 0.f, lo = 0.f;
 #pragma unroll
     for (int w = 0; w < kEigWarps; w++) ff_add(hi, lo, sred[w * kRed + i].x, sred[w * kRed + i].y);
@@ -162,7 +170,6 @@ __device__ __forceinline__ void patch_sums(const double* part, int tb, int tc, i
 // vector + patch) plus the pixel's 32-bit byte offset in its patch (at most
 // 2^28).  The stencil keeps 64-bit sums: with four uniform bases per offset it
 // took 39 us instead of 26.
-constexpr int kGrp = 8;
 __device__ __forceinline__ float ldu(const float* base, uint32_t off) {
   return *(const float*)((const char*)base + off);
 }
@@ -196,8 +203,8 @@ __device__ __forceinline__ float2 ff_warp_reduce8(float (&hi)[kGrp], float (&lo)
   return make_float2(hi[0], lo[0]);
 }
 
-// h_i = v_i . w for i = 0..j over this thread's pixels (w is 0 at a pixel
-// past the tile), reduced per warp into sred[warp][i]; v_j comes from
+// h_i = v_i . w for i = 0..j, of the groups g, g + ng, .. of 8, over this
+// thread's pixels (w is 0 at a pixel past the tile), reduced per warp into sred[warp][i]; v_j comes from
 // registers (xj) when given.  A plain FMA chain over the thread's eight
 // pixels, then float-float across threads: the error of a dot is a few
 // units of rounding times |w| (Cauchy-Schwarz over the thread partials),
@@ -205,8 +212,8 @@ __device__ __forceinline__ float2 ff_warp_reduce8(float (&hi)[kGrp], float (&lo)
 // two orders below what the Ritz residuals need.
 __device__ __forceinline__ void basis_dots(const EigArgs& a, int j, long long base, const uint32_t (&qv)[kEigPix],
                                            const float (&wv)[kEigPix], const float* xj, float2* sred, int warp,
-                                           int lane) {
-  for (int i0 = 0; i0 <= j; i0 += kGrp) {
+                                           int lane, int g = 0, int ng = 1) {
+  for (int i0 = g * kGrp; i0 <= j; i0 += ng * kGrp) {
     float vv[kGrp][kEigPix];
 #pragma unroll
     for (int u = 0; u < kGrp; u++) {
@@ -226,6 +233,46 @@ __device__ __forceinline__ void basis_dots(const EigArgs& a, int j, long long ba
     const int i = i0 + (lane >> 2);
     if ((lane & 3) == 0 && i <= j) sred[warp * kRed + i] = sum;
   }
+}
+
+// A patch's last CTA: its dots, into hbuf and T.  PASS 1 puts h; PASS 2 what
+// pass 1's subtraction missed (h2 = V^T (w - V h)), and T takes h + h2; T is
+// symmetric, and pass 1 wrote both of its entries.
+template <int PASS>
+__device__ __forceinline__ void put_dots(const EigArgs& a, int patch, int j, int warp, int lane) {
+  double* T = a.T + (long long)patch * a.m * a.m;
+  patch_sums(
+      a.part, a.tile_begin[patch], a.tile_count[patch], a.mp1, j + 1, warp, lane,
+      [&](int i) { return PASS == 2 ? T[i * a.m + j] : 0.0; },
+      [&](int i, double s, double was) {
+        a.hbuf[(long long)patch * a.mp1 + i] = s;
+        const double h = PASS == 2 ? was + s : s;
+        T[i * a.m + j] = h;
+        T[j * a.m + i] = h;
+      });
+}
+
+// ------------------------------------------------------------------ dots
+// The groups of 8 basis vectors of a tile dealt over gridDim.y CTAs (the bits
+// do not depend on how many).
+template <int PASS>
+__global__ void __launch_bounds__(kEigThreads, 2) ks_dots(EigArgs a, int j, const float* __restrict__ w) {
+  const EigTile t = a.tiles[blockIdx.x];
+  if (!a.active[t.patch]) return;
+  const long long base = uniform(a.patches[t.patch].vec);
+  uint32_t qv[kEigPix];
+  float wv[kEigPix];
+#pragma unroll
+  for (int r = 0; r < kEigPix; r++) {
+    const int p = t.p0 + threadIdx.x + r * kEigThreads;
+    qv[r] = 4u * (uint32_t)(p < t.p1 ? p : t.p0);
+    wv[r] = p < t.p1 ? ldu(w + base, qv[r]) : 0.f;
+  }
+  __shared__ float2 sred[kEigWarps * kRed];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  basis_dots(a, j, base, qv, wv, nullptr, sred, warp, lane, blockIdx.y, gridDim.y);
+  cta_partials(sred, j + 1, a.part + (long long)blockIdx.x * a.mp1, blockIdx.y, gridDim.y);
+  if (last_cta(a.counter + t.patch, a.tile_count[t.patch] * (int)gridDim.y)) put_dots<PASS>(a, t.patch, j, warp, lane);
 }
 
 // ------------------------------------------------------------------ SpMV
@@ -293,21 +340,56 @@ __global__ void __launch_bounds__(kEigThreads, 2) ks_spmv(EigArgs a, int j, cons
   // h_i = v_i . w for i <= j
   __shared__ float2 sred[kEigWarps * kRed];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // the second pass measures what these dots missed (h2 = V^T (w - V h)),
-  // and T takes h + h2
   basis_dots(a, j, base, qv, wv, xv, sred, warp, lane);
   cta_partials(sred, j + 1, a.part + (long long)blockIdx.x * a.mp1);
-  if (last_cta(a.counter + t.patch, a.tile_count[t.patch])) {
-    const int tb = a.tile_begin[t.patch], tc = a.tile_count[t.patch];
-    double* T = a.T + (long long)t.patch * a.m * a.m;
-    patch_sums(
-        a.part, tb, tc, a.mp1, j + 1, warp, lane, [](int) { return 0.0; },
-        [&](int i, double s, double) {
-          a.hbuf[(long long)t.patch * a.mp1 + i] = s;
-          T[i * a.m + j] = s;
-          T[j * a.m + i] = s;
-        });
+  if (last_cta(a.counter + t.patch, a.tile_count[t.patch])) put_dots<1>(a, t.patch, j, warp, lane);
+}
+
+// w = A v_j and v_j alone: 256 pixels of a tile per CTA, one per thread.  A
+// chain of load latencies on few tiles, so it is spread as wide as it goes:
+// on one 321 x 481 image ks_mult + ks_dots take 8.7 + 11.8 us and
+// ks_project + ks_dots 6.5 + 11.7 us, the whole step 52 us from 59.
+__global__ void __launch_bounds__(kEigThreads) ks_mult(EigArgs a, int j, const float* __restrict__ src,
+                                                       int use_beta, float* __restrict__ dst) {
+  const EigTile t = a.tiles[blockIdx.x / kEigPix];
+  if (!a.active[t.patch]) return;
+  const int p0 = t.p0 + (int)(blockIdx.x % kEigPix) * kEigThreads, p = p0 + threadIdx.x;
+  if (p0 >= t.p1) return;
+  const PatchDev P = a.patches[t.patch];
+  __shared__ int off[kUpper];
+  __shared__ float inv_s;
+  // the FP64 root and quotient run beside the stencil; read after it
+  if (threadIdx.x == kEigThreads - 1) inv_s = use_beta ? (float)(1.0 / sqrt(a.beta2[t.patch])) : 1.f;
+  if (threadIdx.x < kUpper) off[threadIdx.x] = c_up_dy[threadIdx.x] * P.W + c_up_dx[threadIdx.x];
+  __syncthreads();
+  if (p >= t.p1) return;
+  const long long q = P.vec + p;
+  const float* au = a.a_up + q;
+  const float* xs = src + q;
+  float acc = 0.f;
+  constexpr int NO = 8;  // offsets loaded together
+  static_assert(kUpper % NO == 0, "offset groups");
+#pragma unroll 1
+  for (int k0 = 0; k0 < kUpper; k0 += NO, au += NO * a.lvec) {
+    float cu[NO], xu[NO], cl[NO], xl[NO];
+#pragma unroll
+    for (int u = 0; u < NO; u++) {
+      const int o = off[k0 + u];
+      const float* al = au + u * a.lvec;
+      cu[u] = al[0];
+      xu[u] = xs[o];
+      cl[u] = al[-o];
+      xl[u] = xs[-o];
+    }
+#pragma unroll
+    for (int u = 0; u < NO; u++) {
+      acc = fmaf(cu[u], xu[u], acc);
+      acc = fmaf(cl[u], xl[u], acc);
+    }
   }
+  const float inv = inv_s, x = xs[0] * inv;
+  a.V[(long long)j * a.lvec + q] = x;
+  dst[q] = fmaf(acc, inv, a.a_diag[q] * x);
 }
 
 // --------------------------------------------------------------- CGS pass
@@ -403,20 +485,12 @@ __global__ void __launch_bounds__(kEigThreads, 2) ks_orth(EigArgs a, int j, floa
     cta_partials(sred, 1, a.part + (long long)blockIdx.x * a.mp1);
   }
   if (last_cta(a.counter + t.patch, a.tile_count[t.patch])) {
-    const int tb = a.tile_begin[t.patch], tc = a.tile_count[t.patch];
-    double* T = a.T + (long long)t.patch * a.m * a.m;
     if constexpr (MODE == 1) {
-      // T is symmetric, and pass 0 wrote both of its entries
-      patch_sums(
-          a.part, tb, tc, a.mp1, j + 1, warp, lane, [&](int i) { return T[i * a.m + j]; },
-          [&](int i, double s, double was) {
-            a.hbuf[(long long)t.patch * a.mp1 + i] = s;
-            T[i * a.m + j] = was + s;
-            T[j * a.m + i] = was + s;
-          });
+      put_dots<2>(a, t.patch, j, warp, lane);
     } else if (warp == 0) {
+      double* T = a.T + (long long)t.patch * a.m * a.m;
       patch_sums(
-          a.part, tb, tc, a.mp1, 1, warp, lane, [](int) { return 0.0; },
+          a.part, a.tile_begin[t.patch], a.tile_count[t.patch], a.mp1, 1, warp, lane, [](int) { return 0.0; },
           [&](int, double s, double) {
             if (!(s > 1e-60)) s = 1e-60;
             a.beta2[t.patch] = s;
@@ -427,6 +501,52 @@ __global__ void __launch_bounds__(kEigThreads, 2) ks_orth(EigArgs a, int j, floa
             }
           });
     }
+  }
+}
+
+// w -= V h alone, as ks_orth<1> does it: 512 pixels per CTA, two per thread
+constexpr int kProjPix = 2, kProjSplit = kEigPix / kProjPix;
+__global__ void __launch_bounds__(kEigThreads) ks_project(EigArgs a, int j, float* __restrict__ w) {
+  const EigTile t = a.tiles[blockIdx.x / kProjSplit];
+  if (!a.active[t.patch]) return;
+  const int p0 = t.p0 + (int)(blockIdx.x % kProjSplit) * kProjPix * kEigThreads;
+  if (p0 >= t.p1) return;
+  const PatchDev P = a.patches[t.patch];
+  const long long base = uniform(P.vec);
+  __shared__ float hs[kMaxKrylov + 1], hl[kMaxKrylov + 1];
+  for (int i = threadIdx.x; i <= j; i += blockDim.x) {
+    const double h = a.hbuf[(long long)t.patch * a.mp1 + i];
+    hs[i] = (float)h;
+    hl[i] = (float)(h - (double)hs[i]);
+  }
+  __syncthreads();
+  const int pa = p0 + threadIdx.x, pb = pa + kEigThreads;
+  const uint32_t qa = 4u * (uint32_t)(pa < t.p1 ? pa : t.p0), qb = 4u * (uint32_t)(pb < t.p1 ? pb : t.p0);
+  const float wv[2] = {ldu(w + base, qa), ldu(w + base, qb)};
+  F2 sh = f2(0.f, 0.f), sl = sh;
+  constexpr int NV = 16;  // basis vectors loaded together
+  for (int i0 = 0; i0 <= j; i0 += NV) {
+    F2 vv[NV];
+#pragma unroll
+    for (int u = 0; u < NV; u++) {
+      const float* Vi = a.V + (long long)(i0 + u) * a.lvec + base;
+      vv[u] = i0 + u <= j ? f2(ldu(Vi, qa), ldu(Vi, qb)) : f2(0.f, 0.f);
+    }
+#pragma unroll
+    for (int u = 0; u < NV; u++) {
+      if (i0 + u > j) break;
+      ff_add_prod2(sh, sl, f2(hs[i0 + u], hs[i0 + u]), vv[u]);
+      sl = f2_fma(f2(hl[i0 + u], hl[i0 + u]), vv[u], sl);
+    }
+  }
+  const float2 s2 = f2_split(sh), l2 = f2_split(sl);
+#pragma unroll
+  for (int r = 0; r < 2; r++) {
+    const float sr = r ? s2.y : s2.x, lr = r ? l2.y : l2.x;
+    const float d = wv[r] - sr;
+    const float z = d - wv[r];
+    const float e = (wv[r] - (d - z)) - (sr + z);
+    if ((r ? pb : pa) < t.p1) stu(w + base, r ? qb : qa, d + (e - lr));
   }
 }
 
@@ -555,16 +675,28 @@ cudaError_t ks_launch_init(const EigArgs& a, int ntiles, float* w, cudaStream_t 
   ks_init<<<ntiles, kEigThreads, 0, s>>>(a, w);
   return cudaGetLastError();
 }
+// CTAs per tile of the dots: two waves of the 304 that the 152 SMs hold
+static int dot_split(int ntiles, int j) { return std::min(j / kGrp + 1, std::max(1, 608 / ntiles)); }
+
 cudaError_t ks_launch_spmv(const EigArgs& a, int ntiles, int j, const float* src, int use_beta,
                            float* dst, cudaStream_t s) {
-  ks_spmv<<<ntiles, kEigThreads, 0, s>>>(a, j, src, use_beta, dst);
+  if (ntiles > kEigSplitTiles) {
+    ks_spmv<<<ntiles, kEigThreads, 0, s>>>(a, j, src, use_beta, dst);
+  } else {
+    ks_mult<<<ntiles * kEigPix, kEigThreads, 0, s>>>(a, j, src, use_beta, dst);
+    ks_dots<1><<<dim3(ntiles, dot_split(ntiles, j)), kEigThreads, 0, s>>>(a, j, dst);
+  }
   return cudaGetLastError();
 }
 cudaError_t ks_launch_orth(const EigArgs& a, int ntiles, int j, int mode, float* w, cudaStream_t s) {
-  if (mode == 1)
-    ks_orth<1><<<ntiles, kEigThreads, 0, s>>>(a, j, w);
-  else
+  if (mode == 2) {
     ks_orth<2><<<ntiles, kEigThreads, 0, s>>>(a, j, w);
+  } else if (ntiles > kEigSplitTiles) {
+    ks_orth<1><<<ntiles, kEigThreads, 0, s>>>(a, j, w);
+  } else {
+    ks_project<<<ntiles * kProjSplit, kEigThreads, 0, s>>>(a, j, w);
+    ks_dots<2><<<dim3(ntiles, dot_split(ntiles, j)), kEigThreads, 0, s>>>(a, j, w);
+  }
   return cudaGetLastError();
 }
 cudaError_t ks_launch_restart(const EigArgs& a, int ntiles, const float* w, float* vout, float* evec,

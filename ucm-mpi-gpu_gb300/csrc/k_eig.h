@@ -9,8 +9,8 @@ namespace gpb {
 
 constexpr int kEigThreads = 256;
 constexpr int kEigWarps = kEigThreads / 32;
-constexpr int kEigPix = 8;                          // pixels per thread
-constexpr int kEigTile = kEigThreads * kEigPix;     // pixels per CTA
+constexpr int kEigPix = 8;                          // pixels per thread in the reductions
+constexpr int kEigTile = kEigThreads * kEigPix;     // pixels per tile
 constexpr int kMaxKrylov = 64;
 
 struct EigTile {
@@ -41,8 +41,17 @@ struct EigArgs {
 
 void upload_eig(const HostTables& t, cudaStream_t s);
 cudaError_t ks_launch_init(const EigArgs& a, int ntiles, float* w, cudaStream_t s);
+// Batches of up to this many tiles take the five-launch step, which spreads a
+// tile's work over several CTAs.  Milliseconds of one solve, three launches
+// against five: 27.6 / 21.0 at 3 tiles, 124.1 / 96.4 at 22, 330.8 / 297.7 at
+// 76, 434.1 / 427.8 at 88, 421.7 / 428.1 at 102, 573.6 / 617.9 at 118 and
+// 739 / 782 at 560, where the extra reads of w and the launches cost more.
+constexpr int kEigSplitTiles = 96;
+
+// w = A v_j and h = V^T w
 cudaError_t ks_launch_spmv(const EigArgs& a, int ntiles, int j, const float* src, int use_beta,
                            float* dst, cudaStream_t s);
+// a Gram-Schmidt pass: mode 1 w -= V h, h2 = V^T w; mode 2 w -= V h2, |w|^2
 cudaError_t ks_launch_orth(const EigArgs& a, int ntiles, int j, int mode, float* w, cudaStream_t s);
 // the restart of the patches whose decision is 1 and the final Ritz vectors
 // of those whose decision is 2 (each launched only when some patch needs it)
