@@ -56,3 +56,27 @@ def test_stitch_many_overlapping_patches(mode):
         assert np.abs(got - want).max() < 1e-5  # FP32 sums of up to 40 weighted values in [0, 1]
     else:
         assert np.array_equal(got, want.astype(np.float32))
+
+
+@pytest.mark.parametrize("n,H,W", [(1, 2 ** 21 + 40, 1), (128, 70, 90), (129, 70, 90)])
+def test_stitch_box_counts_and_tall_image(n, H, W):
+    """Around the 128 boxes that travel in the launch, and an image of more
+    rows of tiles than a grid's second dimension holds: copies, so exact."""
+    torch = pytest.importorskip("torch")
+    import gpb
+    from gpb import synth
+    img = synth.voronoi_image(64, 64, 12, 8.0, synth.SEED_BASE + 193)
+    cb = synth.make_codebook(img, synth.SEED_BASE + 193, k=4, n_sample=512)
+    packed = synth.pack_bgr(img)
+    ctx = gpb.Context(cb, eig_mode=gpb.EIG_WARM)
+    outs = ctx.compute_batch([np.ascontiguousarray(packed[i % 30:i % 30 + 32, i % 29:i % 29 + 32]) for i in range(n)])
+    places = [(7 * i % W, H - 35 - 11 * i % (H - 34), 0, 0, 32, 32) for i in range(n)]
+    d_nm = torch.full((H, W), -7.0, device="cuda")
+    d_or = torch.full((8, H, W), -7.0, device="cuda")
+    ctx.stitch_device(gpb.STITCH_LAST, W, H, places, d_nm.data_ptr(), d_or.data_ptr())
+    ctx.close()
+    want = np.full((9, H, W), -7.0, np.float32)
+    for (nm, orr), (x0, y0, *_) in zip(outs, places):
+        v = np.concatenate([nm.reshape(1, 32, 32), orr.reshape(8, 32, 32)])
+        want[:, y0:y0 + 32, x0:x0 + 32] = v[:, :min(32, H - y0), :min(32, W - x0)]
+    assert np.array_equal(d_nm.cpu().numpy(), want[0]) and np.array_equal(d_or.cpu().numpy(), want[1:])

@@ -1781,10 +1781,13 @@ extern "C" gpb_status gpb_stitch_device(gpb_ctx* ctx, int mode, uint32_t width, 
       else
         boxes[i] = {q.x0, q.y0, 0, 0, P.W, P.H};
     }
-    CK(grow(b.stitch, b.c_stitch, n));
-    CK(cudaMemcpyAsync(b.stitch, boxes.data(), n * sizeof(StitchBox), cudaMemcpyHostToDevice, s));
-    CK(launch_stitch(b.patches, b.stitch, (int)n, mode == GPB_STITCH_BLEND, b.nmax, b.orient, colmajor, (int)width,
-                     (int)height, rmp, d_nmax, d_orient, s));
+    const bool few = n <= (size_t)kStitchFew;
+    if (!few) {
+      CK(grow(b.stitch, b.c_stitch, n));
+      CK(cudaMemcpyAsync(b.stitch, boxes.data(), n * sizeof(StitchBox), cudaMemcpyHostToDevice, s));
+    }
+    CK(launch_stitch(b.patches, boxes.data(), few ? nullptr : b.stitch, (int)n, mode == GPB_STITCH_BLEND,
+                     b.nmax, b.orient, colmajor, (int)width, (int)height, rmp, d_nmax, d_orient, s));
     CK(cudaStreamSynchronize(s));
     return GPB_OK;
   });

@@ -27,6 +27,11 @@ namespace gpb {
 
 namespace {
 
+// boxes passed in the launch itself: no buffer, no copy
+struct StitchFew {
+  StitchBox b[kStitchFew];
+};
+
 constexpr int ST_T = 32, ST_ROWS = 4;  // tile side; rows per thread, 8 apart
 
 __device__ __forceinline__ float patch_orient(const float* orient, const PatchDev& P, int colmajor, int o, int y,
@@ -49,13 +54,15 @@ __device__ __forceinline__ float stitch_weight(const StitchBox& b, const PatchDe
 
 template <bool BLEND>
 __global__ void __launch_bounds__(256) k_stitch(const PatchDev* __restrict__ patches,
-                                                const StitchBox* __restrict__ boxes, int n,
+                                                const __grid_constant__ StitchFew few,
+                                                const StitchBox* __restrict__ many, int n, unsigned cols,
                                                 const float* __restrict__ nmax, const float* __restrict__ orient,
                                                 int colmajor, int img_w, int img_h, float ramp,
                                                 float* __restrict__ out_nmax, float* __restrict__ out_orient) {
   __shared__ int list[256], warp_n[8];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int tx0 = blockIdx.x * ST_T, ty0 = blockIdx.y * ST_T;
+  const StitchBox* boxes = many ? many : few.b;
+  const int tx0 = (int)(blockIdx.x % cols) * ST_T, ty0 = (int)(blockIdx.x / cols) * ST_T;
   const int gx = tx0 + lane;
   const long long plane = (long long)img_w * img_h;
   int win[ST_ROWS];           // the last covering patch
@@ -135,18 +142,21 @@ __global__ void __launch_bounds__(256) k_stitch(const PatchDev* __restrict__ pat
 
 }  // namespace
 
-cudaError_t launch_stitch(const PatchDev* patches, const StitchBox* boxes, int n, bool blend, const float* nmax,
-                          const float* orient, int colmajor, int img_w, int img_h, float ramp, float* out_nmax,
-                          float* out_orient, cudaStream_t s) {
-  const unsigned rows = (unsigned)((img_h + (long long)ST_T - 1) / ST_T);
-  if (rows > 65535u) return cudaErrorInvalidValue;  // over 2 million image rows
-  const dim3 grid((unsigned)((img_w + (long long)ST_T - 1) / ST_T), rows);
+cudaError_t launch_stitch(const PatchDev* patches, const StitchBox* host_boxes, const StitchBox* boxes, int n,
+                          bool blend, const float* nmax, const float* orient, int colmajor, int img_w, int img_h,
+                          float ramp, float* out_nmax, float* out_orient, cudaStream_t s) {
+  StitchFew few = {};
+  if (!boxes)
+    for (int i = 0; i < n; i++) few.b[i] = host_boxes[i];
+  const unsigned cols = (unsigned)((img_w + (long long)ST_T - 1) / ST_T);
+  const long long tiles = cols * ((img_h + (long long)ST_T - 1) / ST_T);
+  if (tiles > 0x7fffffffLL) return cudaErrorInvalidValue;  // planes of 2^41 pixels
   if (blend)
-    k_stitch<true><<<grid, 256, 0, s>>>(patches, boxes, n, nmax, orient, colmajor, img_w, img_h, ramp, out_nmax,
-                                        out_orient);
+    k_stitch<true><<<(unsigned)tiles, 256, 0, s>>>(patches, few, boxes, n, cols, nmax, orient, colmajor, img_w, img_h,
+                                                   ramp, out_nmax, out_orient);
   else
-    k_stitch<false><<<grid, 256, 0, s>>>(patches, boxes, n, nmax, orient, colmajor, img_w, img_h, ramp, out_nmax,
-                                         out_orient);
+    k_stitch<false><<<(unsigned)tiles, 256, 0, s>>>(patches, few, boxes, n, cols, nmax, orient, colmajor, img_w, img_h,
+                                                    ramp, out_nmax, out_orient);
   return cudaGetLastError();
 }
 

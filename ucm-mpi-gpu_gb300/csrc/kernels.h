@@ -61,11 +61,14 @@ cudaError_t launch_spb(const PatchDev* patches, const int4* work, int nwork, con
 struct StitchBox {
   int ox, oy, x, y, w, h;
 };
-// whole-image planes from n patches' boxes (device arrays, patch order): the
-// last covering box's values, or (blend) their weighted mean
-cudaError_t launch_stitch(const PatchDev* patches, const StitchBox* boxes, int n, bool blend, const float* nmax,
-                          const float* orient, int colmajor, int img_w, int img_h, float ramp, float* out_nmax,
-                          float* out_orient, cudaStream_t s);
+// whole-image planes from n patches' boxes (patch order): the last covering
+// box's values, or (blend) their weighted mean.  Up to kStitchFew boxes travel
+// in the launch's parameters (3 of the 4 KB that those may take), from
+// host_boxes; more are read from the device array boxes.
+constexpr int kStitchFew = 128;
+cudaError_t launch_stitch(const PatchDev* patches, const StitchBox* host_boxes, const StitchBox* boxes, int n,
+                          bool blend, const float* nmax, const float* orient, int colmajor, int img_w, int img_h,
+                          float ramp, float* out_nmax, float* out_orient, cudaStream_t s);
 
 // k_spfeat.cu
 cudaError_t launch_sp_features(const PatchDev* patches, int pi, long long npix, const int32_t* labels, int n,
