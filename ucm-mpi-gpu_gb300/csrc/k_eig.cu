@@ -556,16 +556,13 @@ __global__ void __launch_bounds__(kEigThreads) ks_project(EigArgs a, int j, floa
 // (FINAL), the nk = nvec Ritz vectors into evec_out.  A CTA per 256 pixels: a
 // restart is one launch between host round trips, so it is spread as wide as
 // it goes.
-// Restart: FMA chains over the m basis vectors; the kept vectors come out
-// orthonormal to a few units of rounding, which the next cycle's two CGS
-// passes keep.  A thread takes one pixel and up to 32 outputs per pass over
-// V, so each basis value is loaded once per pass and each 16-byte broadcast
-// of Y (shared memory, zero-padded) feeds 4 FMAs; 80 registers keep three
-// CTAs on an SM.
-// FINAL: the eigenvectors themselves, where an FMA chain's rounding (about
-// sqrt(m) units) would show in their residual: Y is split into FP32 hi + lo,
-// the hi products are summed by FMA in groups of four folded into a
-// float-float by TwoSum, the lo products into the low word.
+// Y is split into FP32 hi + lo; the hi products are summed by FMA in groups of
+// four folded into a float-float by TwoSum, the lo products into the low word:
+// an FMA chain's rounding (about sqrt(m) units) would show in the residuals
+// and, at a restart, in the relation that their estimate relies on.  A thread
+// takes one pixel and 16 outputs per pass over V, so each basis value is loaded
+// once per pass and each 16-byte broadcast of Y (shared memory, zero-padded)
+// feeds 4 FMAs.
 template <bool FINAL>
 __global__ void __launch_bounds__(kEigThreads, 2) ks_restart(EigArgs a, const float* __restrict__ w,
                                                             float* __restrict__ vout,
