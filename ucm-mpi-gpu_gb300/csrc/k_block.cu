@@ -30,6 +30,7 @@
 #include "k_block.h"
 #include "k_eig.h"
 #include "overlap.h"
+#include "per_device.h"
 
 namespace gpb {
 
@@ -1046,22 +1047,12 @@ cudaError_t cf_launch_prolong(const CoarseArgs& c, int nwork_f, const float* xc,
 }
 
 template <class S, bool C, int SBR>
-static cudaError_t step_attr() {
-  return cudaFuncSetAttribute(cf_step_t<S, C, kStepWarps, SBR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)StepSmem<S, kStepWarps, SBR>::bytes);
-}
-template <class S>
-static void step_attrs() {
-  step_attr<S, false, 2>();
-  step_attr<S, true, 2>();
-  step_attr<S, false, 1>();
-  step_attr<S, true, 1>();
-}
-
-template <class S, bool C, int SBR>
 static cudaError_t step_go(const BlkArgs& a, const int4* work, int nwork, const float* Y, const float* X, float* out,
                            int step, int nsm, bool overlap, cudaStream_t s) {
   using SM = StepSmem<S, kStepWarps, SBR>;
+  static PerDevice ready;
+  const cudaError_t e = ready.once([] { return grant_smem(cf_step_t<S, C, kStepWarps, SBR>, SM::bytes); });
+  if (e != cudaSuccess) return e;
   // one persistent CTA per SM
   return launch_overlap(cf_step_t<S, C, kStepWarps, SBR>, std::min(nwork * (kStepTile / SM::ROWS), nsm),
                         (kStepWarps + 2) * 32, SM::bytes, s, overlap, a, work, nwork, Y, X, out, step);
@@ -1075,17 +1066,11 @@ static cudaError_t step_go(const BlkArgs& a, const int4* work, int nwork, const 
 
 cudaError_t cf_launch_step(const BlkArgs& a, const int4* work, int nwork, const float* Y, const float* X, float* out,
                            int step, cudaStream_t s, bool comp, int variant, bool overlap) {
-  static int nsm = 0;
-  if (!nsm) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    step_attrs<DiskStencil>();
-    step_attrs<SquareStencil>();
-    if (nsm <= 0) nsm = 1;
-  }
   if (nwork <= 0) return cudaSuccess;
-  cudaError_t e;
+  int dev = 0, nsm = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  if (e != cudaSuccess) return e;
   if (a.coarse)
     e = comp ? step_go<SquareStencil, true>(a, work, nwork, Y, X, out, step, nsm, variant, overlap, s)
              : step_go<SquareStencil, false>(a, work, nwork, Y, X, out, step, nsm, variant, overlap, s);
@@ -1102,12 +1087,12 @@ cudaError_t cf_launch_full(const PatchDev* patches, const int4* work16, int nwor
 cudaError_t cf_launch_gram(const BlkArgs& a, int npatch, int ntiles, const float* U, const float* V, double* out,
                            cudaStream_t s, double* out2) {
   constexpr int smem = 2 * GR_CH * kBlk * sizeof(float);  // 64 KB; the group sums (32 or 64 KB) reuse it
-  static bool attr = false;
-  if (!attr) {
-    cudaFuncSetAttribute(cf_gram<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    cudaFuncSetAttribute(cf_gram<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    attr = true;
-  }
+  static PerDevice ready;
+  const cudaError_t e = ready.once([] {
+    const cudaError_t f = grant_smem(cf_gram<false>, smem);
+    return f != cudaSuccess ? f : grant_smem(cf_gram<true>, smem);
+  });
+  if (e != cudaSuccess) return e;
   if (out2)
     cf_gram<true><<<ntiles * kBlkSplit, 256, smem, s>>>(a, U, V);
   else
@@ -1118,12 +1103,12 @@ cudaError_t cf_launch_gram(const BlkArgs& a, int npatch, int ntiles, const float
 }
 cudaError_t cf_launch_rotate(const BlkArgs& a, int ntiles, float* U, float* V, int ncols, cudaStream_t s,
                              bool comp) {
-  static bool attr = false;
-  if (!attr) {
-    cudaFuncSetAttribute(cf_rotate<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRotSmem);
-    cudaFuncSetAttribute(cf_rotate<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRotSmem);
-    attr = true;
-  }
+  static PerDevice ready;
+  const cudaError_t e = ready.once([] {
+    const cudaError_t f = grant_smem(cf_rotate<false>, kRotSmem);
+    return f != cudaSuccess ? f : grant_smem(cf_rotate<true>, kRotSmem);
+  });
+  if (e != cudaSuccess) return e;
   if (comp)
     cf_rotate<true><<<ntiles * kBlkSplit, 256, kRotSmem, s>>>(a, U, V, ncols);
   else

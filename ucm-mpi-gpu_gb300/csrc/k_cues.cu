@@ -31,6 +31,7 @@
 
 #include "gpb_internal.h"
 #include "kernels.h"
+#include "per_device.h"
 
 namespace gpb {
 
@@ -506,13 +507,12 @@ cudaError_t launch_maxlabel(const PatchDev* patches, int npatch, const uint32_t*
 
 cudaError_t launch_cues(const PatchDev* patches, const int4* work, int nwork, const uint32_t* lab4,
                         const int* nbins, float* mpbo, float* go, float* raw, uint8_t* counts, cudaStream_t s) {
-  static bool attr = false;
-  if (!attr) {
-    cudaFuncSetAttribute(k_cues<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCueSmem);
-    cudaFuncSetAttribute(k_cues<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCueSmem);
-    attr = true;
-  }
-  if (nwork == 0) return cudaSuccess;
+  static PerDevice ready;
+  const cudaError_t e = ready.once([] {
+    const cudaError_t f = grant_smem(k_cues<false>, kCueSmem);
+    return f != cudaSuccess ? f : grant_smem(k_cues<true>, kCueSmem);
+  });
+  if (e != cudaSuccess || nwork == 0) return e;
   if (raw)
     k_cues<true><<<nwork, CT_WARPS * 32, kCueSmem, s>>>(patches, work, lab4, nbins, mpbo, go, raw, counts);
   else

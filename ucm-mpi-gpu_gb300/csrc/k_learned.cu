@@ -30,6 +30,7 @@
 
 #include "k_block.h"
 #include "k_learned.h"
+#include "per_device.h"
 
 namespace gpb {
 
@@ -771,12 +772,9 @@ template <int CIN, int CO, int MODE, int C1>
 cudaError_t conv_go(const LnPatch* lp, const LnTile* tiles, int ntiles, int cout, const LnIn& in, const float* dA,
                     const bf16* mask, const bf16* w, const float* bias, void* out, cudaStream_t s) {
   constexpr size_t smem = ((size_t)NHALO * (CIN + 8) + (size_t)CO * (9 * CIN + 8)) * sizeof(bf16);
-  static bool attr = false;
-  if (!attr) {
-    cudaFuncSetAttribute(k_ln_conv<CIN, CO, MODE, C1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    attr = true;
-  }
-  if (ntiles == 0) return cudaSuccess;
+  static PerDevice ready;
+  const cudaError_t e = ready.once([] { return grant_smem(k_ln_conv<CIN, CO, MODE, C1>, smem); });
+  if (e != cudaSuccess || ntiles == 0) return e;
   // Up to 16 input channels a tile per CTA: the weights are under 10 KB, and
   // 12-16 CTAs per SM overlap one another's staging (62 us for the three of
   // a forward of 617 kpx against 67 us persistent).  Wider layers: as many
@@ -827,11 +825,9 @@ template <int CIN, int CC, int COUT, int WC, int C1>
 cudaError_t wgrad_go(const LnPatch* lp, const LnTile* tiles, int ntiles, const float* dA, const bf16* mask,
                      const LnIn& X, float* dW, float* db, cudaStream_t s) {
   using G = WgradCfg<CIN, CC, COUT, WC>;
-  static bool attr = false;
-  if (!attr) {
-    cudaFuncSetAttribute(k_ln_wgrad<CIN, CC, COUT, WC, C1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G::smem);
-    attr = true;
-  }
+  static PerDevice ready;
+  const cudaError_t e = ready.once([] { return grant_smem(k_ln_wgrad<CIN, CC, COUT, WC, C1>, G::smem); });
+  if (e != cudaSuccess) return e;
   // about two CTAs per SM over the channel chunks; one where a thread's sums
   // take most of its registers
   constexpr int chunks = CIN / CC, per_sm = G::CPW * G::NT >= 4 ? 1 : 2;
