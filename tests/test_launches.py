@@ -27,3 +27,7 @@ def _run(tmp_path, name, *args):
 @pytest.mark.parametrize("args", [(), ("grants-fail-first",)])
 def test_shared_memory_grants_per_device_and_thread(tmp_path, args):
     _run(tmp_path, "devices_check", *args)
+
+
+def test_stitch_launches_in_proportion_to_its_boxes(tmp_path):
+    _run(tmp_path, "stitch_check")

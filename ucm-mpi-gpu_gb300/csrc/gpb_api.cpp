@@ -134,7 +134,7 @@ struct Buf {
   float* cblk[4] = {nullptr, nullptr, nullptr, nullptr}; size_t c_cblk[4] = {0, 0, 0, 0};
   float* afull = nullptr; size_t c_afull = 0;  // fine stencil rows in the block step's tile layout
   int4* work_act = nullptr; size_t c_wact = 0;  // 16 x 16 tiles of the still active patches
-  StitchBox* stitch = nullptr; size_t c_stitch = 0;  // the boxes of a stitch
+  StitchSpan* stitch = nullptr; size_t c_stitch = 0;  // the boxes of a stitch
   unsigned long long* spsum = nullptr; size_t c_spsum = 0;  // superpixel colour sums, then histograms
   int* berr = nullptr; size_t c_berr = 0;
 };
@@ -1782,10 +1782,7 @@ extern "C" gpb_status gpb_stitch_device(gpb_ctx* ctx, int mode, uint32_t width, 
         boxes[i] = {q.x0, q.y0, 0, 0, P.W, P.H};
     }
     const bool few = n <= (size_t)kStitchFew;
-    if (!few) {
-      CK(grow(b.stitch, b.c_stitch, n));
-      CK(cudaMemcpyAsync(b.stitch, boxes.data(), n * sizeof(StitchBox), cudaMemcpyHostToDevice, s));
-    }
+    if (!few) CK(grow(b.stitch, b.c_stitch, n));
     CK(launch_stitch(b.patches, boxes.data(), few ? nullptr : b.stitch, (int)n, mode == GPB_STITCH_BLEND,
                      b.nmax, b.orient, colmajor, (int)width, (int)height, rmp, d_nmax, d_orient, s));
     CK(cudaStreamSynchronize(s));

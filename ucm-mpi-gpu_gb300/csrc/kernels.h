@@ -61,14 +61,20 @@ cudaError_t launch_spb(const PatchDev* patches, const int4* work, int nwork, con
 struct StitchBox {
   int ox, oy, x, y, w, h;
 };
+// the same as the kernel reads it: the image pixels [x0, x1) x [y0, y1) that
+// the box covers, and the number of the first CTA of its own tiles
+struct StitchSpan {
+  int ox, oy;
+  unsigned x0, y0, x1, y1, first;
+};
 // whole-image planes from n patches' boxes (patch order): the last covering
 // box's values, or (blend) their weighted mean.  Up to kStitchFew boxes travel
-// in the launch's parameters (3 of the 4 KB that those may take), from
-// host_boxes; more are read from the device array boxes.
+// in the launch's parameters (3.5 of the 4 KB that those may take); for more,
+// dev_spans is a device array of n entries, else null.
 constexpr int kStitchFew = 128;
-cudaError_t launch_stitch(const PatchDev* patches, const StitchBox* host_boxes, const StitchBox* boxes, int n,
-                          bool blend, const float* nmax, const float* orient, int colmajor, int img_w, int img_h,
-                          float ramp, float* out_nmax, float* out_orient, cudaStream_t s);
+cudaError_t launch_stitch(const PatchDev* patches, const StitchBox* boxes, StitchSpan* dev_spans, int n, bool blend,
+                          const float* nmax, const float* orient, int colmajor, int img_w, int img_h, float ramp,
+                          float* out_nmax, float* out_orient, cudaStream_t s);
 
 // k_spfeat.cu
 cudaError_t launch_sp_features(const PatchDev* patches, int pi, long long npix, const int32_t* labels, int n,
