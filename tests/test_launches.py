@@ -31,3 +31,7 @@ def test_shared_memory_grants_per_device_and_thread(tmp_path, args):
 
 def test_stitch_launches_in_proportion_to_its_boxes(tmp_path):
     _run(tmp_path, "stitch_check")
+
+
+def test_ucm_launches_in_proportion_to_each_image(tmp_path):
+    _run(tmp_path, "ucm_check")

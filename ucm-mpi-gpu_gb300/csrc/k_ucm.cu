@@ -23,10 +23,12 @@
 //   k_ucm_finish   region labels of the pixels and the padded strength grid
 //                  ws_wt2 (contours2ucm.cpp:439-458)
 //
-// Every launch covers all images of a batch, one per blockIdx.y: grid-stride
-// over the image, except the flooding (one CTA per image) and the artefact
-// fixes (one thread per image).
+// Every launch covers all images of a batch, each with CTAs in proportion to
+// its size (UcmPart), except the flooding, the small scans (one CTA per image)
+// and the artefact fixes (one thread per image).
 #include <stdint.h>
+
+#include <algorithm>
 
 #include "ucm_dev.h"
 
@@ -44,17 +46,45 @@ __device__ __forceinline__ float ord2f(unsigned u) {
 
 }  // namespace
 
+// the images of a launch and the kind of its CTAs
+struct UcmLaunch {
+  const UcmView* __restrict__ views;
+  int n;
+  UcmKind kind;
+};
+// this CTA's image, its number among the image's CTAs and how many those are
+struct UcmPart {
+  const UcmView& V;
+  int cta, ctas;
+};
+// MUL: CTAs per counted one.  Whole warps, before any thread has left: a search
+// by 32 places at a time, one load up to 32 images.
+template <int MUL = 1>
+__device__ __forceinline__ UcmPart ucm_part(const UcmLaunch& l) {
+  const int b = (int)(blockIdx.x / MUL), lane = threadIdx.x & 31;
+  int lo = 0, hi = l.n;  // first of lo <= b < first of hi
+  while (hi - lo > 1) {
+    const int step = (hi - lo + 31) / 32, i = lo + lane * step;
+    const unsigned m = __ballot_sync(0xffffffffu, i < hi && l.views[i].first[l.kind] <= b);
+    lo += (__popc(m) - 1) * step;
+    hi = min(hi, lo + step);
+  }
+  const int f = l.views[lo].first[l.kind] * MUL;
+  return {l.views[lo], (int)blockIdx.x - f, l.views[lo + 1].first[l.kind] * MUL - f};
+}
+
 // ---------------------------------------------------------------- pb, u8
 
-__global__ void __launch_bounds__(256) k_ucm_pbmax(const UcmView* __restrict__ views) {
-  const UcmView& V = views[blockIdx.y];
+__global__ void __launch_bounds__(256) k_ucm_pbmax(UcmLaunch l) {
+  const UcmPart me = ucm_part(l);
+  const UcmView& V = me.V;
   const float* __restrict__ orient = V.orient;
   const long long N = (long long)V.H * V.W;
   float* __restrict__ pb = V.s.pb;
   unsigned* mm = V.s.mm;
-  if ((long long)blockIdx.x * blockDim.x >= N) return;
+  if ((long long)me.cta * blockDim.x >= N) return;
   unsigned lo = 0xffffffffu, hi = 0u;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < N; i += (long long)gridDim.x * blockDim.x) {
+  for (long long i = (long long)me.cta * blockDim.x + threadIdx.x; i < N; i += (long long)me.ctas * blockDim.x) {
     float m = orient[i];
     for (int o = 1; o < 8; o++) {
       const float v = orient[(long long)o * N + i];
@@ -74,15 +104,16 @@ __global__ void __launch_bounds__(256) k_ucm_pbmax(const UcmView* __restrict__ v
   }
 }
 
-__global__ void __launch_bounds__(256) k_ucm_quant(const UcmView* __restrict__ views) {
-  const UcmView& V = views[blockIdx.y];
+__global__ void __launch_bounds__(256) k_ucm_quant(UcmLaunch l) {
+  const UcmPart me = ucm_part(l);
+  const UcmView& V = me.V;
   const float* __restrict__ pb = V.s.pb;
   uint8_t* __restrict__ q = V.s.q;
   const long long N = (long long)V.H * V.W;
   const unsigned* mm = V.s.mm;
   const double lo = (double)ord2f(~mm[0]), hi = (double)ord2f(mm[1]);
   const double alpha = 255.0 / (hi - lo), beta = __ddiv_rn(-255.0 * lo, hi - lo);
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < N; i += (long long)gridDim.x * blockDim.x) {
+  for (long long i = (long long)me.cta * blockDim.x + threadIdx.x; i < N; i += (long long)me.ctas * blockDim.x) {
     const double v = __dadd_rn(__dmul_rn((double)pb[i], alpha), beta);
     uint8_t r = 0;
     if (v == v) {  // NaN (a constant image) saturates to 0
@@ -98,14 +129,15 @@ __global__ void __launch_bounds__(256) k_ucm_quant(const UcmView* __restrict__ v
 // One warp per row: a stable counting sort of the row's columns by level.
 // off[row * 257 + l] is the first position of level l; cols[row * W + k]
 // the k-th column in (level, column) order.
-__global__ void __launch_bounds__(32) k_ws_rowsort(const UcmView* __restrict__ views) {
-  const UcmView& V = views[blockIdx.y];
+__global__ void __launch_bounds__(32) k_ws_rowsort(UcmLaunch l) {
+  const UcmPart me = ucm_part(l);
+  const UcmView& V = me.V;
   const uint8_t* __restrict__ q = V.s.q;
   const int H = V.H, W = V.W;
   int32_t* __restrict__ off = V.s.off;
   uint16_t* __restrict__ cols = V.s.cols;
   __shared__ int cnt[256];
-  const int row = blockIdx.x, lane = threadIdx.x;
+  const int row = me.cta, lane = threadIdx.x;
   if (row >= H) return;
   for (int v = lane; v < 256; v += 32) cnt[v] = 0;
   __syncwarp();
@@ -255,12 +287,13 @@ __global__ void __launch_bounds__(1024) k_ws_flood(const UcmImage* __restrict__ 
   }
 }
 
-__global__ void __launch_bounds__(256) k_ws_bw(const UcmView* __restrict__ views, const int32_t* __restrict__ ws) {
-  const UcmView& V = views[blockIdx.y];
+__global__ void __launch_bounds__(256) k_ws_bw(UcmLaunch l, const int32_t* __restrict__ ws) {
+  const UcmPart me = ucm_part(l);
+  const UcmView& V = me.V;
   const int W = V.W, P = W + 2;
   const long long N = (long long)V.H * W;
   const int32_t* L = ws + V.s.img->wpix + P + 1;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < N; i += (long long)gridDim.x * blockDim.x)
+  for (long long i = (long long)me.cta * blockDim.x + threadIdx.x; i < N; i += (long long)me.ctas * blockDim.x)
     V.s.bw[i] = L[i / W * P + i % W] == 0;
 }
 
@@ -268,15 +301,16 @@ __global__ void __launch_bounds__(256) k_ws_bw(const UcmView* __restrict__ views
 
 // One thread per painted pixel: the edge's orientation plane at that pixel,
 // max-ed into the strength map (which starts at 0, so negatives leave 0).
-__global__ void __launch_bounds__(256) k_ucm_paint(const UcmView* __restrict__ views) {
-  const UcmView& V = views[blockIdx.y];
+__global__ void __launch_bounds__(256) k_ucm_paint(UcmLaunch l) {
+  const UcmPart me = ucm_part(l);
+  const UcmView& V = me.V;
   const int32_t* __restrict__ pix = V.s.paint_pix;
   const uint8_t* __restrict__ ori = V.s.paint_ori;
   const int n = V.np;
   const long long N = (long long)V.H * V.W;
   const float* __restrict__ orient = V.orient;
   unsigned* wswt = (unsigned*)V.s.wswt;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+  for (int i = me.cta * blockDim.x + threadIdx.x; i < n; i += me.ctas * blockDim.x) {
     const int p = pix[i];
     const float v = orient[(long long)ori[i] * N + p];
     if (v > 0.0f) atomicMax(wswt + p, __float_as_uint(v));  // non-negative floats order as their bits
@@ -296,14 +330,15 @@ __device__ __forceinline__ float super_base(const float* w, int H, int W, int r,
   return 0.0f;
 }
 
-__global__ void __launch_bounds__(256) k_ucm_super(const UcmView* __restrict__ views) {
-  const UcmView& V = views[blockIdx.y];
+__global__ void __launch_bounds__(256) k_ucm_super(UcmLaunch l) {
+  const UcmPart me = ucm_part(l);
+  const UcmView& V = me.V;
   const float* __restrict__ wswt = V.s.wswt;
   const int H = V.H, W = V.W;
   float* __restrict__ pb2 = V.s.pb2;
   const long long n = 4LL * H * W;
   const int W2 = 2 * W;
-  for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
+  for (long long k = (long long)me.cta * blockDim.x + threadIdx.x; k < n; k += (long long)me.ctas * blockDim.x) {
     int r = (int)(k / W2);
     const int c = (int)(k % W2);
     if (r == 2 * H - 1) r = 2 * H - 2;
@@ -333,12 +368,13 @@ __device__ __forceinline__ bool isolated_zero(const float* g, int R, int C, int 
 // one warp per row: the row's isolated zeros, counted, or written in column
 // order from the row's place (rowcnt, scanned)
 template <bool WRITE>
-__global__ void __launch_bounds__(32) k_art_rows(const UcmView* __restrict__ views) {
-  const UcmView& V = views[blockIdx.y];
+__global__ void __launch_bounds__(32) k_art_rows(UcmLaunch l) {
+  const UcmPart me = ucm_part<2>(l);
+  const UcmView& V = me.V;
   const float* __restrict__ g = V.s.pb2;
   const int R = 2 * V.H, C = 2 * V.W;
   int32_t* __restrict__ list = V.s.art;
-  const int r = blockIdx.x, lane = threadIdx.x;
+  const int r = me.cta, lane = threadIdx.x;
   if (r >= R) return;
   int k = WRITE ? V.s.rowcnt[r] : 0;
   for (int c0 = 0; c0 < C; c0 += 32) {
@@ -355,7 +391,7 @@ __global__ void __launch_bounds__(32) k_art_rows(const UcmView* __restrict__ vie
 // (total to nart), or of the block sums of the root counts (total to nreg)
 template <bool ROWS>
 __global__ void __launch_bounds__(1024) k_scan_small(const UcmView* __restrict__ views) {
-  const UcmView& V = views[blockIdx.y];
+  const UcmView& V = views[blockIdx.x];
   int32_t* __restrict__ a = ROWS ? V.s.rowcnt : V.s.bsum;
   const int n = ROWS ? 2 * V.H : (int)((4LL * V.H * V.W + 4095) / 4096);
   int32_t* __restrict__ sum = ROWS ? V.s.nart : V.s.nreg;
@@ -384,12 +420,12 @@ __global__ void __launch_bounds__(1024) k_scan_small(const UcmView* __restrict__
 // the grid (artefacts within two cells of the border) read 0; writes there
 // are dropped.
 __global__ void k_art_fix(const UcmView* __restrict__ views) {
-  const UcmView& V = views[blockIdx.y];
+  const UcmView& V = views[blockIdx.x];
   float* __restrict__ g = V.s.pb2;
   const int R = 2 * V.H, C = 2 * V.W;
   const int32_t* __restrict__ list = V.s.art;
   const int32_t* __restrict__ n = V.s.nart;
-  if (threadIdx.x || blockIdx.x) return;
+  if (threadIdx.x) return;
   const long long tot = (long long)R * C;
   auto rd = [&](int r, int c) -> float {
     const long long k = (long long)r * C + c;  // a continuous matrix: columns wrap into the next row
@@ -453,9 +489,10 @@ __device__ __forceinline__ void ccl_union(int32_t* p, int a, int b) {
 
 // one warp per row: every zero cell's parent is the first cell of its
 // horizontal run, so the unions below only join runs of adjacent rows
-__global__ void __launch_bounds__(32) k_ccl_init(const UcmView* __restrict__ views) {
-  const UcmView& V = views[blockIdx.y];
-  const int R = 2 * V.H, C = 2 * V.W, r = blockIdx.x, lane = threadIdx.x;
+__global__ void __launch_bounds__(32) k_ccl_init(UcmLaunch l) {
+  const UcmPart me = ucm_part<2>(l);
+  const UcmView& V = me.V;
+  const int R = 2 * V.H, C = 2 * V.W, r = me.cta, lane = threadIdx.x;
   if (r >= R) return;
   const float* __restrict__ g = V.s.pb2 + (size_t)r * C;
   int32_t* __restrict__ p = V.s.par + (size_t)r * C;
@@ -474,13 +511,14 @@ __global__ void __launch_bounds__(32) k_ccl_init(const UcmView* __restrict__ vie
 // 642 x 962 grid, from 163 us with a union per adjacent pair): with the cell
 // above unless the left neighbour already has that contact; with a diagonal
 // cell only where the cells between offer none.
-__global__ void __launch_bounds__(256) k_ccl_hook(const UcmView* __restrict__ views) {
-  const UcmView& V = views[blockIdx.y];
+__global__ void __launch_bounds__(256) k_ccl_hook(UcmLaunch l) {
+  const UcmPart me = ucm_part(l);
+  const UcmView& V = me.V;
   const float* __restrict__ g = V.s.pb2;
   int32_t* p = V.s.par;
   const int R = 2 * V.H, C = 2 * V.W;
   const long long n = (long long)R * C;
-  for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x + C; k < n; k += (long long)gridDim.x * blockDim.x) {
+  for (long long k = (long long)me.cta * blockDim.x + threadIdx.x + C; k < n; k += (long long)me.ctas * blockDim.x) {
     if (g[k] != 0.0f) continue;
     const int c = (int)(k % C);
     const bool left = c > 0 && g[k - 1] == 0.0f, upleft = c > 0 && g[k - C - 1] == 0.0f;
@@ -494,12 +532,13 @@ __global__ void __launch_bounds__(256) k_ccl_hook(const UcmView* __restrict__ vi
 }
 
 // flatten to roots; rank[k] = 1 where k is a root (the component's first cell)
-__global__ void __launch_bounds__(256) k_ccl_flat(const UcmView* __restrict__ views) {
-  const UcmView& V = views[blockIdx.y];
+__global__ void __launch_bounds__(256) k_ccl_flat(UcmLaunch l) {
+  const UcmPart me = ucm_part(l);
+  const UcmView& V = me.V;
   int32_t* p = V.s.par;
   int32_t* __restrict__ root = V.s.rank;
   const long long n = 4LL * V.H * V.W;
-  for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
+  for (long long k = (long long)me.cta * blockDim.x + threadIdx.x; k < n; k += (long long)me.ctas * blockDim.x) {
     if (p[k] < 0) {
       root[k] = 0;
       continue;
@@ -512,8 +551,9 @@ __global__ void __launch_bounds__(256) k_ccl_flat(const UcmView* __restrict__ vi
 
 // region labels of the pixels (0-based; cells that are not zeros give -1)
 // and ws_wt2, the grid padded by its last row and column
-__global__ void __launch_bounds__(256) k_ucm_finish(const UcmView* __restrict__ views) {
-  const UcmView& V = views[blockIdx.y];
+__global__ void __launch_bounds__(256) k_ucm_finish(UcmLaunch l) {
+  const UcmPart me = ucm_part(l);
+  const UcmView& V = me.V;
   const float* __restrict__ g = V.s.pb2;
   const int32_t* __restrict__ p = V.s.par;
   const int32_t* __restrict__ rank = V.s.rank;
@@ -522,7 +562,7 @@ __global__ void __launch_bounds__(256) k_ucm_finish(const UcmView* __restrict__ 
   float* __restrict__ wswt2 = V.s.wswt2;
   const int R = 2 * H, C = 2 * W;
   const long long n2 = (long long)(R + 1) * (C + 1);
-  for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < n2; k += (long long)gridDim.x * blockDim.x) {
+  for (long long k = (long long)me.cta * blockDim.x + threadIdx.x; k < n2; k += (long long)me.ctas * blockDim.x) {
     const int r = (int)(k / (C + 1)), c = (int)(k % (C + 1));
     wswt2[k] = g[(size_t)(r == R ? R - 1 : r) * C + (c == C ? C - 1 : c)];
     if (r < H && c < W) {
@@ -534,14 +574,15 @@ __global__ void __launch_bounds__(256) k_ucm_finish(const UcmView* __restrict__ 
 }
 
 // exclusive scan of n (up to 2^31) ints through blocks of 1024 x 4
-__global__ void __launch_bounds__(1024) k_scan_blocks(const UcmView* __restrict__ views) {
-  const UcmView& V = views[blockIdx.y];
+__global__ void __launch_bounds__(1024) k_scan_blocks(UcmLaunch l) {
+  const UcmPart me = ucm_part(l);
+  const UcmView& V = me.V;
   int32_t* __restrict__ a = V.s.rank;
   int32_t* __restrict__ bsum = V.s.bsum;
   const long long n = 4LL * V.H * V.W;
-  if ((long long)blockIdx.x * 4096 >= n) return;
+  if ((long long)me.cta * 4096 >= n) return;
   __shared__ int32_t part[1024];
-  const long long b0 = (long long)blockIdx.x * 4096;
+  const long long b0 = (long long)me.cta * 4096;
   const int t = threadIdx.x;
   int32_t v[4], s = 0;
   for (int k = 0; k < 4; k++) {
@@ -563,15 +604,16 @@ __global__ void __launch_bounds__(1024) k_scan_blocks(const UcmView* __restrict_
     if (i < n) a[i] = run;
     run += v[k];
   }
-  if (t == 1023) bsum[blockIdx.x] = part[1023];
+  if (t == 1023) bsum[me.cta] = part[1023];
 }
 
-__global__ void __launch_bounds__(256) k_scan_add(const UcmView* __restrict__ views) {
-  const UcmView& V = views[blockIdx.y];
+__global__ void __launch_bounds__(256) k_scan_add(UcmLaunch l) {
+  const UcmPart me = ucm_part(l);
+  const UcmView& V = me.V;
   int32_t* __restrict__ a = V.s.rank;
   const int32_t* __restrict__ bsum = V.s.bsum;
   const long long n = 4LL * V.H * V.W;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
+  for (long long i = (long long)me.cta * blockDim.x + threadIdx.x; i < n; i += (long long)me.ctas * blockDim.x)
     a[i] += bsum[i / 4096];
 }
 
@@ -582,13 +624,29 @@ static int grid_for(long long n) {
   return (int)(g < 1 ? 1 : (g > 152 * 16 ? 152 * 16 : g));
 }
 
+void ucm_ctas(UcmView* views, UcmBatch& b) {
+  int at[kUcmKinds] = {};
+  for (int i = 0; i <= b.n; i++) {
+    std::copy(at, at + kUcmKinds, views[i].first);
+    if (i == b.n) break;
+    const long long N = (long long)views[i].H * views[i].W;
+    at[kUcmPix] += grid_for(N);
+    at[kUcmCells] += grid_for(4 * N);
+    at[kUcmRows] += views[i].H;
+    at[kUcmPaint] += views[i].np ? grid_for(views[i].np) : 0;
+    at[kUcmScan] += (int)((4 * N + 4095) / 4096);
+  }
+  std::copy(at, at + kUcmKinds, b.ctas);
+}
+
+static UcmLaunch ucm_launch(const UcmBatch& b, UcmKind k) { return {b.views, b.n, k}; }
+
 cudaError_t ucm_prepare(const UcmBatch& b, const UcmScratch& base, cudaStream_t st) {
   const cudaError_t e = cudaMemsetAsync(base.mm, 0, 2 * (size_t)b.n * sizeof(unsigned), st);
   if (e != cudaSuccess) return e;
-  const dim3 g(grid_for(b.max_pix), b.n);
-  k_ucm_pbmax<<<g, 256, 0, st>>>(b.views);
-  k_ucm_quant<<<g, 256, 0, st>>>(b.views);
-  k_ws_rowsort<<<dim3(b.max_h, b.n), 32, 0, st>>>(b.views);
+  k_ucm_pbmax<<<b.ctas[kUcmPix], 256, 0, st>>>(ucm_launch(b, kUcmPix));
+  k_ucm_quant<<<b.ctas[kUcmPix], 256, 0, st>>>(ucm_launch(b, kUcmPix));
+  k_ws_rowsort<<<b.ctas[kUcmRows], 32, 0, st>>>(ucm_launch(b, kUcmRows));
   return cudaGetLastError();
 }
 
@@ -596,32 +654,32 @@ cudaError_t ucm_flood(const UcmBatch& b, const UcmScratch& base, cudaStream_t st
   const cudaError_t e = cudaMemsetAsync(base.ws, 0xff, (size_t)b.ws_cells * sizeof(int32_t), st);
   if (e != cudaSuccess) return e;
   k_ws_flood<<<b.n, 1024, 0, st>>>(base.img, base.off, base.cols, base.ws);
-  k_ws_bw<<<dim3(grid_for(b.max_pix), b.n), 256, 0, st>>>(b.views, base.ws);
+  k_ws_bw<<<b.ctas[kUcmPix], 256, 0, st>>>(ucm_launch(b, kUcmPix), base.ws);
   return cudaGetLastError();
 }
 
 cudaError_t ucm_paint(const UcmBatch& b, const UcmScratch& base, cudaStream_t st) {
   const cudaError_t e = cudaMemsetAsync(base.wswt, 0, (size_t)b.total_pix * sizeof(float), st);
   if (e != cudaSuccess) return e;
-  if (b.max_paint > 0) k_ucm_paint<<<dim3(grid_for(b.max_paint), b.n), 256, 0, st>>>(b.views);
+  if (b.ctas[kUcmPaint] > 0) k_ucm_paint<<<b.ctas[kUcmPaint], 256, 0, st>>>(ucm_launch(b, kUcmPaint));
   return cudaGetLastError();
 }
 
 cudaError_t ucm_mid(const UcmBatch& b, cudaStream_t st) {
-  const long long n = 4 * b.max_pix;
-  const dim3 rows(2 * b.max_h, b.n), one(1, b.n), cells(grid_for(n), b.n);
-  k_ucm_super<<<cells, 256, 0, st>>>(b.views);
-  k_art_rows<false><<<rows, 32, 0, st>>>(b.views);
-  k_scan_small<true><<<one, 1024, 0, st>>>(b.views);
-  k_art_rows<true><<<rows, 32, 0, st>>>(b.views);
-  k_art_fix<<<one, 32, 0, st>>>(b.views);
-  k_ccl_init<<<rows, 32, 0, st>>>(b.views);
-  k_ccl_hook<<<cells, 256, 0, st>>>(b.views);
-  k_ccl_flat<<<cells, 256, 0, st>>>(b.views);
-  k_scan_blocks<<<dim3((unsigned)((n + 4095) / 4096), b.n), 1024, 0, st>>>(b.views);
-  k_scan_small<false><<<one, 1024, 0, st>>>(b.views);
-  k_scan_add<<<cells, 256, 0, st>>>(b.views);
-  k_ucm_finish<<<cells, 256, 0, st>>>(b.views);
+  const UcmLaunch cells = ucm_launch(b, kUcmCells), rows = ucm_launch(b, kUcmRows);
+  const int nc = b.ctas[kUcmCells], nr = 2 * b.ctas[kUcmRows];  // rows of the doubled grid
+  k_ucm_super<<<nc, 256, 0, st>>>(cells);
+  k_art_rows<false><<<nr, 32, 0, st>>>(rows);
+  k_scan_small<true><<<b.n, 1024, 0, st>>>(b.views);
+  k_art_rows<true><<<nr, 32, 0, st>>>(rows);
+  k_art_fix<<<b.n, 32, 0, st>>>(b.views);
+  k_ccl_init<<<nr, 32, 0, st>>>(rows);
+  k_ccl_hook<<<nc, 256, 0, st>>>(cells);
+  k_ccl_flat<<<nc, 256, 0, st>>>(cells);
+  k_scan_blocks<<<b.ctas[kUcmScan], 1024, 0, st>>>(ucm_launch(b, kUcmScan));
+  k_scan_small<false><<<b.n, 1024, 0, st>>>(b.views);
+  k_scan_add<<<nc, 256, 0, st>>>(cells);
+  k_ucm_finish<<<nc, 256, 0, st>>>(cells);
   return cudaGetLastError();
 }
 

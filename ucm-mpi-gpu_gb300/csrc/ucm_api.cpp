@@ -86,7 +86,7 @@ cudaError_t ucm_reserve(UcmState& u, const std::vector<int>& H, const std::vecto
   // slots: mm, pb, q, off, cols, img, ws, bw, wswt, pb2, rowcnt, nart, art, par, rank, bsum, nreg, labels, wswt2, views
   const size_t sizes[] = {2 * n * 4, T.pix * 4, T.pix, T.rows * 257 * 4, T.pix * 2, n * sizeof(UcmImage), T.border * 4,
                           T.pix, T.pix * 4, T.pix4 * 4, T.rows2 * 4, n * 4, T.pix4 * 4, T.pix4 * 4, T.pix4 * 4,
-                          T.bsum * 4, n * 4, T.pix * 4, T.grid2 * 4, n * sizeof(UcmView)};
+                          T.bsum * 4, n * 4, T.pix * 4, T.grid2 * 4, (n + 1) * sizeof(UcmView)};
   constexpr size_t kSlots = sizeof(sizes) / sizeof(sizes[0]);
   size_t need = 0;
   for (size_t b : sizes) need += align256(b);
@@ -195,14 +195,14 @@ extern "C" gpb_status gpb_ucm_batch(gpb_ctx* ctx, size_t n, const uint32_t* widt
     }
     UCK(cudaMemcpyAsync(u.views[0].img, imgs.data(), n * sizeof(UcmImage), cudaMemcpyHostToDevice, st));
     // device: orientation max, quantisation, row sort and flooding
-    std::vector<UcmView> views(n);
-    UcmBatch batch = {u.d_views, ni, 0, 0, (long long)pix[n], 0, ws_cells};
-    for (size_t i = 0; i < n; i++) {
-      views[i] = {u.views[i], d_orient[i], H[i], W[i], 0};
-      batch.max_h = std::max(batch.max_h, H[i]);
-      batch.max_pix = std::max(batch.max_pix, (long long)N[i]);
-    }
-    UCK(cudaMemcpyAsync(u.d_views, views.data(), n * sizeof(UcmView), cudaMemcpyHostToDevice, st));
+    std::vector<UcmView> views(n + 1);
+    UcmBatch batch = {u.d_views, ni, {}, (long long)pix[n], ws_cells};
+    for (size_t i = 0; i < n; i++) views[i] = {u.views[i], d_orient[i], H[i], W[i], 0, {}};
+    auto upload = [&]() -> cudaError_t {
+      ucm_ctas(views.data(), batch);
+      return cudaMemcpyAsync(u.d_views, views.data(), views.size() * sizeof(UcmView), cudaMemcpyHostToDevice, st);
+    };
+    UCK(upload());
     UCK(ucm_prepare(batch, u.views[0], st));
     UCK(ucm_flood(batch, u.views[0], st));
     std::vector<uint8_t> bw(pix[n]);
@@ -249,9 +249,8 @@ extern "C" gpb_status gpb_ucm_batch(gpb_ctx* ctx, size_t n, const uint32_t* widt
       views[i].s.paint_pix = u.paint_pix + poff[i];
       views[i].s.paint_ori = u.paint_ori + poff[i];
       views[i].np = (int)(poff[i + 1] - poff[i]);
-      batch.max_paint = std::max(batch.max_paint, views[i].np);
     }
-    UCK(cudaMemcpyAsync(u.d_views, views.data(), n * sizeof(UcmView), cudaMemcpyHostToDevice, st));
+    UCK(upload());
     UCK(ucm_paint(batch, u.views[0], st));
     UCK(ucm_mid(batch, st));
     std::vector<size_t> g2(n + 1, 0);

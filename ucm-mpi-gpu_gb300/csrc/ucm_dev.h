@@ -36,20 +36,30 @@ struct UcmScratch {
   float* wswt2;        // (2H+1)(2W+1)
 };
 
-// one image of a batch, as the kernels see it (blockIdx.y)
+// The CTAs of a launch belong to the images one after the other, each with as
+// many as its own size asks for: by pixels, by cells of the doubled grid, by
+// rows, by painted pixels, by blocks of the scan.  (As many as the largest
+// image for every one would be 36 M CTAs by rows for an image of 6000 x 2 among
+// 6000 of 2 x 2, which have 18 K rows together.)
+enum UcmKind { kUcmPix, kUcmCells, kUcmRows, kUcmPaint, kUcmScan, kUcmKinds };
+
+// one image of a batch, as the kernels see it
 struct UcmView {
   UcmScratch s;
-  const float* orient;  // 8 planes
-  int H, W, np;         // np: painted pixels
+  const float* orient;   // 8 planes
+  int H, W, np;          // np: painted pixels
+  int first[kUcmKinds];  // its first CTA in launches of each kind
 };
 // what sizes the launches of a batch
 struct UcmBatch {
-  const UcmView* views;  // device, n entries
-  int n, max_h;
-  long long max_pix, total_pix;
-  int max_paint;
+  const UcmView* views;  // device: n images, and an entry behind them whose `first` are the CTAs of all
+  int n;
+  int ctas[kUcmKinds];
+  long long total_pix;
   long long ws_cells;    // of all images' flooding labels
 };
+// fills the `first` of n + 1 views and b.ctas
+void ucm_ctas(UcmView* views, UcmBatch& b);
 
 // max over orientations, quantisation, per-row level sort; base is image 0's
 // view, whose arrays start the batch's concatenated ones
