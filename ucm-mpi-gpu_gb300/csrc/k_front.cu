@@ -412,11 +412,16 @@ __global__ void __launch_bounds__(64 * SPLIT) k_texton(const PatchDev* __restric
   }
 }
 
+constexpr int kRingChunk = 69;  // odd: the 13 rows reach distinct banks
 // FP64 repair, a CTA per flagged pixel: ring sums in integers, the products
 // K32[f][r] * S[r] in parallel, then their sums in ascending ring order and
 // the squared distances, all without contraction.  Bound by latency (a few
 // pixels in a thousand): 24 us at 96 x 131 and 45 us at 1024^2, from 54 and 86
-// us with a warp per pixel and one load at a time.
+// us with a warp per pixel and one load at a time.  The first warp sums a chunk
+// of rings while the others form the next chunk's products: with all products
+// of a pixel in shared memory (30 KB) 7 CTAs fit an SM, and 1024^2 pixels that
+// are all flagged (two equal codewords) take 67 ms; 39 ms in chunks, 59 ms with
+// a warp per pixel.
 __global__ void __launch_bounds__(128) k_texton_repair(const PatchDev* __restrict__ patches,
                                                        const uint8_t* __restrict__ grey,
                                                        uint32_t* __restrict__ lab4,
@@ -424,9 +429,10 @@ __global__ void __launch_bounds__(128) k_texton_repair(const PatchDev* __restric
                                                        const int* __restrict__ repair_count,
                                                        int repair_cap, const double* __restrict__ k32_ring,
                                                        const int* __restrict__ ring_of, int n_rings) {
-  extern __shared__ double prod[];  // [13][n_rings], then the ring sums
-  int* S = (int*)(prod + kNschmid * n_rings);
+  __shared__ double prod[2][kNschmid * kRingChunk];
+  extern __shared__ int S[];  // [n_rings]
   __shared__ double Rsh[kNschmid];
+  const int nch = (n_rings + kRingChunk - 1) / kRingChunk;
   const int tid = threadIdx.x, lane = tid & 31;
   const int total = min(*repair_count, repair_cap);
   for (int item = blockIdx.x; item < total; item += gridDim.x) {
@@ -443,16 +449,30 @@ __global__ void __launch_bounds__(128) k_texton_repair(const PatchDev* __restric
       atomicAdd(&S[ring_of[o]], v);
     }
     __syncthreads();
+    // products of a chunk of rings, [filter][ring of the chunk]
+    auto products = [&](int c, int t0, int nt) {
+      const int r0 = c * kRingChunk, nr = min(kRingChunk, n_rings - r0);
 #pragma unroll 8
-    for (int e = tid; e < kNschmid * n_rings; e += 128) prod[e] = __dmul_rn(k32_ring[e], (double)S[e % n_rings]);
-    __syncthreads();
-    if (tid < 32) {
-      if (lane < kNschmid) {
-        double acc = 0;
-#pragma unroll 8
-        for (int r = 0; r < n_rings; r++) acc = __dadd_rn(acc, prod[lane * n_rings + r]);
-        Rsh[lane] = acc;
+      for (int e = t0; e < kNschmid * kRingChunk; e += nt) {
+        const int f = e / kRingChunk, r = e % kRingChunk;
+        if (r < nr) prod[c & 1][e] = __dmul_rn(k32_ring[f * n_rings + r0 + r], (double)S[r0 + r]);
       }
+    };
+    products(0, tid, 128);
+    __syncthreads();
+    double acc = 0;
+    for (int c = 0; c < nch; c++) {
+      if (tid >= 32) {
+        if (c + 1 < nch) products(c + 1, tid - 32, 96);
+      } else if (lane < kNschmid) {
+        const int nr = min(kRingChunk, n_rings - c * kRingChunk);
+#pragma unroll 8
+        for (int r = 0; r < nr; r++) acc = __dadd_rn(acc, prod[c & 1][lane * kRingChunk + r]);
+      }
+      __syncthreads();
+    }
+    if (tid < 32) {
+      if (lane < kNschmid) Rsh[lane] = acc;
       __syncwarp();
       const int K = c_K;
       double d = 1e300;
@@ -516,9 +536,8 @@ cudaError_t launch_texton_repair(const PatchDev* patches, const uint8_t* grey, u
                                  const int* repair_list, const int* repair_count, int repair_cap,
                                  const double* k32_ring, const int* ring_of, int n_rings,
                                  cudaStream_t s) {
-  const int smem = n_rings * (int)(kNschmid * sizeof(double) + sizeof(int));  // under 48 KB: at most 325 rings
-  k_texton_repair<<<1216, 128, smem, s>>>(patches, grey, lab4, repair_list, repair_count, repair_cap, k32_ring,
-                                          ring_of, n_rings);
+  k_texton_repair<<<1216, 128, n_rings * sizeof(int), s>>>(patches, grey, lab4, repair_list, repair_count, repair_cap,
+                                                           k32_ring, ring_of, n_rings);
   return cudaGetLastError();
 }
 
