@@ -1439,8 +1439,11 @@ static gpb_status run_batch(gpb_ctx* ctx, size_t n, const uint32_t* ws, const ui
   // a third of the tile list (the tiles are independent and the labels the
   // same), timed and scaled to the whole list
   const int ntex = (int)L.work_tex.size();
+  // Too few tiles to time, and to fill the SMs: four sets of threads per tile,
+  // as gpb_texton_labels_static takes up to 152 tiles (4, 20 and 42 tiles: 34 us,
+  // 49 to 51 with two sets).
   if (ctx->tuner.enabled && !ctx->tuner.decided(tx_key) && ntex < 16 * kTextonVariants)
-    ctx->tuner.settle(tx_key, kTextonVariants, 1);  // too few tiles to time
+    ctx->tuner.settle(tx_key, kTextonVariants, 2);
   const bool tx_trial = !ctx->tuner.decided(tx_key);
   if (tx_trial) ctx->tuner.entry(tx_key, kTextonVariants, 1);
   bool tx_unused = false;
