@@ -35,3 +35,7 @@ def test_stitch_launches_in_proportion_to_its_boxes(tmp_path):
 
 def test_ucm_launches_in_proportion_to_each_image(tmp_path):
     _run(tmp_path, "ucm_check")
+
+
+def test_tables_that_do_not_fit_are_an_error(tmp_path):
+    _run(tmp_path, "tables_check")

@@ -365,8 +365,10 @@ static cudaError_t load_tables(gpb_ctx* ctx) {
     cudaStreamWaitEvent(s, bk.static_done, 0);
     bk.static_pending = false;
   }
+  bk.owner = 0;  // nobody's until all of them are in place
   upload_front(ctx->tab, s);
-  upload_cues(ctx->tab, s);
+  const cudaError_t ce = upload_cues(ctx->tab, s);
+  if (ce != cudaSuccess) return ce;
   upload_buildw(ctx->tab, s);
   upload_eig(ctx->tab, s);
   upload_spb(ctx->tab, s);

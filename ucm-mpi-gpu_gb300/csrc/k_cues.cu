@@ -26,8 +26,6 @@
 // the results are the same to the bit.
 #include <float.h>
 #include <stdint.h>
-#include <stdio.h>
-#include <stdlib.h>
 
 #include "gpb_internal.h"
 #include "kernels.h"
@@ -50,7 +48,7 @@ __constant__ int c_nms_nb[kNori][4][2];
 __constant__ float c_nms_d[kNori];
 __constant__ float c_nms_cos[kNori][kNori];
 
-void upload_cues(const HostTables& t, cudaStream_t s) {
+cudaError_t upload_cues(const HostTables& t, cudaStream_t s) {
   int16_t dy[kAnnMax] = {}, dx[kAnnMax] = {};
   const int n = (int)t.ann_dy.size();
   for (int i = 0; i < n && i < kAnnMax; i++) {
@@ -65,10 +63,7 @@ void upload_cues(const HostTables& t, cudaStream_t s) {
     for (int l = 0; l < 32; l++) most = t.ann_count[a][l] > most ? t.ann_count[a][l] : most;
     row[a + 1] = row[a] + most;
   }
-  if (row[kNannulus] > kAnnRows) {
-    fprintf(stderr, "gpb: %d rows of disc offsets, %d fit\n", row[kNannulus], kAnnRows);
-    abort();
-  }
+  if (row[kNannulus] > kAnnRows) return cudaErrorInvalidValue;  // the disc's offsets do not fit
   cudaMemcpyToSymbolAsync(c_ann_dy, dy, sizeof(dy), 0, cudaMemcpyHostToDevice, s);
   cudaMemcpyToSymbolAsync(c_ann_dx, dx, sizeof(dx), 0, cudaMemcpyHostToDevice, s);
   cudaMemcpyToSymbolAsync(c_ann_start, t.ann_start, sizeof(t.ann_start), 0, cudaMemcpyHostToDevice, s);
@@ -82,6 +77,7 @@ void upload_cues(const HostTables& t, cudaStream_t s) {
   cudaMemcpyToSymbolAsync(c_nms_nb, t.nms_nb, sizeof(t.nms_nb), 0, cudaMemcpyHostToDevice, s);
   cudaMemcpyToSymbolAsync(c_nms_d, t.nms_d, sizeof(t.nms_d), 0, cudaMemcpyHostToDevice, s);
   cudaMemcpyToSymbolAsync(c_nms_cos, t.nms_cos, sizeof(t.nms_cos), 0, cudaMemcpyHostToDevice, s);
+  return cudaSuccess;
 }
 
 __device__ __forceinline__ int reflect_c(int i, int n) {

@@ -30,7 +30,7 @@ cudaError_t launch_texton_repair(const PatchDev* patches, const uint8_t* grey, u
 
 // k_cues.cu
 constexpr int kCueTileH = 8, kCueTileW = 16;
-void upload_cues(const HostTables& t, cudaStream_t s);
+cudaError_t upload_cues(const HostTables& t, cudaStream_t s);
 cudaError_t launch_maxlabel(const PatchDev* patches, int npatch, const uint32_t* lab4, int* nbins,
                             cudaStream_t s);
 cudaError_t launch_cues(const PatchDev* patches, const int4* work, int nwork, const uint32_t* lab4,
