@@ -58,7 +58,6 @@ struct HostTables {
   int group_ring[kSchmidGroups];
   int n_rings;
   std::vector<double> k32_ring;  // [13][n_rings]
-  float err_bound[kNschmid];     // FP32 response error bound per filter
   // colour
   double gamma_lut[256];
   // local cues

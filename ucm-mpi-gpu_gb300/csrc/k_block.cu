@@ -67,13 +67,6 @@ void upload_block(const HostTables& t, cudaStream_t s) {
   cudaMemcpyToSymbolAsync(c_bup_dx, dx, sizeof(dx), 0, cudaMemcpyHostToDevice, s);
 }
 
-__device__ __forceinline__ void fma4(float4& acc, float a, const float4& x) {
-  acc.x = fmaf(a, x.x, acc.x);
-  acc.y = fmaf(a, x.y, acc.y);
-  acc.z = fmaf(a, x.z, acc.z);
-  acc.w = fmaf(a, x.w, acc.w);
-}
-
 // ------------------------------------------------------------ Chebyshev step
 // The operator of a level is stored per 16 x 16 pixel tile (the tiles of the
 // 16 x 16 work list, in its order), ready for the step's loads: 4 consecutive

@@ -9,7 +9,6 @@
 namespace gpb {
 
 constexpr int kBlk = 32;          // block width
-constexpr int kBlkThreads = 256;  // 64 pixels x 4 quarters per pass
 constexpr int kMaxCheb = 128;     // largest filter degree
 
 struct BlkArgs {

@@ -319,13 +319,6 @@ void build_tables(HostTables& t, int compat) {
       }
       g++;
     }
-  // FP32 error bound of a response: sum of 325 products with |prod| <= 2040|k|,
-  // accumulated in FP32 (Higham's gamma_n bound with n = 2*325, doubled)
-  for (int f = 0; f < kNschmid; f++) {
-    double s = 0;
-    for (int q = 0; q < kSchmidGroups; q++) s += 2040.0 * fabs((double)t.k32_group[f][q]);
-    t.err_bound[f] = (float)(2.0 * 650 * ldexp(1.0, -24) * s);
-  }
   // colour: gamma 2.5 of u8/255 (lib_image.cc:123-140 after globalPb.cpp:20)
   for (int i = 0; i < 256; i++) t.gamma_lut[i] = pow(i * (1.0 / 255.0), 2.5);
   // bin smoothing kernels: lib_image::gaussian(0.1*25) and (0.05*25)
