@@ -1015,7 +1015,9 @@ static gpb_status solve_block(gpb_ctx* ctx, const Level& lv, bool have_start, do
   a.mat = b.bmat;
   a.theta = b.btheta;
   const size_t BB = (size_t)kBlk * kBlk;
-  // block-step variant per level and tile-count bucket
+  // block-step variant per level and tile-count bucket (log2: a bucket's choice
+  // is up to 11 % of a call behind for its other counts, 4993 against 4752 us for
+  // 120 tiles after 72, since the better tile height follows the number of waves)
   auto step_key = [&](int nw) {
     return std::string(lv.coarse ? "step/coarse" : "step/fine") + "/tiles2^" + std::to_string(ilog2(nw));
   };

@@ -701,7 +701,10 @@ __global__ void __launch_bounds__(256, TWO ? 2 : 3) cf_gram(BlkArgs a, const flo
 
 // The Gram matrices' sums over a patch's CTA slots, 128 elements per CTA: a
 // patch of 0.4 Mpx has 800 slots (13 MB for two matrices), which its last
-// cf_gram CTA alone took longer to add than the others to form.
+// cf_gram CTA alone took longer to add than the others to form.  It pays for
+// few slots too: cf_gram + this launch take 8.6 + 2.5 us for one matrix of a
+// 64 x 80 image (12 slots) and 12.2 + 2.5 for two, from 13.4 and 20.0 us with
+// the last CTA adding; 9.4 + 6.7 from 30.1 and 13.0 + 6.7 from 52.8 for 266^2.
 constexpr int kSumThreads = 128;
 __global__ void __launch_bounds__(kSumThreads) cf_gram_sum(BlkArgs a, int ngram, double* __restrict__ out,
                                                            double* __restrict__ out2) {

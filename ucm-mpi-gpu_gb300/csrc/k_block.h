@@ -21,7 +21,8 @@ struct BlkArgs {
   long long lvec;
   const float3* coef;   // [npatch][max_steps] (alpha, beta, gamma)
   int max_steps;
-  double* part;         // [ntiles][32*32]
+  double* part;         // partial sums, FP32 hi + lo pairs: [ntiles * kBlkSplit][1 or 2 Gram
+                        // matrices, or 32 residuals]
   int* counter;         // [npatch]
   const int* active;    // [npatch]
   const int* done;      // [npatch]

@@ -281,7 +281,7 @@ __global__ void __launch_bounds__(kEigThreads, 2) ks_spmv(EigArgs a, int j, cons
   const EigTile t = a.tiles[blockIdx.x];
   if (!a.active[t.patch]) return;
   const PatchDev P = a.patches[t.patch];
-  // the FP64 root and quotient run beside the stencil; read after it
+  // one thread forms the FP64 root and quotient; all wait for it at the barrier below
   __shared__ float inv_s;
   if (threadIdx.x == 0) inv_s = use_beta ? (float)(1.0 / sqrt(a.beta2[t.patch])) : 1.f;
   const long long base = uniform(P.vec);
@@ -358,7 +358,7 @@ __global__ void __launch_bounds__(kEigThreads) ks_mult(EigArgs a, int j, const f
   const PatchDev P = a.patches[t.patch];
   __shared__ int off[kUpper];
   __shared__ float inv_s;
-  // the FP64 root and quotient run beside the stencil; read after it
+  // one thread forms the FP64 root and quotient; all wait for it at the barrier
   if (threadIdx.x == kEigThreads - 1) inv_s = use_beta ? (float)(1.0 / sqrt(a.beta2[t.patch])) : 1.f;
   if (threadIdx.x < kUpper) off[threadIdx.x] = c_up_dy[threadIdx.x] * P.W + c_up_dx[threadIdx.x];
   __syncthreads();

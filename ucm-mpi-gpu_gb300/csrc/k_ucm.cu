@@ -194,10 +194,12 @@ __global__ void __launch_bounds__(32) k_ws_rowsort(UcmLaunch l) {
 // ws is -1 (not reached), 0 (watershed pixel) or a region label (> 0): a
 // new region takes the label 1 + its pixel index.  It has a border of one
 // pixel that stays -1, so the gathers need no bounds checks.
-// Bound by instruction issue on the image's one SM (its 32 warps issue about
-// 4,000 instructions per step): 255 x 2 + H steps, 1.93 ms for 321 x 481, from
-// 2.87 ms with bounds checks and a branch per neighbour.  Loading each level's
-// place and columns a step ahead cost more instructions than it hid: 3.45 ms.
+// Bound by the chain of 255 x 2 + H steps on the image's one SM: it issues in
+// a third of its cycles (321 x 481: 6.3 M instructions, 34 %; 1024^2: 31 %), and
+// the warps wait for the busiest one at each step's barrier (10 cycles per
+// issue) and for its gathers (7 to 9).  1.93 ms for 321 x 481, from 2.87 ms with
+// bounds checks and a branch per neighbour.  Loading each level's place and
+// columns a step ahead lengthened the busiest warp's step: 3.45 ms.
 __global__ void __launch_bounds__(1024) k_ws_flood(const UcmImage* __restrict__ imgs, const int32_t* __restrict__ off,
                                                    const uint16_t* __restrict__ cols, int32_t* __restrict__ ws) {
   const UcmImage I = imgs[blockIdx.x];
