@@ -593,9 +593,9 @@ __global__ void __launch_bounds__(256) k_ln_gram(const LnPatch* __restrict__ lp,
 // (32 x 32) into cm, and the loss 9 - <C1, B>; bad is set where the
 // regularised G is not positive definite.  One CTA per patch in FP64 with
 // unfused operations in the order of a sequential Cholesky inverse, so the
-// values are those of host code.  Bound by the FP64 roots, quotients and
-// subtraction chains: 147 us for any number of patches up to the SMs, against
-// 0.77 ms for the host round trip of 16.
+// values are those of ln_solve_host.  Bound by the latency of the FP64 roots,
+// quotients and subtraction chains: 147 us for any number of patches up to the
+// SMs, against 0.77 ms for the host round trip of 16 (see kHostSolve).
 __global__ void __launch_bounds__(256) k_ln_solve(const double* __restrict__ gb, float* __restrict__ cm,
                                                   double* __restrict__ loss, int* __restrict__ bad) {
   constexpr int K = kLnOut, T = kLnTargets, LP = K + 1;
@@ -1113,6 +1113,61 @@ cudaError_t LearnedNet::forward(cudaStream_t s, float* out) {
   return cudaSuccess;
 }
 
+// k_ln_solve on the host, for one patch: the same operations in the same
+// order (the host's code is compiled without contraction); false where the
+// regularised Gram matrix is not positive definite
+static bool ln_solve_host(const double* g, float* cm, double* loss) {
+  constexpr int K = kLnOut, T = kLnTargets;
+  double A[K][K], Gi[K][K] = {}, C1[T * K];
+  const double* B = g + K * K;
+  double tr = 0;
+  for (int i = 0; i < K; i++) tr += g[i * K + i];
+  const double eps = 1e-4 * tr / K + 1e-30;
+  for (int i = 0; i < K; i++)
+    for (int j = 0; j < K; j++) A[i][j] = g[i * K + j] + (i == j ? eps : 0.0);
+  for (int i = 0; i < K; i++) Gi[i][i] = 1.0;
+  for (int j = 0; j < K; j++) {  // A becomes L, Gi becomes L^-1
+    if (!(A[j][j] > 0)) return false;
+    const double s = std::sqrt(A[j][j]);
+    A[j][j] = s;
+    for (int r = j + 1; r < K; r++) A[r][j] /= s;
+    for (int q = 0; q <= j; q++) Gi[j][q] /= s;
+    for (int r = j + 1; r < K; r++) {
+      for (int q = j + 1; q <= r; q++) A[r][q] -= A[r][j] * A[q][j];
+      for (int q = 0; q <= j; q++) Gi[r][q] -= A[r][j] * Gi[j][q];
+    }
+  }
+  for (int i = K - 1; i >= 0; i--) {  // (L L^T)^-1
+    for (int k = i + 1; k < K; k++)
+      for (int c = 0; c < K; c++) Gi[i][c] -= A[k][i] * Gi[k][c];
+    for (int c = 0; c < K; c++) Gi[i][c] /= A[i][i];
+  }
+  double cap = 0;
+  for (int i = 0; i < T; i++)
+    for (int j = 0; j < K; j++) {
+      double v = 0;
+      for (int k = 0; k < K; k++) v += B[i * K + k] * Gi[k][j];
+      C1[i * K + j] = v;
+      cm[i * K + j] = (float)v;
+      cap += v * B[i * K + j];
+    }
+  for (int a = 0; a < K; a++)
+    for (int b = 0; b < K; b++) {
+      double v = 0;
+      for (int i = 0; i < T; i++) v += C1[i * K + a] * C1[i * K + b];
+      cm[T * K + a * K + b] = (float)v;
+    }
+  *loss = T - cap;
+  return true;
+}
+
+// Gradients of up to this many patches solve on the host: a round trip and
+// about 17 us a patch against the 147 us of k_ln_solve's chain.  Microseconds
+// of one gradient of 64^2 patches, host / device: 1 patch 648 / 771 (48^2),
+// 4 patches 711 / 806, 8 patches 812 / 851, 10 patches 852 / 870, 12 patches
+// 905 / 890, 16 patches 1015 / 940.
+constexpr int kHostSolve = 8;
+
 cudaError_t LearnedNet::loss_backward(const float* d_v, double* loss, cudaStream_t s) {
   Impl& m = *im_;
   if (!m.have) return cudaErrorInvalidValue;
@@ -1124,10 +1179,23 @@ cudaError_t LearnedNet::loss_backward(const float* d_v, double* loss, cudaStream
       m.d_lp[0], m.y, d_v, m.gram);
   m.launches++;
   CKE(cudaGetLastError());
-  CKE(cudaMemsetAsync(m.bad, 0, sizeof(int), s));
-  k_ln_solve<<<np, 256, 0, s>>>(m.gram, m.cm, m.ploss, m.bad);
-  m.launches++;
-  CKE(cudaGetLastError());
+  const bool on_host = np <= kHostSolve;
+  m.h_loss.resize(np);
+  if (on_host) {
+    std::vector<double> g((size_t)np * kGramLen);
+    std::vector<float> c((size_t)np * kGramLen);
+    CKE(cudaMemcpyAsync(g.data(), m.gram, np * kGramLen * sizeof(double), cudaMemcpyDeviceToHost, s));
+    CKE(cudaStreamSynchronize(s));
+    for (int p = 0; p < np; p++)
+      if (!ln_solve_host(&g[(size_t)p * kGramLen], &c[(size_t)p * kGramLen], &m.h_loss[p]))
+        return cudaErrorInvalidValue;
+    CKE(cudaMemcpyAsync(m.cm, c.data(), np * kGramLen * sizeof(float), cudaMemcpyHostToDevice, s));
+  } else {
+    CKE(cudaMemsetAsync(m.bad, 0, sizeof(int), s));
+    k_ln_solve<<<np, 256, 0, s>>>(m.gram, m.cm, m.ploss, m.bad);
+    m.launches++;
+    CKE(cudaGetLastError());
+  }
   k_ln_dy<<<dim3((unsigned)std::max(1LL, std::min(m.maxpix[0] / 512 + 1, 1024LL)), np), 256, 0, s>>>(
       m.d_lp[0], m.y, d_v, m.cm, m.dY);
   m.launches++;
@@ -1167,12 +1235,13 @@ cudaError_t LearnedNet::loss_backward(const float* d_v, double* loss, cudaStream
   CKE(pool_bwd(0, 16, m.dP0, m.dS0));
   CKE(m.conv_bwd(1, 0, m.dS0, m.S0, m.one(m.A0a), m.dA0a, s));
   CKE(m.conv_bwd(0, 0, m.dA0a, m.A0a, m.one(m.X0), nullptr, s));
-  int bad = 0;
-  m.h_loss.resize(np);
-  CKE(cudaMemcpyAsync(m.h_loss.data(), m.ploss, np * sizeof(double), cudaMemcpyDeviceToHost, s));
-  CKE(cudaMemcpyAsync(&bad, m.bad, sizeof(int), cudaMemcpyDeviceToHost, s));
-  CKE(cudaStreamSynchronize(s));
-  if (bad) return cudaErrorInvalidValue;  // a patch's Gram matrix is not positive definite
+  if (!on_host) {
+    int bad = 0;
+    CKE(cudaMemcpyAsync(m.h_loss.data(), m.ploss, np * sizeof(double), cudaMemcpyDeviceToHost, s));
+    CKE(cudaMemcpyAsync(&bad, m.bad, sizeof(int), cudaMemcpyDeviceToHost, s));
+    CKE(cudaStreamSynchronize(s));
+    if (bad) return cudaErrorInvalidValue;  // a patch's Gram matrix is not positive definite
+  }
   *loss = 0;
   for (double l : m.h_loss) *loss += l;
 #undef CKE
