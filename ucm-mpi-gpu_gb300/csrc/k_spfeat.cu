@@ -6,9 +6,10 @@
 //   k_sp_accum  one thread per pixel: integer counts per (superpixel, texton),
 //               (superpixel, grey bin) and size, 64-bit colour sums (labels
 //               outside [0, n) are skipped).  Pixels of a warp in the same
-//               superpixel add up first, so the size and colour sums cost 4
-//               atomics per superpixel and warp instead of 4 per pixel, all
-//               to the same addresses (4 us instead of 13 for 266^2)
+//               superpixel add up first where the superpixels are large, so
+//               the size and colour sums cost 4 atomics per superpixel and
+//               warp instead of 4 per pixel, all to the same addresses (4 us
+//               instead of 13 for 266^2)
 //   k_sp_final  one thread per (superpixel, column): counts / size * 10,
 //               colour sums / size * (10 / 255), in FP64 in the reference's
 //               order of operations; a zero column for the Harris corner
@@ -20,6 +21,13 @@
 
 namespace gpb {
 
+// A warp whose 32 pixels form more runs of equal labels than this adds pixel by
+// pixel: matching many small groups costs more than their atomics.  Microseconds
+// of the launch grouping always / up to 7 runs / never: 300 superpixels in 266^2
+// 4.3 / 4.3 / 13.6, 2000 in 266^2 4.7 / 4.5 / 5.4, 2000 in 128^2 5.5 / 3.0 / 3.0,
+// 2000 in 64^2 6.6 / 2.9 / 2.9, random labels in 320^2 11.7 / 7.2 / 7.2 (up to 8
+// runs: 3.7 for 2000 in 128^2).
+constexpr int kSpRuns = 7;
 __global__ void __launch_bounds__(256) k_sp_accum(const PatchDev* __restrict__ patches, int pi,
                                                   const int32_t* __restrict__ labels, int n,
                                                   const uint32_t* __restrict__ lab4, const uint8_t* __restrict__ grey,
@@ -32,15 +40,21 @@ __global__ void __launch_bounds__(256) k_sp_accum(const PatchDev* __restrict__ p
     const long long i = i0 + threadIdx.x;
     const int l = i < P.N ? labels[i] : -1;
     const bool in = l >= 0 && l < n;
-    const unsigned peers = __match_any_sync(0xffffffffu, in ? l : -1 - lane);
+    const int key = in ? l : -1 - lane, left = __shfl_up_sync(0xffffffffu, key, 1);
+    const int runs = __popc(__ballot_sync(0xffffffffu, lane == 0 || key != left));
+    const unsigned peers = runs <= kSpRuns ? __match_any_sync(0xffffffffu, key) : 1u << lane;
     if (!in) continue;
     uint32_t* row = counts + (long long)l * ncnt;
     const int t = (int)(lab4[P.pix + i] >> 24);
     if (K > 0 && t < K) atomicAdd(row + t, 1u);
     atomicAdd(row + K + grey[P.pix + i] / bin_step, 1u);
     const uint32_t px = packed[P.pix + i];
-    const uint32_t sb = __reduce_add_sync(peers, (px >> 16) & 255u), sg = __reduce_add_sync(peers, (px >> 8) & 255u),
-                   sr = __reduce_add_sync(peers, px & 255u);
+    uint32_t sb = (px >> 16) & 255u, sg = (px >> 8) & 255u, sr = px & 255u;
+    if (runs <= kSpRuns) {
+      sb = __reduce_add_sync(peers, sb);
+      sg = __reduce_add_sync(peers, sg);
+      sr = __reduce_add_sync(peers, sr);
+    }
     if (lane == __ffs(peers) - 1) {
       atomicAdd(row + K + nbins, (uint32_t)__popc(peers));
       atomicAdd(csum + 3LL * l + 0, (unsigned long long)sb);
