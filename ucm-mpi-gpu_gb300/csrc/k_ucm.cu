@@ -126,7 +126,9 @@ __global__ void __launch_bounds__(256) k_ucm_quant(UcmLaunch l) {
 
 // ---------------------------------------------------------------- flooding
 
-// One warp per row: a stable counting sort of the row's columns by level.
+// One warp per row: a stable counting sort of the row's columns by level.  The
+// levels are read with __ldg, so that the loads may pass the warp's barriers
+// (60,000 columns: 662 us, 1057 without).
 // off[row * 257 + l] is the first position of level l; cols[row * W + k]
 // the k-th column in (level, column) order.
 __global__ void __launch_bounds__(32) k_ws_rowsort(UcmLaunch l) {
@@ -146,7 +148,7 @@ __global__ void __launch_bounds__(32) k_ws_rowsort(UcmLaunch l) {
   for (int c0 = 0; c0 < W; c0 += 32) {
     const int c = c0 + lane;
     const bool in = c < W;
-    const int v = in ? r[c] : 256 + lane;  // out-of-row lanes match nobody
+    const int v = in ? __ldg(r + c) : 256 + lane;  // out-of-row lanes match nobody
     const unsigned peers = __match_any_sync(0xffffffffu, v);
     if (in && (peers & lt) == 0) cnt[v] += __popc(peers);
     __syncwarp();
@@ -173,7 +175,7 @@ __global__ void __launch_bounds__(32) k_ws_rowsort(UcmLaunch l) {
   for (int c0 = 0; c0 < W; c0 += 32) {
     const int c = c0 + lane;
     const bool in = c < W;
-    const int v = in ? r[c] : 256 + lane;
+    const int v = in ? __ldg(r + c) : 256 + lane;
     const unsigned peers = __match_any_sync(0xffffffffu, v);
     if (in) cols[(size_t)row * W + cnt[v] + __popc(peers & lt)] = (uint16_t)c;
     __syncwarp();
@@ -489,30 +491,36 @@ __device__ __forceinline__ void ccl_union(int32_t* p, int a, int b) {
   }
 }
 
-// one warp per row: every zero cell's parent is the first cell of its
-// horizontal run, so the unions below only join runs of adjacent rows
-__global__ void __launch_bounds__(32) k_ccl_init(UcmLaunch l) {
+// one CTA per row, its warps taking segments of kCclSeg cells: every zero cell's
+// parent is the first cell of its horizontal run in the segment, so the unions
+// below only join runs of adjacent rows and segments.  (One warp per row took
+// 834 us for rows of 120,000 cells, a thread per cell none of note; 222 us so.)
+constexpr int kCclSeg = 512, kCclWarps = 4;
+__global__ void __launch_bounds__(32 * kCclWarps) k_ccl_init(UcmLaunch l) {
   const UcmPart me = ucm_part<2>(l);
   const UcmView& V = me.V;
-  const int R = 2 * V.H, C = 2 * V.W, r = me.cta, lane = threadIdx.x;
+  const int R = 2 * V.H, C = 2 * V.W, r = me.cta, lane = threadIdx.x & 31;
   if (r >= R) return;
   const float* __restrict__ g = V.s.pb2 + (size_t)r * C;
   int32_t* __restrict__ p = V.s.par + (size_t)r * C;
-  int start = 0;  // the run that reaches the chunk's first cell begins here, if any does
-  for (int c0 = 0; c0 < C; c0 += 32) {
-    const int c = c0 + lane;
-    const bool zero = c < C && g[c] == 0.0f;
-    const unsigned walls = ~__ballot_sync(0xffffffffu, zero);
-    const unsigned before = walls & ((1u << lane) - 1u);
-    if (c < C) p[c] = zero ? r * C + (before ? c0 + 32 - __clz(before) : start) : -1;
-    if (walls) start = c0 + 32 - __clz(walls);
+  for (int s0 = (threadIdx.x >> 5) * kCclSeg; s0 < C; s0 += kCclWarps * kCclSeg) {
+    int start = s0;  // the run that reaches the chunk's first cell begins here, if any does
+    for (int c0 = s0; c0 < min(s0 + kCclSeg, C); c0 += 32) {
+      const int c = c0 + lane;
+      const bool zero = c < C && __ldg(g + c) == 0.0f;
+      const unsigned walls = ~__ballot_sync(0xffffffffu, zero);
+      const unsigned before = walls & ((1u << lane) - 1u);
+      if (c < C) p[c] = zero ? r * C + (before ? c0 + 32 - __clz(before) : start) : -1;
+      if (walls) start = c0 + 32 - __clz(walls);
+    }
   }
 }
 
 // Joins with the row above, one union per contact of two runs (12 us for a
 // 642 x 962 grid, from 163 us with a union per adjacent pair): with the cell
 // above unless the left neighbour already has that contact; with a diagonal
-// cell only where the cells between offer none.
+// cell only where the cells between offer none; and with the left cell where a
+// segment begins.
 __global__ void __launch_bounds__(256) k_ccl_hook(UcmLaunch l) {
   const UcmPart me = ucm_part(l);
   const UcmView& V = me.V;
@@ -520,10 +528,13 @@ __global__ void __launch_bounds__(256) k_ccl_hook(UcmLaunch l) {
   int32_t* p = V.s.par;
   const int R = 2 * V.H, C = 2 * V.W;
   const long long n = (long long)R * C;
-  for (long long k = (long long)me.cta * blockDim.x + threadIdx.x + C; k < n; k += (long long)me.ctas * blockDim.x) {
+  for (long long k = (long long)me.cta * blockDim.x + threadIdx.x; k < n; k += (long long)me.ctas * blockDim.x) {
     if (g[k] != 0.0f) continue;
     const int c = (int)(k % C);
-    const bool left = c > 0 && g[k - 1] == 0.0f, upleft = c > 0 && g[k - C - 1] == 0.0f;
+    const bool left = c > 0 && g[k - 1] == 0.0f;
+    if (left && c % kCclSeg == 0) ccl_union(p, (int)k, (int)k - 1);
+    if (k < C) continue;
+    const bool upleft = c > 0 && g[k - C - 1] == 0.0f;
     if (g[k - C] == 0.0f) {
       if (!(left && upleft)) ccl_union(p, (int)k, (int)(k - C));
       continue;
@@ -675,7 +686,7 @@ cudaError_t ucm_mid(const UcmBatch& b, cudaStream_t st) {
   k_scan_small<true><<<b.n, 1024, 0, st>>>(b.views);
   k_art_rows<true><<<nr, 32, 0, st>>>(rows);
   k_art_fix<<<b.n, 32, 0, st>>>(b.views);
-  k_ccl_init<<<nr, 32, 0, st>>>(rows);
+  k_ccl_init<<<nr, 32 * kCclWarps, 0, st>>>(rows);
   k_ccl_hook<<<nc, 256, 0, st>>>(cells);
   k_ccl_flat<<<nc, 256, 0, st>>>(cells);
   k_scan_blocks<<<b.ctas[kUcmScan], 1024, 0, st>>>(ucm_launch(b, kUcmScan));
