@@ -595,7 +595,7 @@ __global__ void __launch_bounds__(256) k_ln_gram(const LnPatch* __restrict__ lp,
 // unfused operations in the order of a sequential Cholesky inverse, so the
 // values are those of ln_solve_host.  Bound by the latency of the FP64 roots,
 // quotients and subtraction chains: 147 us for any number of patches up to the
-// SMs, against 0.77 ms for the host round trip of 16 (see kHostSolve).
+// SMs (few patches solve on the host, see kHostSolve).
 __global__ void __launch_bounds__(256) k_ln_solve(const double* __restrict__ gb, float* __restrict__ cm,
                                                   double* __restrict__ loss, int* __restrict__ bad) {
   constexpr int K = kLnOut, T = kLnTargets, LP = K + 1;
